@@ -582,6 +582,59 @@ __device__ __forceinline__ float2 solve_tet(const Mat& bp, const TetRec& r, floa
 	return make_float2(l0, l1);
 }
 
+// The six solves of a whole-cube cluster in sequence, on the cluster's eight
+// vertices (local slots; only D's xyz changes). The cube's tets turn around
+// its diagonal (slots 0 and 3): tet t shares one vertex P with the tet before
+// it and brings one vertex N of the ring 2 1 4 5 6 7 (2), in the slots
+// (0, N, P, 3) for even t and (0, 3, N, P) for odd t. So the six run as three
+// turns of one loop of two solves, the ring moved by two places per turn.
+// A pass is one warp's chain of instructions, and six solves unrolled (34 KB
+// of code with the advance behind it) waited for instruction fetch 1.85 of
+// every 4.7 cycles on the 192-tet cantilever; the loop waits 0.44. Its 42 moves
+// per turn cost less: one frame 693 -> 631 us there, 1,048 -> 1,009 us on the
+// 1.57 M-tet mesh, 2,403 -> 2,188 us on 608,256 damped tets. Turning the
+// vertex advance into a loop as well lost (1,009 -> 1,163 us): it moves all
+// eight vertices eight times.
+// before(t, Dt) and after(t, multipliers) see each tet.
+template <bool EXT, class Before, class After>
+__device__ __forceinline__ void solve_cube(const Mat& mat, const float4* rec, float inv_dt, float inv_dt2, float4 O[8],
+                                           float4 D[8], Before before, After after) {
+	float4 ro[6] = {O[2], O[1], O[4], O[5], O[6], O[7]};
+	Vec3 rd[6] = {v3(D[2]), v3(D[1]), v3(D[4]), v3(D[5]), v3(D[6]), v3(D[7])};
+	auto f4 = [](const Vec3& a) { return make_float4(a.x, a.y, a.z, 0.0f); };
+	Vec3 d0 = v3(D[0]), d3 = v3(D[3]);
+#pragma unroll 1
+	for (int t = 0; t < 6; t += 2) {
+		const float4* r = rec + t * 4 * kLanes;
+		{
+			const TetRec tr = {r[0], r[kLanes], r[2 * kLanes], r[3 * kLanes]};
+			const float4 Ot[4] = {O[0], ro[1], ro[0], O[3]};
+			float4 Dt[4] = {f4(d0), f4(rd[1]), f4(rd[0]), f4(d3)};
+			before(t, Dt);
+			after(t, solve_tet<EXT>(mat, tr, inv_dt, inv_dt2, Ot, Dt));
+			d0 = v3(Dt[0]), rd[1] = v3(Dt[1]), rd[0] = v3(Dt[2]), d3 = v3(Dt[3]);
+		}
+		{
+			const TetRec tr = {r[4 * kLanes], r[5 * kLanes], r[6 * kLanes], r[7 * kLanes]};
+			const float4 Ot[4] = {O[0], O[3], ro[2], ro[1]};
+			float4 Dt[4] = {f4(d0), f4(d3), f4(rd[2]), f4(rd[1])};
+			before(t + 1, Dt);
+			after(t + 1, solve_tet<EXT>(mat, tr, inv_dt, inv_dt2, Ot, Dt));
+			d0 = v3(Dt[0]), d3 = v3(Dt[1]), rd[2] = v3(Dt[2]), rd[1] = v3(Dt[3]);
+		}
+		const float4 o0 = ro[0], o1 = ro[1];
+		const Vec3 e0 = rd[0], e1 = rd[1];
+#pragma unroll
+		for (int k = 0; k < 4; k++) ro[k] = ro[k + 2], rd[k] = rd[k + 2];
+		ro[4] = o0, ro[5] = o1, rd[4] = e0, rd[5] = e1;
+	}
+	// three turns of two: every vertex is back in its place
+	O[2] = ro[0], O[1] = ro[1], O[4] = ro[2], O[5] = ro[3], O[6] = ro[4], O[7] = ro[5];
+	auto back = [](float4& a, const Vec3& b) { a.x = b.x, a.y = b.y, a.z = b.z; };
+	back(D[0], d0), back(D[3], d3), back(D[2], rd[0]), back(D[1], rd[1]), back(D[4], rd[2]), back(D[5], rd[3]),
+	    back(D[6], rd[4]), back(D[7], rd[5]);
+}
+
 // PbdDamp (XPBDFEM/Xpbd.h:307-346): moves the tet's velocities towards its
 // rigid motion (mass-weighted centre velocity plus the rotation that carries
 // its angular momentum) by the fraction `damping`.
@@ -735,8 +788,8 @@ __device__ __forceinline__ bool stage_acquire(const DevCtx& C, Stage& st, uint32
 
 // Chunks whose clusters are all whole cubes of the 6-tet split in the
 // generator's corner order (every configuration mesh) share one local
-// topology, so the 8 vertices stay in registers and the 6 solves unroll with
-// compile-time slots: no shared-memory round trip inside the sequential chain.
+// topology, so the 8 vertices stay in registers (solve_cube): no shared-memory
+// round trip inside the sequential chain.
 // Local slot k of tet t: {0123, 0341, 0543, 0365, 0763, 0327}, packed four bits per slot.
 __host__ __device__ constexpr int cube_slot(int t, int k) {
 	return (int)(((t == 0   ? 0x3210u

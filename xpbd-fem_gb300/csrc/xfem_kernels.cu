@@ -123,18 +123,14 @@ __device__ __forceinline__ void run_chunk_cube(const DevCtx& C, Stage& st, int n
 				advance_vertex(C, vid[s], O[s], D[s], first, dt, inv_dt);
 				if (TAPE) tape_vertex(C, vid[s], O[s], Dbefore, s_launch, first);
 			}
-#pragma unroll
-		for (int t = 0; t < 6; t++) {
-			const float4* r = rec + t * 4 * kLanes + lane;
-			const TetRec tr = {r[0], r[kLanes], r[2 * kLanes], r[3 * kLanes]};
-			const float4 Ot[4] = {O[cube_slot(t, 0)], O[cube_slot(t, 1)], O[cube_slot(t, 2)], O[cube_slot(t, 3)]};
-			float4 Dt[4] = {D[cube_slot(t, 0)], D[cube_slot(t, 1)], D[cube_slot(t, 2)], D[cube_slot(t, 3)]};
-			if (TAPE) tape_tet(C, s_launch, trow + t, lane, Dt);
-			const float2 lam = solve_tet<EXT>(mat, tr, inv_dt, inv_dt2, Ot, Dt);
-#pragma unroll
-			for (int k = 0; k < 4; k++) D[cube_slot(t, k)] = Dt[k];
-			if (LAMBDAS) C.tlam[(size_t)(trow + t) * kLanes + lane] = lam;
-		}
+		solve_cube<EXT>(
+		    mat, rec + lane, inv_dt, inv_dt2, O, D,
+		    [&](int t, const float4* Dt) {
+			    if (TAPE) tape_tet(C, s_launch, trow + t, lane, Dt);
+		    },
+		    [&](int t, const float2& lam) {
+			    if (LAMBDAS) C.tlam[(size_t)(trow + t) * kLanes + lane] = lam;
+		    });
 	}
 	if (next >= 0) stage_issue_m(C, st, (uint32_t)next, mnext, lane);  // buffer consumed: prefetch
 	if (live) {
@@ -742,16 +738,8 @@ __device__ __forceinline__ void run_chunk_brick(const DevCtx& C, Stage& st, int 
 				else
 					advance_vertex(C, v, O[s], D[s], first, dt, inv_dt, bodies);
 			}
-#pragma unroll
-		for (int t = 0; t < 6; t++) {
-			const float4* r = rec + t * 4 * kLanes + lane;
-			const TetRec tr = {r[0], r[kLanes], r[2 * kLanes], r[3 * kLanes]};
-			const float4 Ot[4] = {O[cube_slot(t, 0)], O[cube_slot(t, 1)], O[cube_slot(t, 2)], O[cube_slot(t, 3)]};
-			float4 Dt[4] = {D[cube_slot(t, 0)], D[cube_slot(t, 1)], D[cube_slot(t, 2)], D[cube_slot(t, 3)]};
-			solve_tet<false>(mat, tr, inv_dt, inv_dt2, Ot, Dt);
-#pragma unroll
-			for (int k = 0; k < 4; k++) D[cube_slot(t, k)] = Dt[k];
-		}
+		solve_cube<false>(
+		    mat, rec + lane, inv_dt, inv_dt2, O, D, [](int, const float4*) {}, [](int, const float2&) {});
 	}
 	if (next >= 0) brick_issue(C, st, (uint32_t)next, lane);  // buffer consumed: prefetch
 	if (live) {
