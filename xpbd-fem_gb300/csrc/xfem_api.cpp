@@ -1733,6 +1733,15 @@ int build_device(xfem_body* h) {
 	return update_right_targets(h);
 }
 
+// Whether the persistent form (sync_mode 1) of this handle runs as one
+// thread-block cluster, and of how many blocks (cluster_plan). Returns a
+// cudaError_t value.
+int pick_cluster(xfem_body* h) {
+	h->cfg.cluster = ClusterPlan();
+	if (h->cfg.sync_mode != 1 || h->cfg.lambdas || !h->nchunks) return 0;
+	return cluster_plan(h->ctx, h->max_colour_chunks, h->cfg.block, false, h->cfg.ext, &h->cfg.cluster);
+}
+
 int set_config(xfem_body* h, int sync_mode, int block) {
 	int optin = 0;
 	XCUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device));
@@ -1775,6 +1784,8 @@ int set_config(xfem_body* h, int sync_mode, int block) {
 		if (e) return fail(XFEM_ECUDA, std::string("occupancy query failed: ") + cudaGetErrorString((cudaError_t)e));
 		h->cfg.blocks = blocks;
 	}
+	if (const int e = pick_cluster(h))
+		return fail(XFEM_ECUDA, std::string("cluster query failed: ") + cudaGetErrorString((cudaError_t)e));
 	if (h->graph) {
 		cudaGraphExecDestroy(h->graph);
 		h->graph = nullptr;
@@ -2236,6 +2247,8 @@ int xfem_set_settings(xfem_body* h, uint32_t body, const xfem_settings* s) {
 			int blocks = 0;
 			if (persistent_grid(h->cfg, &blocks) == 0) h->cfg.blocks = blocks;
 		}
+		if (const int e = pick_cluster(h))
+			return fail(XFEM_ECUDA, std::string("cluster query failed: ") + cudaGetErrorString((cudaError_t)e));
 	}
 	if (h->ring_mode) h->ctx.ext = ring_damp_of(h->bodies) ? 1u : 0u;
 	const float4* rt_before = h->ctx.right_target;
@@ -3046,7 +3059,7 @@ int xfem_adjoint_forward(xfem_body* h, uint32_t nsub, float dt, uint32_t checkpo
 		if (nseg > 1)
 			XCUDA(cudaMemcpyAsync(a.ckpt.p + 2 * nv * j, h->vert.p, 2 * nv * sizeof(float4), cudaMemcpyDeviceToDevice,
 			                      h->stream));
-		const int e = launch_substeps_tape(tape_ctx(h, j), block, h->cfg.warp_smem, seg_len(a, j), dt, h->stream);
+		const int e = launch_substeps_tape(tape_ctx(h, j), block, h->cfg.warp_smem, h->max_colour_chunks, seg_len(a, j), dt, h->stream);
 		if (e) return fail(XFEM_ECUDA, std::string("recording launch: ") + cudaGetErrorString((cudaError_t)e));
 	}
 	if (nseg > 1)
@@ -3103,7 +3116,7 @@ int xfem_adjoint_backward(xfem_body* h, const float* grad_tip_traj, const float*
 		if (a.nseg > 1) {  // rebuild this segment's tape from its checkpoint
 			XCUDA(cudaMemcpyAsync(h->vert.p, a.ckpt.p + 2 * nv * j, 2 * nv * sizeof(float4), cudaMemcpyDeviceToDevice,
 			                      h->stream));
-			const int e = launch_substeps_tape(c, block, h->cfg.warp_smem, seg_len(a, j), a.dt, h->stream);
+			const int e = launch_substeps_tape(c, block, h->cfg.warp_smem, h->max_colour_chunks, seg_len(a, j), a.dt, h->stream);
 			if (e) return fail(XFEM_ECUDA, std::string("recording launch: ") + cudaGetErrorString((cudaError_t)e));
 		}
 		const int e = launch_reverse(c, actx, block, h->cfg.warp_smem, h->max_colour_chunks, seg_len(a, j), a.dt,

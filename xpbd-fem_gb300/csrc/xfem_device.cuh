@@ -102,6 +102,77 @@ __device__ __forceinline__ void st_vertex(float4* p, const float4& a, const floa
 	             : "memory");
 }
 
+// Barrier of a launch that is one thread-block cluster (every block of the
+// grid): a hardware barrier, which every thread reaches the same number of
+// times, so no wait of the kernel's own is involved. Orders the blocks'
+// global and distributed shared memory accesses. About 0.2 us with 16 blocks
+// against 1.4 us for grid_sync over 152 blocks.
+__device__ __forceinline__ void cluster_barrier() {
+	asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+	asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+}
+
+// Where the solve kernels find a vertex's state (O, w) and (D, bits): in
+// DevCtx::vert, or spread over the shared memory of the launch's one cluster
+// (block r holds device vertices [r * per, (r + 1) * per), O at
+// base + 16 * slot and D at base + 16 * (per + slot)).
+struct GlobalVerts {
+	__device__ __forceinline__ void ld(const DevCtx& C, uint32_t v, float4& O, float4& D) const {
+		ld_vertex(C.vert + 2 * (size_t)v, O, D);
+	}
+	// two 128-bit loads: the damping and volume sweeps keep them (with the
+	// 256-bit form in both of them, ptxas of CUDA 13.0 fails on xfem_kernels.cu)
+	__device__ __forceinline__ void ld2(const DevCtx& C, uint32_t v, float4& O, float4& D) const {
+		O = __ldcg(C.vert + 2 * (size_t)v);
+		D = __ldcg(C.vert + 2 * (size_t)v + 1);
+	}
+	__device__ __forceinline__ void st(const DevCtx& C, uint32_t v, const float4& O, const float4& D) const {
+		st_vertex(C.vert + 2 * (size_t)v, O, D);
+	}
+	__device__ __forceinline__ void st_o(const DevCtx& C, uint32_t v, const float4& O) const {
+		__stcg(C.vert + 2 * (size_t)v, O);
+	}
+	__device__ __forceinline__ void st_d(const DevCtx& C, uint32_t v, const float4& D) const {
+		__stcg(C.vert + 2 * (size_t)v + 1, D);
+	}
+};
+
+struct ClusterVerts {
+	uint32_t base, per, inv;  // shared address in every block, vertices per block, ceil(2^32 / per)
+
+	__device__ __forceinline__ uint32_t at(uint32_t v) const {
+		const uint32_t r = __umulhi(v, inv);  // v / per: v * per < 2^32
+		uint32_t a;
+		asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(base + 16u * (v - r * per)), "r"(r));
+		return a;
+	}
+	static __device__ __forceinline__ float4 get(uint32_t a) {
+		float4 x;
+		asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+		             : "=f"(x.x), "=f"(x.y), "=f"(x.z), "=f"(x.w)
+		             : "r"(a)
+		             : "memory");
+		return x;
+	}
+	static __device__ __forceinline__ void put(uint32_t a, const float4& x) {
+		asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(a), "f"(x.x), "f"(x.y), "f"(x.z), "f"(x.w)
+		             : "memory");
+	}
+	__device__ __forceinline__ void ld(const DevCtx&, uint32_t v, float4& O, float4& D) const {
+		const uint32_t a = at(v);
+		O = get(a);
+		D = get(a + 16u * per);
+	}
+	__device__ __forceinline__ void ld2(const DevCtx& C, uint32_t v, float4& O, float4& D) const { ld(C, v, O, D); }
+	__device__ __forceinline__ void st(const DevCtx&, uint32_t v, const float4& O, const float4& D) const {
+		const uint32_t a = at(v);
+		put(a, O);
+		put(a + 16u * per, D);
+	}
+	__device__ __forceinline__ void st_o(const DevCtx&, uint32_t v, const float4& O) const { put(at(v), O); }
+	__device__ __forceinline__ void st_d(const DevCtx&, uint32_t v, const float4& D) const { put(at(v) + 16u * per, D); }
+};
+
 struct Vec3 {
 	float x, y, z;
 };
@@ -232,6 +303,33 @@ __device__ __forceinline__ Mat load_mat(const BodyParams* bodies, uint32_t body)
 	        __ldg(&b->simultaneous), type < 2u ? __ldg(&b->damping) : 0.0f, type == 1u ? 1u : 0u,
 	        __ldg(&b->hw),         __ldg(&b->compliance),   __ldg(&b->volume_passes)};
 }
+
+// Where the solve kernels find a body's parameters: in DevCtx::bodies, or,
+// for a handle of one body, in registers (the vertex advance is then no chain
+// of loads per vertex).
+struct AnyBody {
+	__device__ __forceinline__ Mat mat(const DevCtx& C, uint32_t body) const { return load_mat(C.bodies, body); }
+	__device__ __forceinline__ void advance(const DevCtx& C, uint32_t v, float4& O, float4& D, bool first, float dt,
+	                                        float inv_dt) const {
+		advance_vertex(C, v, O, D, first, dt, inv_dt);
+	}
+	__device__ __forceinline__ void finalize(const DevCtx& C, uint32_t v, float4& O, float4& D, float inv_dt) const {
+		finalize_vertex(C, v, O, D, inv_dt);
+	}
+};
+
+struct OneBody {
+	BodyParams bp;
+	Mat m;
+	__device__ __forceinline__ Mat mat(const DevCtx&, uint32_t) const { return m; }
+	__device__ __forceinline__ void advance(const DevCtx& C, uint32_t v, float4& O, float4& D, bool first, float dt,
+	                                        float inv_dt) const {
+		advance_vertex_bp(C, bp, v, O, D, first, dt, inv_dt);
+	}
+	__device__ __forceinline__ void finalize(const DevCtx& C, uint32_t v, float4& O, float4& D, float inv_dt) const {
+		finalize_vertex_bp(C, bp, v, O, D, inv_dt);
+	}
+};
 
 // Hydrostatic term at the single point (XPBDFEM/Fem.cpp:539-549 with the
 // adjugate :284-300, F :311-323 and the gradient :338-354). J is formed as

@@ -452,9 +452,17 @@ constexpr int kErrNonFinite = 4;  // a finished position or velocity is NaN or i
 constexpr uint64_t kDefaultTimeoutNs = 2000000000ull;
 
 // ---- kernel launchers (xfem_kernels.cu) ---------------------------------------
+// The one-cluster form of the persistent kernel (xfem_cluster.cu), for small
+// handles: blocks of the cluster (0: the handle does not take this form), the
+// warps of a block that take chunks, and the chunk buffers of each.
+struct ClusterPlan {
+	uint32_t blocks = 0, warps = 0, bufs = 0;
+};
+
 struct LaunchCfg {
 	int block = 256;
 	int blocks = 0;        // persistent grid size
+	ClusterPlan cluster;   // sync_mode 1: the one-cluster form, when the handle takes it
 	int sync_mode = 1;     // 1 persistent + grid barrier, 2 per-colour launches (CUDA graph), 3 persistent dataflow,
 	                       // 4 persistent bricks (k_bricks: brick-resident vertices, neighbour waits)
 	bool lambdas = false;
@@ -472,6 +480,11 @@ int launch_substeps(const DevCtx& ctx, const LaunchCfg& cfg, uint32_t nsub, floa
 int configure_kernels(const LaunchCfg& cfg);
 // Largest co-resident grid for the persistent kernel at this block size.
 int persistent_grid(const LaunchCfg& cfg, int* blocks_out);
+// The one-cluster form's plan for a handle and a block size, and its launch
+// (tape: the recording forward). Both return a cudaError_t value.
+int cluster_plan(const DevCtx& ctx, uint32_t max_colour_chunks, int block, bool tape, bool ext, ClusterPlan* plan);
+int launch_cluster(const DevCtx& ctx, const ClusterPlan& plan, int block, bool tape, bool ext, uint32_t nsub, float dt,
+                   void* stream);
 // Dynamic shared memory bytes per block of the brick kernel, and whether
 // `nbricks` blocks of `block` threads fit on the device at once (the
 // cooperative launch needs the whole grid resident). Returns a cudaError_t
@@ -496,7 +509,8 @@ int launch_substeps_noalloc(const DevCtx& ctx, int block, uint32_t warp_smem, bo
 // backwards from that tape (`last`: the run's final segment, whose closing
 // finish receives the caller's dL/dX, dL/dV). Both are cooperative
 // persistent launches.
-int launch_substeps_tape(const DevCtx& ctx, int block, uint32_t warp_smem, uint32_t nsub, float dt, void* stream);
+int launch_substeps_tape(const DevCtx& ctx, int block, uint32_t warp_smem, uint32_t max_colour_chunks, uint32_t nsub,
+                         float dt, void* stream);
 int launch_reverse(const DevCtx& ctx, const AdjCtx& adj, int block, uint32_t warp_smem, uint32_t max_colour_chunks,
                    uint32_t nsub, float dt, bool last, void* stream);
 int configure_adjoint_kernels(int block, uint32_t warp_smem);

@@ -28,434 +28,13 @@
 #include <utility>
 #include <vector>
 
+#include "xfem_chunk.cuh"
 #include "xfem_device.cuh"
 #include "xfem_internal.h"
 
 namespace xfem {
 
 namespace {
-
-// Adjoint tape: the owner of a vertex records O right after the advance
-// (the position the substep starts from, with the inverse mass the solves
-// use) and D right before it, in one 32-byte sector, and, from the second
-// substep of a launch on, the tip trajectory (O is then the position after
-// the previous substep).
-__device__ __forceinline__ void tape_vertex(const DevCtx& C, uint32_t v, const float4& O, const float4& Dbefore,
-                                            uint32_t s, bool first) {
-	float4* p = C.tape_v + 2 * ((size_t)s * C.nverts + v);
-	__stcs(p, O);
-	__stcs(p + 1, Dbefore);
-	if (!first) {
-		const int q = __ldg(C.tip_of + v);
-		if (q >= 0) C.traj[(size_t)(C.sub_base + s - 1) * C.ntips + q] = O;
-	}
-}
-
-// Adjoint tape: the input displacement of one solve's four vertices.
-__device__ __forceinline__ void tape_tet(const DevCtx& C, uint32_t s, uint32_t row, uint32_t lane, const float4 D[4]) {
-	float4* p = C.tape_t + ((size_t)s * C.ntrows + row) * 3 * kLanes + lane;
-	__stcs(p, make_float4(D[0].x, D[0].y, D[0].z, D[1].x));
-	__stcs(p + kLanes, make_float4(D[1].y, D[1].z, D[2].x, D[2].y));
-	__stcs(p + 2 * kLanes, make_float4(D[2].z, D[3].x, D[3].y, D[3].z));
-}
-
-// ---- damping after the velocity update (GeoLinear3d::Damp) ------------------
-// State during the damping sweeps: vert[2v] = (X, w), vert[2v+1] = (V, bits).
-
-// Whether tet row `row` (lane `lane`) of body bp is damped at this tick, and
-// with which Rayleigh ratio and PBD fraction (XPBDFEM/Geo.cpp:346-352,
-// 792-798): the amortized type damps one eighth of the body's order per
-// tick, x 8.
-struct DampTet {
-	bool on;
-	float rayleigh, pbd;
-};
-
-__device__ __forceinline__ DampTet damp_of(const DevCtx& C, const BodyParams& bp, uint32_t row, uint32_t lane,
-                                           uint32_t tick, int kind) {
-	const uint32_t type = __ldg(&bp.rayleigh_type);
-	const bool amort = type == 3u;
-	DampTet d = {false, 0.0f, 0.0f};
-	if (kind == 0) {
-		d.rayleigh = __ldg(&bp.damping) * (amort ? 8.0f : 1.0f);
-		d.on = type >= 2u && d.rayleigh > 0.0f;
-	} else {
-		d.on = __ldg(&bp.pbd_on) != 0u;
-	}
-	if (!d.on) return d;
-	const size_t k = (size_t)row * kLanes + lane;
-	if (amort) {
-		const uint32_t nt = __ldg(&bp.ntets), f = __ldg(C.tflat + k), m = tick % 8u;
-		d.on = f >= nt * m / 8u && f < nt * (m + 1u) / 8u;
-	}
-	if (kind == 1) d.pbd = fminf(1.0f, (amort ? __ldg(&bp.pbd_coeff_amortized) : __ldg(&bp.pbd_coeff)) / __ldg(C.tarea + k));
-	return d;
-}
-
-// Header word of a cluster lane: nv | nt << 4 | advance mask << 8 | body << 16.
-// A vertex is advanced (previous substep finalized, next one predicted) by
-// the lowest-colour cluster touching it, just before that cluster's solve.
-
-template <bool LAMBDAS, bool TAPE, bool EXT>
-__device__ __forceinline__ void run_chunk_cube(const DevCtx& C, Stage& st, int next, const uint4& mnext, uint32_t lane,
-                                               bool first, float dt, float inv_dt, float inv_dt2, uint32_t trow,
-                                               uint32_t s_launch, uint32_t chunk, bool finish_last) {
-	const float4* rec = reinterpret_cast<const float4*>(st.buf);
-	const uint32_t* hdrs = reinterpret_cast<const uint32_t*>(st.buf + 2048u * 6u);
-	const uint32_t* vids = hdrs + kLanes;
-	const uint32_t hdr = hdrs[lane];
-	const bool live = (hdr & 15u) != 0;
-	const uint32_t mask = (hdr >> 8) & 0xffu;
-	uint32_t vid[8];
-	float4 O[8], D[8];
-	bool fin = false;  // this pass is the lane's last of the substep (its body runs no volume passes)
-	if (live) {
-		const Mat mat = load_mat(C.bodies, hdr >> 16);
-		fin = EXT && finish_last && mat.nvol == 0u;
-#pragma unroll
-		for (int s = 0; s < 8; s++) vid[s] = vids[s * kLanes + lane];
-#pragma unroll
-		for (int s = 0; s < 8; s++) ld_vertex(C.vert + 2 * (size_t)vid[s], O[s], D[s]);
-#pragma unroll
-		for (int s = 0; s < 8; s++)
-			if (mask & (1u << s)) {
-				const float4 Dbefore = D[s];
-				advance_vertex(C, vid[s], O[s], D[s], first, dt, inv_dt);
-				if (TAPE) tape_vertex(C, vid[s], O[s], Dbefore, s_launch, first);
-			}
-		solve_cube<EXT>(
-		    mat, rec + lane, inv_dt, inv_dt2, O, D,
-		    [&](int t, const float4* Dt) {
-			    if (TAPE) tape_tet(C, s_launch, trow + t, lane, Dt);
-		    },
-		    [&](int t, const float2& lam) {
-			    if (LAMBDAS) C.tlam[(size_t)(trow + t) * kLanes + lane] = lam;
-		    });
-	}
-	if (next >= 0) stage_issue_m(C, st, (uint32_t)next, mnext, lane);  // buffer consumed: prefetch
-	if (live) {
-		// with damping sweeps, the vertex's last solve of the substep finishes
-		// it (to the canonical X, V that the sweeps work on)
-		const uint32_t last = fin ? __ldg(C.lastmask + (size_t)chunk * kLanes + lane) : 0u;
-		// O changes only where this cluster advanced or finished the vertex
-		// (then the whole 32-byte state is stored); no other cluster of the
-		// pass touches these vertices
-#pragma unroll
-		for (int s = 0; s < 8; s++) {
-			if (EXT && (last & (1u << s))) finalize_vertex(C, vid[s], O[s], D[s], inv_dt);
-			if ((mask | last) & (1u << s))
-				st_vertex(C.vert + 2 * (size_t)vid[s], O[s], D[s]);
-			else  // only D moved: a 16-byte store
-				__stcg(C.vert + 2 * (size_t)vid[s] + 1, D[s]);
-		}
-	}
-}
-
-// One warp processes one resident chunk; lane = cluster. `next` >= 0 is the
-// warp's next chunk: its copy is issued as soon as this chunk's records have
-// been consumed, so it overlaps the write-back and what follows.
-template <bool LAMBDAS, bool TAPE = false, bool EXT = false>
-__device__ __forceinline__ void run_chunk(const DevCtx& C, Stage& st, uint32_t chunk, int next, uint32_t lane, bool first,
-                                          float dt, float inv_dt, float inv_dt2, uint32_t s_launch = 0,
-                                          bool finish_last = false) {
-	// the staged chunk's descriptor came with its copy; the next one's is
-	// loaded now, off the critical path of the prefetch
-	const uint4 m = st.meta;
-	const uint4 mnext = next >= 0 ? __ldg(reinterpret_cast<const uint4*>(C.chunks) + next) : make_uint4(0u, 0u, 0u, 0u);
-	const uint32_t ntmax = m.z & 0xffu, nvmax = (m.z >> 8) & 0xffu, trow = m.w;
-	if (m.z & kShapeCube) {
-		run_chunk_cube<LAMBDAS, TAPE, EXT>(C, st, next, mnext, lane, first, dt, inv_dt, inv_dt2, trow, s_launch, chunk,
-		                                    finish_last);
-		return;
-	}
-	const float4* rec = reinterpret_cast<const float4*>(st.buf);
-	const uint32_t* hdrs = reinterpret_cast<const uint32_t*>(st.buf + 2048u * ntmax);
-	const uint32_t* vids = hdrs + kLanes;
-	const uint32_t* slots = vids + kLanes * nvmax;
-	const uint32_t hdr = hdrs[lane];
-	const uint32_t nv = hdr & 15u, nt = (hdr >> 4) & 15u, mask = (hdr >> 8) & 0xffu;
-	float4* sO = st.vs + lane;
-	float4* sD = st.vs + kLanes * nvmax + lane;
-	uint32_t vid[kMaxClusterVerts];
-	bool fin = false;
-	if (nv) {
-		const Mat mat = load_mat(C.bodies, hdr >> 16);
-		fin = EXT && finish_last && mat.nvol == 0u;
-#pragma unroll
-		for (uint32_t s = 0; s < kMaxClusterVerts; s++)
-			if (s < nv) vid[s] = vids[s * kLanes + lane];
-#pragma unroll
-		for (uint32_t s = 0; s < kMaxClusterVerts; s++) {
-			if (s < nv) {
-				float4 O, D;
-				ld_vertex(C.vert + 2 * (size_t)vid[s], O, D);
-				if (mask & (1u << s)) {
-					const float4 Dbefore = D;
-					advance_vertex(C, vid[s], O, D, first, dt, inv_dt);
-					if (TAPE) tape_vertex(C, vid[s], O, Dbefore, s_launch, first);
-				}
-				sO[s * kLanes] = O;
-				sD[s * kLanes] = D;
-			}
-		}
-		for (uint32_t t = 0; t < nt; t++) {
-			const float4* r = rec + t * 4 * kLanes + lane;
-			const TetRec tr = {r[0], r[kLanes], r[2 * kLanes], r[3 * kLanes]};
-			const uint32_t sl = slots[t * kLanes + lane];
-			const uint32_t s0 = sl & 15u, s1 = (sl >> 4) & 15u, s2 = (sl >> 8) & 15u, s3 = (sl >> 12) & 15u;
-			const float4 O[4] = {sO[s0 * kLanes], sO[s1 * kLanes], sO[s2 * kLanes], sO[s3 * kLanes]};
-			float4 D[4] = {sD[s0 * kLanes], sD[s1 * kLanes], sD[s2 * kLanes], sD[s3 * kLanes]};
-			if (TAPE) tape_tet(C, s_launch, trow + t, lane, D);
-			const float2 lam = solve_tet<EXT>(mat, tr, inv_dt, inv_dt2, O, D);
-			sD[s0 * kLanes] = D[0];
-			sD[s1 * kLanes] = D[1];
-			sD[s2 * kLanes] = D[2];
-			sD[s3 * kLanes] = D[3];
-			if (LAMBDAS) C.tlam[(size_t)(trow + t) * kLanes + lane] = lam;
-		}
-	}
-	if (next >= 0) stage_issue_m(C, st, (uint32_t)next, mnext, lane);  // buffer consumed: prefetch
-	if (nv) {
-		const uint32_t last = fin ? __ldg(C.lastmask + (size_t)chunk * kLanes + lane) : 0u;
-#pragma unroll
-		for (uint32_t s = 0; s < kMaxClusterVerts; s++) {
-			if (s < nv) {
-				float4 O = sO[s * kLanes], D = sD[s * kLanes];
-				if (EXT && (last & (1u << s))) finalize_vertex(C, vid[s], O, D, inv_dt);
-				st_vertex(C.vert + 2 * (size_t)vid[s], O, D);
-			}
-		}
-	}
-}
-
-// The damping and volume sweeps keep two 128-bit vertex accesses: with the
-// 256-bit form in both of them, ptxas (CUDA 13.0) fails on this file.
-
-// Volume sweep k (1-based) over a resident chunk: SolveElementVolume on each
-// tet of the cluster in order (GeoLinear3d::Constrain, XPBDFEM/Geo.cpp:
-// 780-783), for lanes whose body runs at least k volume passes. The state is
-// (O, D), as in the solve sweep; only D changes, except that with damping
-// sweeps (finish) the body's last volume sweep finishes the vertices whose
-// last solve this cluster makes. CUBE: canonical cube chunks, all in
-// registers. Not inlined, like the damping passes.
-template <bool CUBE>
-__device__ __noinline__ void vol_chunk(const DevCtx& C, Stage& st, uint32_t chunk, uint32_t ntmax, uint32_t nvmax,
-                                       int next, uint32_t lane, float inv_dt, float inv_dt2, uint32_t k, bool finish) {
-	constexpr uint32_t NV = CUBE ? 8u : kMaxClusterVerts;
-	constexpr uint32_t NT = CUBE ? 6u : kMaxClusterTets;
-	const float4* rec = reinterpret_cast<const float4*>(st.buf);
-	const uint32_t* hdrs = reinterpret_cast<const uint32_t*>(st.buf + 2048u * ntmax);
-	const uint32_t* vids = hdrs + kLanes;
-	const uint32_t* slots = vids + kLanes * nvmax;
-	const uint32_t hdr = hdrs[lane];
-	const uint32_t nv = CUBE ? 8u : (hdr & 15u), nt = CUBE ? 6u : ((hdr >> 4) & 15u);
-	bool live = (hdr & 15u) != 0;
-	uint32_t vid[NV], last = 0;
-	float4 O[NV], D[NV];
-	if (live) {
-		const Mat mat = load_mat(C.bodies, hdr >> 16);
-		live = mat.nvol >= k;
-		if (finish && mat.nvol == k) last = __ldg(C.lastmask + (size_t)chunk * kLanes + lane);
-		if (live) {
-#pragma unroll
-			for (uint32_t s = 0; s < NV; s++) {
-				if (s < nv) {
-					vid[s] = vids[s * kLanes + lane];
-					O[s] = __ldcg(C.vert + 2 * (size_t)vid[s]);
-					D[s] = __ldcg(C.vert + 2 * (size_t)vid[s] + 1);
-				}
-			}
-#pragma unroll
-			for (uint32_t t = 0; t < NT; t++) {
-				if (t < nt) {
-					const uint32_t sl = CUBE ? (uint32_t)(cube_slot(t, 0) | cube_slot(t, 1) << 4 | cube_slot(t, 2) << 8 |
-					                                      cube_slot(t, 3) << 12)
-					                         : slots[t * kLanes + lane];
-					const float4* r = rec + t * 4 * kLanes + lane;
-					const TetRec tr = {r[0], r[kLanes], r[2 * kLanes], r[3 * kLanes]};
-					float4 Ot[4], Dt[4];
-#pragma unroll
-					for (int j = 0; j < 4; j++) {
-						Ot[j] = O[(sl >> (4 * j)) & 15u];
-						Dt[j] = D[(sl >> (4 * j)) & 15u];
-					}
-					volume_tet(mat, tr, inv_dt2, Ot, Dt);
-#pragma unroll
-					for (int j = 0; j < 4; j++) D[(sl >> (4 * j)) & 15u] = Dt[j];
-				}
-			}
-		}
-	}
-	if (next >= 0) stage_issue(C, st, (uint32_t)next, lane);  // records consumed: prefetch
-	if (live) {
-#pragma unroll
-		for (uint32_t s = 0; s < NV; s++) {
-			if (s < nv) {
-				if (last & (1u << s)) {
-					finalize_vertex(C, vid[s], O[s], D[s], inv_dt);
-					__stcg(C.vert + 2 * (size_t)vid[s], O[s]);
-				}
-				__stcg(C.vert + 2 * (size_t)vid[s] + 1, D[s]);
-			}
-		}
-	}
-}
-
-__device__ __forceinline__ void run_vol_chunk(const DevCtx& C, Stage& st, uint32_t chunk, int next, uint32_t lane,
-                                              float inv_dt, float inv_dt2, uint32_t k, bool finish) {
-	const uint4 m = __ldg(reinterpret_cast<const uint4*>(C.chunks) + chunk);
-	const uint32_t ntmax = m.z & 0xffu, nvmax = (m.z >> 8) & 0xffu;
-	if (m.z & kShapeCube)
-		vol_chunk<true>(C, st, chunk, ntmax, nvmax, next, lane, inv_dt, inv_dt2, k, finish);
-	else
-		vol_chunk<false>(C, st, chunk, ntmax, nvmax, next, lane, inv_dt, inv_dt2, k, finish);
-}
-
-// One damping pass over a resident chunk (KIND 0: element Rayleigh damping,
-// 1: PBD damping); lane = cluster, tets in the cluster's order. The state is
-// the canonical (X, V): each vertex's last solve of the substep finished it.
-// Only velocities change. CUBE: canonical cube chunks, all in registers. Not
-// inlined: the damping passes then cost the solve path no registers.
-template <bool CUBE, int KIND>
-__device__ __noinline__ void damp_chunk(const DevCtx& C, Stage& st, uint32_t ntmax, uint32_t nvmax, uint32_t trow,
-                                        int next, uint32_t lane, float inv_dt, uint32_t tick) {
-	constexpr uint32_t NV = CUBE ? 8u : kMaxClusterVerts;
-	constexpr uint32_t NT = CUBE ? 6u : kMaxClusterTets;
-	const float4* rec = reinterpret_cast<const float4*>(st.buf);
-	const uint32_t* hdrs = reinterpret_cast<const uint32_t*>(st.buf + 2048u * ntmax);
-	const uint32_t* vids = hdrs + kLanes;
-	const uint32_t* slots = vids + kLanes * nvmax;
-	const uint32_t hdr = hdrs[lane];
-	const bool live = (hdr & 15u) != 0;
-	const uint32_t nv = CUBE ? 8u : (hdr & 15u), nt = CUBE ? 6u : ((hdr >> 4) & 15u);
-	uint32_t vid[NV];
-	float4 X[NV], V[NV];
-	if (live) {
-		const BodyParams& bp = C.bodies[hdr >> 16];
-		const Mat mat = load_mat(C.bodies, hdr >> 16);
-#pragma unroll
-		for (uint32_t k = 0; k < NV; k++) {
-			if (k < nv) {
-				vid[k] = vids[k * kLanes + lane];
-				X[k] = __ldcg(C.vert + 2 * (size_t)vid[k]);
-				V[k] = __ldcg(C.vert + 2 * (size_t)vid[k] + 1);
-			}
-		}
-#pragma unroll
-		for (uint32_t t = 0; t < NT; t++) {
-			if (t < nt) {
-				const DampTet d = damp_of(C, bp, trow + t, lane, tick, KIND);
-				if (d.on) {
-					const uint32_t sl = CUBE ? (uint32_t)(cube_slot(t, 0) | cube_slot(t, 1) << 4 | cube_slot(t, 2) << 8 |
-					                                      cube_slot(t, 3) << 12)
-					                         : slots[t * kLanes + lane];
-					float4 Xt[4], Vt[4];
-#pragma unroll
-					for (int k = 0; k < 4; k++) {
-						Xt[k] = X[(sl >> (4 * k)) & 15u];
-						Vt[k] = V[(sl >> (4 * k)) & 15u];
-					}
-					if (KIND == 0) {
-						const float4* r = rec + t * 4 * kLanes + lane;
-						const TetRec tr = {r[0], r[kLanes], r[2 * kLanes], r[3 * kLanes]};
-						rayleigh_tet(mat, tr, Xt, Vt, inv_dt, d.rayleigh);
-					} else {
-						pbd_tet(Xt, Vt, d.pbd);
-					}
-#pragma unroll
-					for (int k = 0; k < 4; k++) V[(sl >> (4 * k)) & 15u] = Vt[k];
-				}
-			}
-		}
-	}
-	if (next >= 0) stage_issue(C, st, (uint32_t)next, lane);  // records consumed: prefetch
-	if (live) {
-#pragma unroll
-		for (uint32_t k = 0; k < NV; k++) {
-			if (k < nv) __stcg(C.vert + 2 * (size_t)vid[k] + 1, V[k]);
-		}
-	}
-}
-
-// kind 0: element Rayleigh damping, 1: PBD damping.
-__device__ __forceinline__ void run_damp_chunk(const DevCtx& C, Stage& st, uint32_t chunk, int next, uint32_t lane,
-                                               int kind, float inv_dt, uint32_t tick) {
-	const uint4 m = __ldg(reinterpret_cast<const uint4*>(C.chunks) + chunk);
-	const uint32_t ntmax = m.z & 0xffu, nvmax = (m.z >> 8) & 0xffu, trow = m.w;
-	if (m.z & kShapeCube) {
-		if (kind == 0)
-			damp_chunk<true, 0>(C, st, ntmax, nvmax, trow, next, lane, inv_dt, tick);
-		else
-			damp_chunk<true, 1>(C, st, ntmax, nvmax, trow, next, lane, inv_dt, tick);
-	} else {
-		if (kind == 0)
-			damp_chunk<false, 0>(C, st, ntmax, nvmax, trow, next, lane, inv_dt, tick);
-		else
-			damp_chunk<false, 1>(C, st, ntmax, nvmax, trow, next, lane, inv_dt, tick);
-	}
-}
-
-// Whether damping pass (kind index k >= 1, colour c) has work at this tick.
-__device__ __forceinline__ bool pass_on(const DevCtx& C, int dk, uint32_t c, uint32_t tick) {
-	return __ldg(C.pass_on + ((size_t)dk * 8u + tick % 8u) * C.ncolours + c) != 0;
-}
-
-// Vertices in no tet: nothing else touches them, so one thread takes each
-// through all nsub substeps at once (predict, then finalize + predict); the
-// final finalize pass closes the last one.
-// With damping sweeps the launch ends in the canonical state without a
-// closing finalize pass, so these vertices are finalized here (finalize_end).
-template <bool TAPE = false>
-__device__ __forceinline__ void run_isolated(const DevCtx& C, uint32_t begin, uint32_t step, uint32_t nsub, float dt,
-                                             float inv_dt, bool finalize_end = false) {
-	for (uint32_t i = begin; i < C.nisolated; i += step) {
-		const uint32_t v = __ldg(C.isolated + i);
-		float4 O, D;
-		ld_vertex(C.vert + 2 * (size_t)v, O, D);
-		for (uint32_t s = 0; s < nsub; s++) {
-			const float4 Dbefore = D;
-			advance_vertex(C, v, O, D, s == 0, dt, inv_dt);
-			if (TAPE) tape_vertex(C, v, O, Dbefore, s, s == 0);
-		}
-		if (finalize_end) finalize_vertex(C, v, O, D, inv_dt);
-		st_vertex(C.vert + 2 * (size_t)v, O, D);
-	}
-}
-
-template <bool TAPE = false>
-__device__ __forceinline__ void run_finalize(const DevCtx& C, uint32_t begin, uint32_t step, float inv_dt,
-                                             uint32_t nsub = 0) {
-	for (uint32_t v = begin; v < C.nverts; v += step) {
-		float4 O, D;
-		ld_vertex(C.vert + 2 * (size_t)v, O, D);
-		if (TAPE) __stcs(C.tape_fin + v, D);
-		finalize_vertex(C, v, O, D, inv_dt);
-		if (TAPE) {
-			const int q = __ldg(C.tip_of + v);
-			if (q >= 0) C.traj[(size_t)(C.sub_base + nsub - 1) * C.ntips + q] = O;
-		}
-		st_vertex(C.vert + 2 * (size_t)v, O, D);
-	}
-}
-
-// A substep is P = kinds x ncolours passes: the solve sweep over the colours,
-// the volume sweeps (DevCtx::nvol), then each damping sweep
-// (DevCtx::damp_kinds) over them again; pass q works on colour q % ncolours.
-__device__ __forceinline__ uint32_t pass_kinds(const DevCtx& C) {
-	return 1u + C.nvol + (uint32_t)__popc(C.damp_kinds);
-}
-
-// Damping kind of pass-kind index k > nvol: 0 element Rayleigh, 1 PBD.
-__device__ __forceinline__ int damp_kind(const DevCtx& C, uint32_t k) {
-	return (k == C.nvol + 1u && (C.damp_kinds & 1u)) ? 0 : 1;
-}
-
-// Whether pass q (P passes per substep) runs at `tick`: the solve and volume
-// passes always, a damping pass only if some tet of its colour is damped then.
-__device__ __forceinline__ bool pass_runs(const DevCtx& C, uint32_t q, uint32_t tick) {
-	const uint32_t kind = q / C.ncolours;
-	return kind <= C.nvol || pass_on(C, damp_kind(C, kind), q - kind * C.ncolours, tick);
-}
 
 // The warp's next chunk after `ch` (pass q of substep s, P passes per
 // substep, tick0 the launch's first tick): the next chunk of the same colour,
@@ -509,7 +88,7 @@ __global__ void __launch_bounds__(256) k_persistent(DevCtx C, uint32_t nsub, flo
 		for (uint32_t i = threadIdx.x; i <= C.ncolours; i += blockDim.x) s_ccb[i] = __ldg(C.colour_chunk_begin + i);
 	__syncthreads();
 	const uint32_t* ccb = ccb_sh ? s_ccb : C.colour_chunk_begin;
-	run_isolated<TAPE>(C, gtid, nthreads, nsub, dt, inv_dt, dmode);
+	run_isolated<TAPE>(C, GlobalVerts{}, gtid, nthreads, nsub, dt, inv_dt, dmode);
 	uint32_t target = C.bar_base;
 	bool ok = true;
 	for (uint32_t s = 0; s < nsub && ok; s++) {
@@ -526,12 +105,12 @@ __global__ void __launch_bounds__(256) k_persistent(DevCtx C, uint32_t nsub, flo
 				}
 				const int next = next_chunk(C, s, nsub, q, P, ch, gwarp, nwarps, tick0, ccb);
 				if (!EXT || kind == 0)
-					run_chunk<LAMBDAS, TAPE, EXT>(C, st, ch, next, lane, dmode || s == 0, dt, inv_dt, inv_dt2, s,
+					run_chunk<LAMBDAS, TAPE, EXT>(C, GlobalVerts{}, AnyBody{}, st, ch, next, lane, dmode || s == 0, dt, inv_dt, inv_dt2, s,
 					                               dmode);
 				else if (kind <= C.nvol)
-					run_vol_chunk(C, st, ch, next, lane, inv_dt, inv_dt2, kind, dmode);
+					run_vol_chunk(C, GlobalVerts{}, st, ch, next, lane, inv_dt, inv_dt2, kind, dmode);
 				else
-					run_damp_chunk(C, st, ch, next, lane, damp_kind(C, kind), inv_dt, tick0 + s);
+					run_damp_chunk(C, GlobalVerts{}, st, next, lane, damp_kind(C, kind), inv_dt, tick0 + s);
 			}
 			if (!grid_sync(C, target)) ok = false;
 		}
@@ -541,7 +120,7 @@ __global__ void __launch_bounds__(256) k_persistent(DevCtx C, uint32_t nsub, flo
 		if (st.inflight >= 0) mbar_wait(C, st.mbar, st.parity);
 		return;
 	}
-	if (!dmode) run_finalize<TAPE>(C, gtid, nthreads, inv_dt, nsub);
+	if (!dmode) run_finalize<TAPE>(C, GlobalVerts{}, gtid, C.nverts, nthreads, inv_dt, nsub);
 	if (gtid == 0) *C.tick = tick0 + nsub;
 }
 
@@ -600,7 +179,7 @@ __global__ void __launch_bounds__(256) k_dataflow(DevCtx C, uint32_t nsub, float
 	const uint32_t gtid = blockIdx.x * blockDim.x + threadIdx.x, nthreads = gridDim.x * blockDim.x;
 	const uint32_t tick0 = __ldcg(C.tick);
 	Stage st = stage_init(C, lane);
-	run_isolated(C, gtid, nthreads, nsub, dt, inv_dt);
+	run_isolated(C, GlobalVerts{}, gtid, nthreads, nsub, dt, inv_dt);
 	bool ok = true;
 	for (uint32_t s = 0; s < nsub && ok; s++) {
 		for (uint32_t c = 0; c < C.ncolours && ok; c++) {
@@ -612,7 +191,7 @@ __global__ void __launch_bounds__(256) k_dataflow(DevCtx C, uint32_t nsub, float
 					ok = false;
 					break;
 				}
-				run_chunk<LAMBDAS>(C, st, ch, next, lane, s == 0, dt, inv_dt, inv_dt2);
+				run_chunk<LAMBDAS>(C, GlobalVerts{}, AnyBody{}, st, ch, next, lane, s == 0, dt, inv_dt, inv_dt2);
 				__syncwarp();
 				if (lane == 0) {
 					__threadfence();
@@ -627,7 +206,7 @@ __global__ void __launch_bounds__(256) k_dataflow(DevCtx C, uint32_t nsub, float
 	}
 	uint32_t target = C.bar_base;
 	if (!grid_sync(C, target) || !ok) return;
-	run_finalize(C, gtid, nthreads, inv_dt);
+	run_finalize(C, GlobalVerts{}, gtid, C.nverts, nthreads, inv_dt);
 	if (gtid == 0) *C.tick = tick0 + nsub;
 }
 
@@ -843,7 +422,7 @@ __global__ void __launch_bounds__(256) k_bricks(DevCtx C, uint32_t nsub, float d
 	}
 	__syncthreads();
 	// vertices in no tet, finalized here too (no closing pass over all vertices)
-	run_isolated(C, gtid, nthreads, nsub, dt, inv_dt, true);
+	run_isolated(C, GlobalVerts{}, gtid, nthreads, nsub, dt, inv_dt, true);
 	const uint32_t nb0 = __ldg(C.bnb_begin + b), nb1 = __ldg(C.bnb_begin + b + 1);
 	// A pass: the warps whose chunk holds only interior clusters (every vertex
 	// private) start at once; a warp with a boundary cluster first waits
@@ -924,7 +503,7 @@ __global__ void __launch_bounds__(256, 1) k_colour(DevCtx C, uint32_t colour, in
 	const float inv_dt = 1.0f / dt, inv_dt2 = 1.0f / (dt * dt);
 	if (blockIdx.x >= solve_blocks) {
 		const uint32_t b = blockIdx.x - solve_blocks, nb = gridDim.x - solve_blocks;
-		run_isolated(C, b * blockDim.x + threadIdx.x, nb * blockDim.x, nsub, dt, inv_dt, EXT && C.damp_kinds != 0u);
+		run_isolated(C, GlobalVerts{}, b * blockDim.x + threadIdx.x, nb * blockDim.x, nsub, dt, inv_dt, EXT && C.damp_kinds != 0u);
 		return;
 	}
 	const uint32_t lane = threadIdx.x & 31u;
@@ -940,15 +519,15 @@ __global__ void __launch_bounds__(256, 1) k_colour(DevCtx C, uint32_t colour, in
 	if (!stage_acquire(C, st, ch, lane)) return;
 	const bool dmode = EXT && C.damp_kinds != 0u;
 	if (!EXT || kind == 0)
-		run_chunk<LAMBDAS, false, EXT>(C, st, ch, -1, lane, first != 0, dt, inv_dt, inv_dt2, 0, dmode);
+		run_chunk<LAMBDAS, false, EXT>(C, GlobalVerts{}, AnyBody{}, st, ch, -1, lane, first != 0, dt, inv_dt, inv_dt2, 0, dmode);
 	else if (!damp_pass)
-		run_vol_chunk(C, st, ch, -1, lane, inv_dt, inv_dt2, kind, dmode);
+		run_vol_chunk(C, GlobalVerts{}, st, ch, -1, lane, inv_dt, inv_dt2, kind, dmode);
 	else
-		run_damp_chunk(C, st, ch, -1, lane, dk, inv_dt, tick);
+		run_damp_chunk(C, GlobalVerts{}, st, -1, lane, dk, inv_dt, tick);
 }
 
 __global__ void k_finalize(DevCtx C, float dt) {
-	run_finalize(C, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x, 1.0f / dt);
+	run_finalize(C, GlobalVerts{}, blockIdx.x * blockDim.x + threadIdx.x, C.nverts, gridDim.x * blockDim.x, 1.0f / dt);
 }
 
 // Advances the tick word by a call's substeps (CUDA-graph mode).
@@ -1144,6 +723,9 @@ int launch_substeps(const DevCtx& ctx, const LaunchCfg& cfg, uint32_t nsub, floa
 		}
 		return 0;
 	}
+	// the hooks that make grid-barrier waits run out or wrap need that barrier
+	if (cfg.sync_mode == 1 && cfg.cluster.blocks && !ctx.wait_miss && !ctx.bar_base)
+		return launch_cluster(ctx, cfg.cluster, cfg.block, false, cfg.ext, nsub, dt, stream);
 	if (cfg.sync_mode == 1 || cfg.sync_mode == 3) {
 		e = reset_barrier(ctx, st);
 		if (e == cudaSuccess && cfg.sync_mode == 3) e = cudaMemsetAsync(ctx.done, 0, sizeof(uint32_t) * ctx.nchunks, st);
@@ -1194,9 +776,16 @@ int launch_substeps(const DevCtx& ctx, const LaunchCfg& cfg, uint32_t nsub, floa
 // The recording forward: k_persistent with the tape writes compiled in. The
 // arithmetic is the same inlined code as the plain launch, so the trajectory
 // is the plain launch's bit for bit.
-int launch_substeps_tape(const DevCtx& ctx, int block, uint32_t warp_smem, uint32_t nsub, float dt, void* stream) {
+int launch_substeps_tape(const DevCtx& ctx, int block, uint32_t warp_smem, uint32_t max_colour_chunks, uint32_t nsub,
+                         float dt, void* stream) {
 	if (nsub == 0) return 0;
 	cudaStream_t st = (cudaStream_t)stream;
+	ClusterPlan plan;
+	if (!ctx.wait_miss && !ctx.bar_base) {
+		const int ec = cluster_plan(ctx, max_colour_chunks, block, true, false, &plan);
+		if (ec) return ec;
+	}
+	if (plan.blocks) return launch_cluster(ctx, plan, block, true, false, nsub, dt, stream);
 	const void* f = (const void*)k_persistent<false, true>;
 	const size_t smem = solve_smem_bytes(block, warp_smem);
 	cudaError_t e = set_smem_attr(f, smem);
