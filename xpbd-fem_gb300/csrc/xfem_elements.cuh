@@ -225,8 +225,14 @@ template <class E>
 __global__ void __launch_bounds__(256, E::kMinBlocks) k_elements(DevCtx C, uint32_t nsub, float dt) {
 	const float inv_dt = 1.0f / dt, inv_dt2 = 1.0f / (dt * dt);
 	const uint32_t gtid = blockIdx.x * blockDim.x + threadIdx.x, nthreads = gridDim.x * blockDim.x;
-	// the element loops run over units: threads, or warps (warp-uniform i)
-	const uint32_t unit = E::kWarp ? gtid >> 5 : gtid, nunits = E::kWarp ? nthreads >> 5 : nthreads;
+	// the element loops run over units: threads, or warps (warp-uniform i);
+	// consecutive warps' worth of elements go to consecutive blocks, so that a
+	// pass with fewer elements than threads still spreads over every SM
+	// (230,400 T10s, about 10,000 per colour, sat on 39 of 152 SMs: 6,019 ->
+	// 4,202 us per frame; 262,144 hexes 1,042 -> 975; 28,800 H27s 3,089 -> 2,931)
+	const uint32_t gwarp = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+	const uint32_t unit = E::kWarp ? gwarp : gwarp * 32u + (threadIdx.x & 31u);
+	const uint32_t nunits = E::kWarp ? nthreads >> 5 : nthreads;
 	const uint32_t tick0 = __ldcg(C.tick);
 	const bool dmode = C.damp_kinds != 0u;
 	uint32_t target = C.bar_base;

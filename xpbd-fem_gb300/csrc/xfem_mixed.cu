@@ -62,6 +62,8 @@ __device__ __forceinline__ const BodyParams& body_of_mt(const DevCtx& C, uint32_
 __global__ void __launch_bounds__(256) k_mixed(DevCtx C, uint32_t nsub, float dt) {
 	const float inv_dt = 1.0f / dt, inv_dt2 = 1.0f / (dt * dt);
 	const uint32_t gtid = blockIdx.x * blockDim.x + threadIdx.x, nthreads = gridDim.x * blockDim.x;
+	// elements go to the blocks a warp's worth at a time, so that a small colour spreads over every SM
+	const uint32_t unit = ((threadIdx.x >> 5) * gridDim.x + blockIdx.x) * 32u + (threadIdx.x & 31u);
 	const uint32_t tick0 = __ldcg(C.tick);
 	const bool dmode = C.damp_kinds != 0u;
 	uint32_t target = C.bar_base;
@@ -77,7 +79,7 @@ __global__ void __launch_bounds__(256) k_mixed(DevCtx C, uint32_t nsub, float dt
 		for (uint32_t it = 0; it <= C.nvol; it++) {
 			for (uint32_t c = 0; c < C.mt_colours; c++) {
 				const uint32_t b = __ldg(C.colour_mt_begin + c), e = __ldg(C.colour_mt_begin + c + 1);
-				for (uint32_t i = b + gtid; i < e; i += nthreads) {
+				for (uint32_t i = b + unit; i < e; i += nthreads) {
 					if (it == 0)
 						mixed_tet_pass<kSolve>(C, i, inv_dt, inv_dt2, 0.0f);
 					else if (it <= __ldg(&body_of_mt(C, i).volume_passes))
@@ -87,7 +89,7 @@ __global__ void __launch_bounds__(256) k_mixed(DevCtx C, uint32_t nsub, float dt
 			}
 			for (uint32_t c = 0; c < C.el_colours; c++) {
 				const uint32_t b = __ldg(C.colour_el_begin + c), e = __ldg(C.colour_el_begin + c + 1);
-				for (uint32_t i = b + gtid; i < e; i += nthreads) {
+				for (uint32_t i = b + unit; i < e; i += nthreads) {
 					if (it == 0)
 						hex_pass<kSolve>(C, i, inv_dt, inv_dt2, 0.0f);
 					else if (it <= __ldg(&body_of_el<HexElem>(C, i).volume_passes))
@@ -108,7 +110,7 @@ __global__ void __launch_bounds__(256) k_mixed(DevCtx C, uint32_t nsub, float dt
 		if (C.damp_kinds & 1u) {
 			for (uint32_t c = 0; c < C.mt_colours; c++) {
 				const uint32_t b = __ldg(C.colour_mt_begin + c), e = __ldg(C.colour_mt_begin + c + 1);
-				for (uint32_t i = b + gtid; i < e; i += nthreads) {
+				for (uint32_t i = b + unit; i < e; i += nthreads) {
 					const BodyParams& bp = body_of_mt(C, i);
 					const uint32_t type = __ldg(&bp.rayleigh_type);
 					const float rd = __ldg(&bp.damping) * (type == 3u ? 8.0f : 1.0f);
@@ -119,7 +121,7 @@ __global__ void __launch_bounds__(256) k_mixed(DevCtx C, uint32_t nsub, float dt
 			}
 			for (uint32_t c = 0; c < C.el_colours; c++) {
 				const uint32_t b = __ldg(C.colour_el_begin + c), e = __ldg(C.colour_el_begin + c + 1);
-				for (uint32_t i = b + gtid; i < e; i += nthreads) {
+				for (uint32_t i = b + unit; i < e; i += nthreads) {
 					const BodyParams& bp = body_of_el<HexElem>(C, i);
 					const uint32_t type = __ldg(&bp.rayleigh_type);
 					const float rd = __ldg(&bp.damping) * (type == 3u ? 8.0f : 1.0f);
@@ -132,7 +134,7 @@ __global__ void __launch_bounds__(256) k_mixed(DevCtx C, uint32_t nsub, float dt
 		if (C.damp_kinds & 2u) {
 			for (uint32_t c = 0; c < C.mt_colours; c++) {
 				const uint32_t b = __ldg(C.colour_mt_begin + c), e = __ldg(C.colour_mt_begin + c + 1);
-				for (uint32_t i = b + gtid; i < e; i += nthreads) {
+				for (uint32_t i = b + unit; i < e; i += nthreads) {
 					const BodyParams& bp = body_of_mt(C, i);
 					if (!__ldg(&bp.pbd_on) || !in_slice_of(bp, __ldg(C.mt_flat + i), __ldg(&bp.ntets), tick)) continue;
 					const float coeff = __ldg(&bp.rayleigh_type) == 3u ? __ldg(&bp.pbd_coeff_amortized) : __ldg(&bp.pbd_coeff);
@@ -144,7 +146,7 @@ __global__ void __launch_bounds__(256) k_mixed(DevCtx C, uint32_t nsub, float dt
 			}
 			for (uint32_t c = 0; c < C.el_colours; c++) {
 				const uint32_t b = __ldg(C.colour_el_begin + c), e = __ldg(C.colour_el_begin + c + 1);
-				for (uint32_t i = b + gtid; i < e; i += nthreads) {
+				for (uint32_t i = b + unit; i < e; i += nthreads) {
 					const BodyParams& bp = body_of_el<HexElem>(C, i);
 					if (__ldg(&bp.pbd_on) && in_slice_of(bp, __ldg(C.el_flat + i), __ldg(&bp.nhexes), tick))
 						hex_pbd_inl(C, i, __ldg(&bp.rayleigh_type) == 3u ? __ldg(&bp.pbd_coeff_amortized) : __ldg(&bp.pbd_coeff));

@@ -31,9 +31,12 @@ __device__ __forceinline__ bool in_slice_n(const DevCtx& C, const BodyParams& bp
 // One pass kind over the colours of one element kind (units: threads for
 // T10s, warps for H27s); false when a barrier gave up.
 template <class E, int KIND>
-__device__ __forceinline__ bool sweep(const DevCtx& C, const DevCtx& B, uint32_t gtid, uint32_t nthreads, float inv_dt,
-                                      float inv_dt2, uint32_t it, uint32_t tick, uint32_t& target) {
-	const uint32_t unit = E::kWarp ? gtid >> 5 : gtid, nunits = E::kWarp ? nthreads >> 5 : nthreads;
+__device__ __forceinline__ bool sweep(const DevCtx& C, const DevCtx& B, uint32_t nthreads, float inv_dt, float inv_dt2,
+                                      uint32_t it, uint32_t tick, uint32_t& target) {
+	// a warp's worth of elements at a time to each block, as in k_elements
+	const uint32_t gwarp = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+	const uint32_t unit = E::kWarp ? gwarp : gwarp * 32u + (threadIdx.x & 31u);
+	const uint32_t nunits = E::kWarp ? nthreads >> 5 : nthreads;
 	for (uint32_t c = 0; c < C.el_colours; c++) {
 		const uint32_t b = __ldg(C.colour_el_begin + c), e = __ldg(C.colour_el_begin + c + 1);
 		for (uint32_t i = b + unit; i < e; i += nunits) {
@@ -76,11 +79,11 @@ __global__ void __launch_bounds__(256, 1) k_qmixed(DevCtx Ch, DevCtx Ct, uint32_
 		}
 		if (!grid_sync(Ch, target)) return;
 		const uint32_t tick = tick0 + s;
-		if (!sweep<T10, kSolve>(Ct, Ch, gtid, nthreads, inv_dt, inv_dt2, 0, tick, target)) return;
-		if (!sweep<H27, kSolve>(Ch, Ch, gtid, nthreads, inv_dt, inv_dt2, 0, tick, target)) return;
+		if (!sweep<T10, kSolve>(Ct, Ch, nthreads, inv_dt, inv_dt2, 0, tick, target)) return;
+		if (!sweep<H27, kSolve>(Ch, Ch, nthreads, inv_dt, inv_dt2, 0, tick, target)) return;
 		for (uint32_t it = 0; it < Ch.nvol; it++) {
-			if (!sweep<T10, kVolume>(Ct, Ch, gtid, nthreads, inv_dt, inv_dt2, it, tick, target)) return;
-			if (!sweep<H27, kVolume>(Ch, Ch, gtid, nthreads, inv_dt, inv_dt2, it, tick, target)) return;
+			if (!sweep<T10, kVolume>(Ct, Ch, nthreads, inv_dt, inv_dt2, it, tick, target)) return;
+			if (!sweep<H27, kVolume>(Ch, Ch, nthreads, inv_dt, inv_dt2, it, tick, target)) return;
 		}
 		if (!dmode) continue;
 		for (uint32_t v = gtid; v < Ch.nverts; v += nthreads) {
@@ -91,12 +94,12 @@ __global__ void __launch_bounds__(256, 1) k_qmixed(DevCtx Ch, DevCtx Ct, uint32_
 		}
 		if (!grid_sync(Ch, target)) return;
 		if (Ch.damp_kinds & 1u) {
-			if (!sweep<T10, kRayleigh>(Ct, Ch, gtid, nthreads, inv_dt, inv_dt2, 0, tick, target)) return;
-			if (!sweep<H27, kRayleigh>(Ch, Ch, gtid, nthreads, inv_dt, inv_dt2, 0, tick, target)) return;
+			if (!sweep<T10, kRayleigh>(Ct, Ch, nthreads, inv_dt, inv_dt2, 0, tick, target)) return;
+			if (!sweep<H27, kRayleigh>(Ch, Ch, nthreads, inv_dt, inv_dt2, 0, tick, target)) return;
 		}
 		if (Ch.damp_kinds & 2u) {
-			if (!sweep<T10, kPbd>(Ct, Ch, gtid, nthreads, inv_dt, inv_dt2, 0, tick, target)) return;
-			if (!sweep<H27, kPbd>(Ch, Ch, gtid, nthreads, inv_dt, inv_dt2, 0, tick, target)) return;
+			if (!sweep<T10, kPbd>(Ct, Ch, nthreads, inv_dt, inv_dt2, 0, tick, target)) return;
+			if (!sweep<H27, kPbd>(Ch, Ch, nthreads, inv_dt, inv_dt2, 0, tick, target)) return;
 		}
 	}
 	if (!dmode) {
