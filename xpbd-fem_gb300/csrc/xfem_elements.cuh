@@ -210,29 +210,53 @@ __device__ __forceinline__ bool in_slice(const DevCtx& C, const BodyParams& bp, 
 	return f >= nh * m / 8u && f < nh * (m + 1u) / 8u;
 }
 
+// Calls f(i, live) on the elements [b, e) of a colour, LANES lanes of a warp
+// per element (32 / LANES elements per warp). Consecutive warps' worth of
+// elements go to consecutive blocks, so that a pass with fewer elements than
+// threads still spreads over every SM (230,400 T10s, about 10,000 per colour,
+// one lane each, sat on 39 of 152 SMs: 6,019 -> 4,202 us per frame; 262,144
+// hexes 1,042 -> 975; 28,800 H27s 3,089 -> 2,931). With 2 to 16 lanes per
+// element every lane of the warp calls f together, a group past the end with
+// the last element and live = false.
+constexpr uint32_t kNoElem = 0xffffffffu;
+template <int LANES, class F>
+__device__ __forceinline__ void for_elements(uint32_t b, uint32_t e, F f) {
+	constexpr uint32_t n = 32u / LANES;
+	const uint32_t gwarp = (threadIdx.x >> 5) * gridDim.x + blockIdx.x, nwarps = (blockDim.x >> 5) * gridDim.x;
+	const uint32_t sub = (threadIdx.x & 31u) / LANES;
+	if constexpr (LANES == 1 || LANES == 32) {
+		for (uint32_t i = b + gwarp * n + sub; i < e; i += nwarps * n) f(i, true);
+	} else {
+		for (uint32_t i0 = b + gwarp * n; i0 < e; i0 += nwarps * n) f(min(i0 + sub, e - 1u), i0 + sub < e);
+	}
+}
+
 template <class E>
 __device__ __forceinline__ const BodyParams& body_of_el(const DevCtx& C, uint32_t i) {
 	const uint32_t v0 = __ldg(&C.el_vid[E::kVid4 * (size_t)i].x);
 	return C.bodies[__float_as_uint(__ldcg(&C.vert[2 * (size_t)v0 + 1].w)) >> 8];
 }
 
+// Whether the calling lanes have an element to work on: for elements of 2 to 16
+// lanes the whole warp decides together.
+template <class E>
+__device__ __forceinline__ bool any_live(bool live) {
+	if constexpr (E::kLanes == 1 || E::kLanes == 32)
+		return live;
+	else
+		return __any_sync(0xffffffffu, live);
+}
+
 // The persistent element kernel (cooperative launch, co-resident grid). E:
-// the element type (kVid4 uint4 of vertex ids per element; pass<KIND>, pbd;
-// kWarp: one warp per element, every lane of the warp calling with the same
-// element, else one thread per element; kMinBlocks: the blocks per SM the
-// register budget is sized for).
+// the element type (kVid4 uint4 of vertex ids per element; pass<KIND>(C, i,
+// live, ...) by kLanes lanes of a warp per element, pbd by kPbdLanes;
+// kMinBlocks: the blocks per SM the register budget is sized for; smem(), the
+// dynamic shared memory of a block, set up by init).
 template <class E>
 __global__ void __launch_bounds__(256, E::kMinBlocks) k_elements(DevCtx C, uint32_t nsub, float dt) {
 	const float inv_dt = 1.0f / dt, inv_dt2 = 1.0f / (dt * dt);
 	const uint32_t gtid = blockIdx.x * blockDim.x + threadIdx.x, nthreads = gridDim.x * blockDim.x;
-	// the element loops run over units: threads, or warps (warp-uniform i);
-	// consecutive warps' worth of elements go to consecutive blocks, so that a
-	// pass with fewer elements than threads still spreads over every SM
-	// (230,400 T10s, about 10,000 per colour, sat on 39 of 152 SMs: 6,019 ->
-	// 4,202 us per frame; 262,144 hexes 1,042 -> 975; 28,800 H27s 3,089 -> 2,931)
-	const uint32_t gwarp = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
-	const uint32_t unit = E::kWarp ? gwarp : gwarp * 32u + (threadIdx.x & 31u);
-	const uint32_t nunits = E::kWarp ? nthreads >> 5 : nthreads;
+	E::init(C);
 	const uint32_t tick0 = __ldcg(C.tick);
 	const bool dmode = C.damp_kinds != 0u;
 	uint32_t target = C.bar_base;
@@ -246,14 +270,30 @@ __global__ void __launch_bounds__(256, E::kMinBlocks) k_elements(DevCtx C, uint3
 		if (!grid_sync(C, target)) return;
 		for (uint32_t c = 0; c < C.el_colours; c++) {
 			const uint32_t b = __ldg(C.colour_el_begin + c), e = __ldg(C.colour_el_begin + c + 1);
-			for (uint32_t i = b + unit; i < e; i += nunits) E::template pass<kSolve>(C, i, inv_dt, inv_dt2, 0.0f);
+			if constexpr (E::kLanes == 32) {
+				// one warp per element: its next element is fetched ahead
+				const uint32_t gwarp = (threadIdx.x >> 5) * gridDim.x + blockIdx.x, nwarps = nthreads >> 5;
+				for (uint32_t i = b + gwarp; i < e; i += nwarps) {
+					uint32_t next = i + nwarps;
+					if (next >= e) {
+						const uint32_t c2 = c + 1 < C.el_colours ? c + 1 : 0;
+						next = __ldg(C.colour_el_begin + c2) + gwarp;
+						if (next >= __ldg(C.colour_el_begin + c2 + 1) || (c2 == 0 && s + 1 == nsub)) next = kNoElem;
+					}
+					E::template pass<kSolve>(C, i, true, inv_dt, inv_dt2, 0.0f, next);
+				}
+			} else {
+				for_elements<E::kLanes>(b, e, [&](uint32_t i, bool live) { E::template pass<kSolve>(C, i, live, inv_dt, inv_dt2, 0.0f); });
+			}
 			if (!grid_sync(C, target)) return;
 		}
 		for (uint32_t it = 0; it < C.nvol; it++)
 			for (uint32_t c = 0; c < C.el_colours; c++) {
 				const uint32_t b = __ldg(C.colour_el_begin + c), e = __ldg(C.colour_el_begin + c + 1);
-				for (uint32_t i = b + unit; i < e; i += nunits)
-					if (it < __ldg(&body_of_el<E>(C, i).volume_passes)) E::template pass<kVolume>(C, i, inv_dt, inv_dt2, 0.0f);
+				for_elements<E::kLanes>(b, e, [&](uint32_t i, bool live) {
+					live = live && it < __ldg(&body_of_el<E>(C, i).volume_passes);
+					if (any_live<E>(live)) E::template pass<kVolume>(C, i, live, inv_dt, inv_dt2, 0.0f);
+				});
 				if (!grid_sync(C, target)) return;
 			}
 		if (!dmode) continue;
@@ -268,22 +308,23 @@ __global__ void __launch_bounds__(256, E::kMinBlocks) k_elements(DevCtx C, uint3
 		if (C.damp_kinds & 1u)
 			for (uint32_t c = 0; c < C.el_colours; c++) {
 				const uint32_t b = __ldg(C.colour_el_begin + c), e = __ldg(C.colour_el_begin + c + 1);
-				for (uint32_t i = b + unit; i < e; i += nunits) {
+				for_elements<E::kLanes>(b, e, [&](uint32_t i, bool live) {
 					const BodyParams& bp = body_of_el<E>(C, i);
 					const uint32_t type = __ldg(&bp.rayleigh_type);
 					const float rd = __ldg(&bp.damping) * (type == 3u ? 8.0f : 1.0f);
-					if (type >= 2u && rd > 0.0f && in_slice(C, bp, i, tick)) E::template pass<kRayleigh>(C, i, inv_dt, inv_dt2, rd);
-				}
+					live = live && type >= 2u && rd > 0.0f && in_slice(C, bp, i, tick);
+					if (any_live<E>(live)) E::template pass<kRayleigh>(C, i, live, inv_dt, inv_dt2, rd);
+				});
 				if (!grid_sync(C, target)) return;
 			}
 		if (C.damp_kinds & 2u)
 			for (uint32_t c = 0; c < C.el_colours; c++) {
 				const uint32_t b = __ldg(C.colour_el_begin + c), e = __ldg(C.colour_el_begin + c + 1);
-				for (uint32_t i = b + unit; i < e; i += nunits) {
+				for_elements<E::kPbdLanes>(b, e, [&](uint32_t i, bool) {
 					const BodyParams& bp = body_of_el<E>(C, i);
 					if (__ldg(&bp.pbd_on) && in_slice(C, bp, i, tick))
 						E::pbd(C, i, __ldg(&bp.rayleigh_type) == 3u ? __ldg(&bp.pbd_coeff_amortized) : __ldg(&bp.pbd_coeff));
-				}
+				});
 				if (!grid_sync(C, target)) return;
 			}
 	}
@@ -306,14 +347,16 @@ int launch_elements(const DevCtx& ctx, int block, uint32_t nsub, float dt, void*
 	int dev = 0, sms = 0, per_sm = 0;
 	cudaError_t e = cudaGetDevice(&dev);
 	if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-	if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f, block, 0);
+	if (e == cudaSuccess && E::smem() > 0)
+		e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)E::smem());
+	if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f, block, E::smem());
 	if (e != cudaSuccess) return (int)e;
 	if (per_sm <= 0) return (int)cudaErrorInvalidConfiguration;
 	e = reset_barrier(ctx, st);
 	if (e != cudaSuccess) return (int)e;
 	DevCtx c = ctx;
 	void* args[] = {&c, &nsub, &dt};
-	return (int)cudaLaunchCooperativeKernel(f, dim3(per_sm * sms), dim3(block), args, 0, st);
+	return (int)cudaLaunchCooperativeKernel(f, dim3(per_sm * sms), dim3(block), args, E::smem(), st);
 }
 
 

@@ -12,7 +12,7 @@
 // its share of the prefactored I1, its gradient rows, its update); lane p
 // owns quadrature point p when the deformation gradients are formed. The
 // node offsets P and each point's G Ji (the energy gradient mapped back to
-// the reference frame) pass between the two through 2.2 KB of shared memory
+// the reference frame) pass between the two through 3 KB of shared memory
 // per warp, next to the warp's copy of the element's record. Sums over lanes
 // are xor butterflies, so every lane holds the same bits and every lane takes
 // the same branch.
@@ -52,7 +52,7 @@ struct H27RingScratch {
 };
 
 template <bool DAMP, bool VMODE>
-__device__ __forceinline__ void h27_ring_solve(const DevCtx& C, H27RingScratch& S, uint32_t r, uint32_t lane,
+__device__ __forceinline__ void h27_ring_solve(const DevCtx& C, H27RingScratch& S, const Tables& T, uint32_t r, uint32_t lane,
                                                float inv_dt, float inv_dt2, uint32_t tick) {
 	__syncwarp();  // every lane is done with the previous ring's scratch
 	const uint4 h = __ldg(C.ring_hdr + r);
@@ -99,9 +99,11 @@ __device__ __forceinline__ void h27_ring_solve(const DevCtx& C, H27RingScratch& 
 		__syncwarp();  // the previous H27's record and point terms are consumed
 		const float4* src = C.el_rec + (size_t)ei * (kRec / 4);
 		for (uint32_t k = lane; k < kRec / 4; k += 32) S.el.rec[k] = __ldg(src + k);
+		if (lane == 0) S.el.have = kNoElem;  // the PBD passes fetch their own
 		__syncwarp();
 		Elem E;
 		E.lane = lane;
+		E.T = &T;
 		E.R = reinterpret_cast<const float*>(S.el.rec);
 		E.O = E.D = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 		E.w = 0.0f;
@@ -117,15 +119,17 @@ __device__ __forceinline__ void h27_ring_solve(const DevCtx& C, H27RingScratch& 
 		Vec3 g0, g1;
 		if (e == 10u) {
 			points<kDev>(C, S.el, E, 1, bp, e, a, u0, u1, ew, true);
-			g0 = root(E, gather(C, S.el.M0, E, 1));
-			U0 += wsum(u0);
+			g0 = root_u(E, gather(S.el.M0, E, 1), u0);
+			U0 += u0;
 		} else {
-			U0 = fmaf(ew, pref_i1(S.el, E, g0), U0);
+			float up = pref_row(S.el, E, g0);
+			g0 = root_u(E, g0, up);
+			U0 = fmaf(ew, up, U0);
 			g0 = {ew * g0.x, ew * g0.y, ew * g0.z};
 		}
 		points<kHydro>(C, S.el, E, 0, bp, e, a, u0, u1, ew, false);
-		g1 = root(E, gather(C, S.el.M1, E, 0));
-		U1 += wsum(u1);
+		g1 = root_u(E, gather(S.el.M1, E, 0), u1);
+		U1 += u1;
 		if (lane < 27) {
 			S.g0[slot][0] += g0.x;
 			S.g0[slot][1] += g0.y;
@@ -174,7 +178,10 @@ __global__ void __launch_bounds__(128) k_h27_rings(DevCtx C, uint32_t nsub, floa
 	const uint32_t lane = threadIdx.x & 31u, wib = threadIdx.x >> 5;
 	const uint32_t gwarp = wib * gridDim.x + blockIdx.x, nwarps = (blockDim.x >> 5) * gridDim.x;
 	const uint32_t gtid = blockIdx.x * blockDim.x + threadIdx.x, nthreads = gridDim.x * blockDim.x;
-	H27RingScratch& S = reinterpret_cast<H27RingScratch*>(smem)[wib];
+	Tables& T = *reinterpret_cast<Tables*>(smem);
+	H27RingScratch& S = reinterpret_cast<H27RingScratch*>(smem + sizeof(Tables))[wib];
+	if (lane == 0) S.el.have = kNoElem;
+	load_tables(C, T);
 	const uint32_t tick0 = __ldcg(C.tick);
 	const bool dmode = DAMP && C.damp_kinds != 0u;
 	uint32_t target = C.bar_base;
@@ -188,7 +195,7 @@ __global__ void __launch_bounds__(128) k_h27_rings(DevCtx C, uint32_t nsub, floa
 		if (!grid_sync(C, target)) return;
 		for (uint32_t c = 0; c < C.ring_colours; c++) {
 			const uint32_t rb = __ldg(C.colour_ring_begin + c), re = __ldg(C.colour_ring_begin + c + 1);
-			for (uint32_t r = rb + gwarp; r < re; r += nwarps) h27_ring_solve<DAMP, false>(C, S, r, lane, inv_dt, inv_dt2, 0);
+			for (uint32_t r = rb + gwarp; r < re; r += nwarps) h27_ring_solve<DAMP, false>(C, S, T, r, lane, inv_dt, inv_dt2, 0);
 			if (!grid_sync(C, target)) return;
 		}
 		if (!dmode) continue;
@@ -205,7 +212,7 @@ __global__ void __launch_bounds__(128) k_h27_rings(DevCtx C, uint32_t nsub, floa
 				for (uint32_t c = 0; c < C.ring_colours; c++) {
 					const uint32_t rb = __ldg(C.colour_ring_begin + c), re = __ldg(C.colour_ring_begin + c + 1);
 					for (uint32_t r = rb + gwarp; r < re; r += nwarps)
-						h27_ring_solve<true, true>(C, S, r, lane, inv_dt, inv_dt2, tick);
+						h27_ring_solve<true, true>(C, S, T, r, lane, inv_dt, inv_dt2, tick);
 					if (!grid_sync(C, target)) return;
 				}
 			if (C.damp_kinds & 2u)
@@ -217,7 +224,7 @@ __global__ void __launch_bounds__(128) k_h27_rings(DevCtx C, uint32_t nsub, floa
 							const float coeff =
 							    __ldg(&bp.rayleigh_type) == 3u ? __ldg(&bp.pbd_coeff_amortized) : __ldg(&bp.pbd_coeff);
 							__syncwarp();  // the scratch's last readers are done
-							h27_pbd_in(C, S.el, i, coeff);
+							h27_pbd_in(C, S.el, T, i, coeff);
 						}
 					}
 					if (!grid_sync(C, target)) return;
@@ -241,7 +248,7 @@ int launch_h27_rings(const DevCtx& ctx, int block, uint32_t nsub, float dt, void
 	if (nsub == 0) return 0;
 	cudaStream_t st = (cudaStream_t)stream;
 	const void* f = ctx.ext ? (const void*)k_h27_rings<true> : (const void*)k_h27_rings<false>;
-	const size_t smem = (size_t)(block / 32) * sizeof(H27RingScratch);
+	const size_t smem = sizeof(Tables) + (size_t)(block / 32) * sizeof(H27RingScratch);
 	int dev = 0, sms = 0, per_sm = 0;
 	cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
 	if (e == cudaSuccess) e = cudaGetDevice(&dev);

@@ -13,10 +13,17 @@
 // its share of the prefactored I1, its gradient rows, its update); lane p
 // owns quadrature point p when the deformation gradients are formed. The
 // node offsets P and each point's G Ji (the energy gradient mapped back to
-// the reference frame) pass between the two through 2.2 KB of shared memory
+// the reference frame) pass between the two through 3 KB of shared memory
 // per warp, next to the warp's copy of the element's record. Sums over lanes
 // are xor butterflies, so every lane holds the same bits and every lane takes
 // the same branch.
+//
+// A pass is one warp's chain of some 1,300 instructions with 24 warps per SM.
+// What shortened it (28,800 H27s, 20 substeps, 2,931 -> 1,763 us): the
+// gradient tables in shared memory in the order each phase reads them, node
+// offsets as one 16-byte read, three lanes per point on the 8-point rule, the
+// prefactored row without branches, eight sums in one butterfly, and the next
+// element's record and ids fetched while the pass ends.
 //
 // Records: 704 floats per H27 (the 703 of the reference's flattening, one
 // pad), element-major, read by every lane of the element's warp. The
@@ -42,18 +49,60 @@ __device__ __forceinline__ float wsum(float v) {
 	return v;
 }
 
+// N sums at once: their butterflies' latencies overlap.
+template <int N>
+__device__ __forceinline__ void wsums(float (&v)[N]) {
+#pragma unroll
+	for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+		for (int k = 0; k < N; k++) v[k] += __shfl_xor_sync(kAll, v[k], o);
+}
+
+// The gradient tables in shared memory, once per block: by node and point (a
+// lane per point reads a node's row), and by point, axis and node (a lane per
+// node reads a point's rows).
+struct Tables {
+	float4 a8[26][8], a27[26][27];
+	float b8[8][3][32], b27[27][3][32];
+};
+
+__device__ __forceinline__ float tab(const DevCtx& C, int hi, int p, int n, int k) {
+	return __ldg(C.el_tab + (hi ? kTab27 : kTab8) + (p * 27 + n) * 3 + k);
+}
+
+__device__ __forceinline__ void load_tables(const DevCtx& C, Tables& T) {
+	for (uint32_t i = threadIdx.x; i < 27u * 32u; i += blockDim.x) {
+		const int p = (int)(i / 32u), n = (int)(i % 32u);
+		const float x = n < 27 ? tab(C, 1, p, n, 0) : 0.0f, y = n < 27 ? tab(C, 1, p, n, 1) : 0.0f,
+		            z = n < 27 ? tab(C, 1, p, n, 2) : 0.0f;
+		T.b27[p][0][n] = x, T.b27[p][1][n] = y, T.b27[p][2][n] = z;
+		if (n < 26) T.a27[n][p] = make_float4(x, y, z, 0.0f);
+		if (p < 8) {
+			const float u = n < 27 ? tab(C, 0, p, n, 0) : 0.0f, v = n < 27 ? tab(C, 0, p, n, 1) : 0.0f,
+			            w = n < 27 ? tab(C, 0, p, n, 2) : 0.0f;
+			T.b8[p][0][n] = u, T.b8[p][1][n] = v, T.b8[p][2][n] = w;
+			if (n < 26) T.a8[n][p] = make_float4(u, v, w, 0.0f);
+		}
+	}
+	__syncthreads();
+}
+
 // per-warp scratch: the element's record (copied in once per element, so
-// the lanes' scattered reads of it wait on shared memory, not on L2), node
-// offsets from node 26, and each point's G Ji for the first and the second
-// constraint
+// the lanes' scattered reads of it wait on shared memory, not on L2) and
+// vertex ids, node offsets from node 26, and each point's G Ji, a row of three
+// per axis, for the first and the second constraint
 struct Scratch {
 	float4 rec[kRec / 4];
-	float P[26][3];
-	float M0[27][9], M1[27][9];
+	uint32_t vid[28];
+	uint32_t have;  // the element whose record and ids are here or on their way
+	uint32_t pad[3];
+	float4 P[26];
+	float4 M0[27][3], M1[27][3];
 };
 
 struct Elem {
 	const float* R;  // the record (this warp's shared copy)
+	const Tables* T;
 	uint32_t lane;
 	float4 O, D;  // this lane's node (lanes >= 27: zero)
 	float w;
@@ -67,16 +116,11 @@ __device__ __forceinline__ void share_rel(Scratch& s, const Elem& E, bool vmode)
 	const float ox = __shfl_sync(kAll, E.O.x, 26), oy = __shfl_sync(kAll, E.O.y, 26), oz = __shfl_sync(kAll, E.O.z, 26);
 	const float dx = __shfl_sync(kAll, E.D.x, 26), dy = __shfl_sync(kAll, E.D.y, 26), dz = __shfl_sync(kAll, E.D.z, 26);
 	__syncwarp();
-	if (E.lane < 26) {
-		s.P[E.lane][0] = vmode ? E.O.x - ox : (E.O.x - ox) + (E.D.x - dx);
-		s.P[E.lane][1] = vmode ? E.O.y - oy : (E.O.y - oy) + (E.D.y - dy);
-		s.P[E.lane][2] = vmode ? E.O.z - oz : (E.O.z - oz) + (E.D.z - dz);
-	}
+	if (E.lane < 26)
+		s.P[E.lane] = vmode ? make_float4(E.O.x - ox, E.O.y - oy, E.O.z - oz, 0.0f)
+		                    : make_float4((E.O.x - ox) + (E.D.x - dx), (E.O.y - oy) + (E.D.y - dy),
+		                                  (E.O.z - oz) + (E.D.z - dz), 0.0f);
 	__syncwarp();
-}
-
-__device__ __forceinline__ float tab(const DevCtx& C, int hi, int p, int n, int k) {
-	return __ldg(C.el_tab + (hi ? kTab27 : kTab8) + (p * 27 + n) * 3 + k);
 }
 
 __device__ __forceinline__ float trace_xtx(const float F[3][3]) {
@@ -103,34 +147,53 @@ template <int TERM>
 __device__ __forceinline__ void points(const DevCtx& C, Scratch& s, const Elem& E, int hi, const BodyParams& bp,
                                        uint32_t e, float a, float& u0, float& u1, float wscale = 1.0f,
                                        bool skin = false) {
-	const int np = hi ? 27 : 8;
 	u0 = u1 = 0.0f;
-	const int p = (int)E.lane;
-	if (p < np) {
-		float Ji[3][3];
-		const int jb = (hi ? kJH : kJL) + 9 * p;
+	// On the 27 points a lane takes one; on the 8 points three lanes share one,
+	// lane p + 8 c forming column c of its F and row c of its G Ji.
+	const int p = hi ? (int)E.lane : (int)(E.lane & 7u), own = hi ? 0 : (int)(E.lane >> 3);
+	float Ji[3][3], F[3][3], A[3][3], G0[3][3], G1[3][3];
+	const bool on = E.lane < (hi ? 27u : 24u);
+	{
+		const int pj = on ? p : 0, jb = (hi ? kJH : kJL) + 9 * pj;
 #pragma unroll
 		for (int c = 0; c < 3; c++)
 #pragma unroll
 			for (int r = 0; r < 3; r++) Ji[c][r] = rec(E, jb + 3 * c + r);
-		const float wt = wscale * rec(E, (hi ? kWH : kWL) + p);
-		float Dm[3][3] = {{0.0f, 0.0f, 0.0f}, {0.0f, 0.0f, 0.0f}, {0.0f, 0.0f, 0.0f}};
+		if (hi) {
+			float Dm[3][3] = {{0.0f, 0.0f, 0.0f}, {0.0f, 0.0f, 0.0f}, {0.0f, 0.0f, 0.0f}};
 #pragma unroll 2
-		for (int n = 0; n < 26; n++) {
-			const float px = s.P[n][0], py = s.P[n][1], pz = s.P[n][2];
-#pragma unroll
-			for (int r = 0; r < 3; r++) {
-				const float d = tab(C, hi, p, n, r);
-				Dm[0][r] = fmaf(d, px, Dm[0][r]);
-				Dm[1][r] = fmaf(d, py, Dm[1][r]);
-				Dm[2][r] = fmaf(d, pz, Dm[2][r]);
+			for (int n = 0; n < 26; n++) {
+				const float4 x = s.P[n], d = E.T->a27[n][pj];
+				Dm[0][0] = fmaf(d.x, x.x, Dm[0][0]), Dm[1][0] = fmaf(d.x, x.y, Dm[1][0]), Dm[2][0] = fmaf(d.x, x.z, Dm[2][0]);
+				Dm[0][1] = fmaf(d.y, x.x, Dm[0][1]), Dm[1][1] = fmaf(d.y, x.y, Dm[1][1]), Dm[2][1] = fmaf(d.y, x.z, Dm[2][1]);
+				Dm[0][2] = fmaf(d.z, x.x, Dm[0][2]), Dm[1][2] = fmaf(d.z, x.y, Dm[1][2]), Dm[2][2] = fmaf(d.z, x.z, Dm[2][2]);
 			}
+#pragma unroll
+			for (int c = 0; c < 3; c++)
+#pragma unroll
+				for (int r = 0; r < 3; r++) F[c][r] = fmaf(Ji[0][r], Dm[c][0], fmaf(Ji[1][r], Dm[c][1], Ji[2][r] * Dm[c][2]));
+		} else {
+			const float* Pc = reinterpret_cast<const float*>(s.P) + (own < 3 ? own : 0);
+			float Dm[3] = {0.0f, 0.0f, 0.0f};
+#pragma unroll
+			for (int n = 0; n < 26; n++) {
+				const float x = Pc[4 * n];
+				const float4 d = E.T->a8[n][p];
+				Dm[0] = fmaf(d.x, x, Dm[0]);
+				Dm[1] = fmaf(d.y, x, Dm[1]);
+				Dm[2] = fmaf(d.z, x, Dm[2]);
+			}
+			float Fc[3];
+#pragma unroll
+			for (int r = 0; r < 3; r++) Fc[r] = fmaf(Ji[0][r], Dm[0], fmaf(Ji[1][r], Dm[1], Ji[2][r] * Dm[2]));
+#pragma unroll
+			for (int c = 0; c < 3; c++)
+#pragma unroll
+				for (int r = 0; r < 3; r++) F[c][r] = __shfl_sync(kAll, Fc[r], p + 8 * c);
 		}
-		float F[3][3], A[3][3], G0[3][3], G1[3][3];
-#pragma unroll
-		for (int c = 0; c < 3; c++)
-#pragma unroll
-			for (int r = 0; r < 3; r++) F[c][r] = fmaf(Ji[0][r], Dm[c][0], fmaf(Ji[1][r], Dm[c][1], Ji[2][r] * Dm[c][2]));
+	}
+	if (on) {
+		const float wt = wscale * rec(E, (hi ? kWH : kWL) + p);
 		const float J = adj_det(F, A);
 		const float Ja = J - a;
 		if (TERM == kHydro || TERM == kDevHydro) {
@@ -169,72 +232,111 @@ __device__ __forceinline__ void points(const DevCtx& C, Scratch& s, const Elem& 
 				for (int r = 0; r < 3; r++) G0[c][r] = F[r][c] * sc;
 		}
 		// M[j][r] = sum_k G[k][r] Ji[j][k]
-		if (TERM != kHydro)
+		auto row = [&](const float G[3][3], const float J[3]) {
+			return make_float4(fmaf(G[0][0], J[0], fmaf(G[1][0], J[1], G[2][0] * J[2])),
+			                   fmaf(G[0][1], J[0], fmaf(G[1][1], J[1], G[2][1] * J[2])),
+			                   fmaf(G[0][2], J[0], fmaf(G[1][2], J[1], G[2][2] * J[2])), 0.0f);
+		};
+		if (hi) {
 #pragma unroll
-			for (int j = 0; j < 3; j++)
-#pragma unroll
-				for (int r = 0; r < 3; r++)
-					s.M0[p][3 * j + r] = fmaf(G0[0][r], Ji[j][0], fmaf(G0[1][r], Ji[j][1], G0[2][r] * Ji[j][2]));
-		if (TERM == kHydro || TERM == kDevHydro)
-#pragma unroll
-			for (int j = 0; j < 3; j++)
-#pragma unroll
-				for (int r = 0; r < 3; r++)
-					s.M1[p][3 * j + r] = fmaf(G1[0][r], Ji[j][0], fmaf(G1[1][r], Ji[j][1], G1[2][r] * Ji[j][2]));
+			for (int j = 0; j < 3; j++) {
+				if (TERM != kHydro) s.M0[p][j] = row(G0, Ji[j]);
+				if (TERM == kHydro || TERM == kDevHydro) s.M1[p][j] = row(G1, Ji[j]);
+			}
+		} else {
+			const float Jc[3] = {own == 0 ? Ji[0][0] : own == 1 ? Ji[1][0] : Ji[2][0],
+			                     own == 0 ? Ji[0][1] : own == 1 ? Ji[1][1] : Ji[2][1],
+			                     own == 0 ? Ji[0][2] : own == 1 ? Ji[1][2] : Ji[2][2]};
+			if (TERM != kHydro) s.M0[p][own] = row(G0, Jc);
+			if (TERM == kHydro || TERM == kDevHydro) s.M1[p][own] = row(G1, Jc);
+			if (own) u0 = u1 = 0.0f;  // one lane's share per point
+		}
 	}
 	__syncwarp();
 }
 
 // g_n += sum_p M_p dN_p[n] for this lane's node (n < 26) from slot M
-__device__ __forceinline__ Vec3 gather(const DevCtx& C, const float (*M)[9], const Elem& E, int hi) {
+__device__ __forceinline__ Vec3 gather(const float4 (*M)[3], const Elem& E, int hi) {
 	Vec3 g = {0.0f, 0.0f, 0.0f};
+	const float(*T)[3][32] = hi ? E.T->b27 : E.T->b8;
 	const int np = hi ? 27 : 8, n = (int)E.lane;
 	if (n < 26)
-#pragma unroll 1
+#pragma unroll 4
 		for (int p = 0; p < np; p++) {
-			const float d0 = tab(C, hi, p, n, 0), d1 = tab(C, hi, p, n, 1), d2 = tab(C, hi, p, n, 2);
-			g.x += fmaf(M[p][0], d0, fmaf(M[p][3], d1, M[p][6] * d2));
-			g.y += fmaf(M[p][1], d0, fmaf(M[p][4], d1, M[p][7] * d2));
-			g.z += fmaf(M[p][2], d0, fmaf(M[p][5], d1, M[p][8] * d2));
+			const float d0 = T[p][0][n], d1 = T[p][1][n], d2 = T[p][2][n];
+			const float4 a = M[p][0], b = M[p][1], c = M[p][2];
+			g.x += fmaf(a.x, d0, fmaf(b.x, d1, c.x * d2));
+			g.y += fmaf(a.y, d0, fmaf(b.y, d1, c.y * d2));
+			g.z += fmaf(a.z, d0, fmaf(b.z, d1, c.z * d2));
 		}
 	return g;
 }
 
-// node 26 takes minus the others' sum
-__device__ __forceinline__ Vec3 root(const Elem& E, Vec3 g) {
-	const float sx = wsum(E.lane < 26 ? g.x : 0.0f), sy = wsum(E.lane < 26 ? g.y : 0.0f),
-	            sz = wsum(E.lane < 26 ? g.z : 0.0f);
-	return E.lane == 26 ? Vec3{g.x - sx, g.y - sy, g.z - sz} : E.lane < 26 ? g : Vec3{0.0f, 0.0f, 0.0f};
+// node 26 takes minus the others' sum s
+__device__ __forceinline__ Vec3 root_of(const Elem& E, const Vec3& g, const float* s) {
+	return E.lane == 26 ? Vec3{g.x - s[0], g.y - s[1], g.z - s[2]} : E.lane < 26 ? g : Vec3{0.0f, 0.0f, 0.0f};
+}
+
+// The gradient with node 26's from the others' sum; u (this lane's energy
+// contribution) summed over the lanes.
+__device__ __forceinline__ Vec3 root_u(const Elem& E, const Vec3& g, float& u) {
+	const bool on = E.lane < 26;
+	float v[4] = {on ? g.x : 0.0f, on ? g.y : 0.0f, on ? g.z : 0.0f, u};
+	wsums(v);
+	u = v[3];
+	return root_of(E, g, v);
+}
+
+// The same for two gradients and energies together.
+__device__ __forceinline__ void root2_u(const Elem& E, Vec3& g0, float& u0, Vec3& g1, float& u1) {
+	const bool on = E.lane < 26;
+	float v[8] = {on ? g0.x : 0.0f, on ? g0.y : 0.0f, on ? g0.z : 0.0f, u0,
+	              on ? g1.x : 0.0f, on ? g1.y : 0.0f, on ? g1.z : 0.0f, u1};
+	wsums(v);
+	u0 = v[3];
+	u1 = v[7];
+	g0 = root_of(E, g0, v);
+	g1 = root_of(E, g1, v + 4);
 }
 
 // The prefactored I1 over the 26 offsets (XPBDFEM/Fem.cpp:163-192): this
-// lane's gradient row (root included) and U.
-__device__ __forceinline__ float pref_i1(const Scratch& s, const Elem& E, Vec3& g) {
+// lane's gradient row (without node 26's) and its share of U.
+__device__ __forceinline__ float pref_row(const Scratch& s, const Elem& E, Vec3& g) {
 	float u = 0.0f;
 	g = {0.0f, 0.0f, 0.0f};
 	const int i = (int)E.lane;
 	if (i < 26) {
 		const float qq = rec(E, kQQ + i);
-		const Vec3 Pi = {s.P[i][0], s.P[i][1], s.P[i][2]};
+		const Vec3 Pi = v3(s.P[i]);
 		u = qq * dot(Pi, Pi);
 		g = {2.0f * qq * Pi.x, 2.0f * qq * Pi.y, 2.0f * qq * Pi.z};
-		// QR of the pair (lo, hi), lo < hi: row lo starts at lo (51 - lo) / 2
-#pragma unroll 2
+		// QR of the pair (lo, hi), lo < hi: row lo starts at lo (51 - lo) / 2.
+		// No branches: the pair's place is selected, and j = i adds 0 P_i.
+		const int below = kQR + i - 1;                       // + j (51 - j) / 2 - j: pairs (j, i)
+		const int above = kQR + i * (51 - i) / 2 - i - 1;  // + j: pairs (i, j)
+#pragma unroll
 		for (int j = 0; j < 26; j++) {
-			if (j == i) continue;
-			const int lo = i < j ? i : j, hi = i < j ? j : i;
-			const float qr = rec(E, kQR + lo * (51 - lo) / 2 + (hi - lo - 1));
-			const Vec3 Pj = {s.P[j][0], s.P[j][1], s.P[j][2]};
+			const Vec3 Pj = v3(s.P[j]);
+			const float q = E.R[j < i ? below + (j * (51 - j) / 2 - j) : above + j];
+			const float qr = j == i ? 0.0f : q;
 			g = {fmaf(qr, Pj.x, g.x), fmaf(qr, Pj.y, g.y), fmaf(qr, Pj.z, g.z)};
-			if (j > i) u = fmaf(qr, dot(Pi, Pj), u);
+			const float un = fmaf(qr, dot(Pi, Pj), u);
+			u = j > i ? un : u;
 		}
 	}
-	g = root(E, g);
-	return wsum(u);
+	return u;
 }
 
 __device__ __forceinline__ float wgg_of(const Elem& E, const Vec3& a, const Vec3& b) {
 	return 1.0e-22f + wsum(E.lane < 27 ? E.w * dot(a, b) : 0.0f);
+}
+__device__ __forceinline__ void wgg3_of(const Elem& E, const Vec3& g0, const Vec3& g1, float& s00, float& s10, float& s11) {
+	const bool on = E.lane < 27;
+	float v[3] = {on ? E.w * dot(g0, g0) : 0.0f, on ? E.w * dot(g1, g0) : 0.0f, on ? E.w * dot(g1, g1) : 0.0f};
+	wsums(v);
+	s00 = 1.0e-22f + v[0];
+	s10 = 1.0e-22f + v[1];
+	s11 = 1.0e-22f + v[2];
 }
 __device__ __forceinline__ float gD_of(const Elem& E, const Vec3& g) {
 	return wsum(E.lane < 27 ? fmaf(g.x, E.D.x, fmaf(g.y, E.D.y, g.z * E.D.z)) : 0.0f);
@@ -252,36 +354,57 @@ __device__ __forceinline__ void move2(Elem& E, float l0, const Vec3& g0, float l
 	E.D.z = fmaf(s1, g1.z, fmaf(s0, g0.z, E.D.z));
 }
 
-__device__ __forceinline__ Scratch& scratch() {
-	__shared__ Scratch s[8];  // 256-thread blocks: 8 warps
-	return s[threadIdx.x >> 5];
+struct Shared {
+	Tables t;
+	Scratch s[8];  // 256-thread blocks: 8 warps
+};
+__device__ __forceinline__ Shared& shared() {
+	extern __shared__ __align__(128) unsigned char h27_smem[];
+	return *reinterpret_cast<Shared*>(h27_smem);
 }
 
-__device__ __forceinline__ void load(const DevCtx& C, uint32_t i, Scratch& s, Elem& E) {
-	E.lane = threadIdx.x & 31u;
-	// the record, 176 float4, coalesced across the warp, once every lane is
-	// done with the previous element's copy
-	__syncwarp();
+// Starts the copy of element i's record and vertex ids into the warp's
+// scratch (asynchronous 16-byte copies: a warp's next element is known, so
+// its 2.9 KB come while the pass ends and the barrier is waited for).
+__device__ __forceinline__ void fetch(const DevCtx& C, uint32_t i, Scratch& s, uint32_t lane) {
+	__syncwarp();  // every lane is done with the last element's copy
 	const float4* src = C.el_rec + (size_t)i * (kRec / 4);
-	for (uint32_t k = E.lane; k < kRec / 4; k += 32) s.rec[k] = __ldg(src + k);
+	auto copy = [](void* dst, const void* from) {
+		asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(from) : "memory");
+	};
+	for (uint32_t k = lane; k < kRec / 4; k += 32) copy(&s.rec[k], src + k);
+	if (lane < 7u) copy(&s.vid[4 * lane], C.el_vid + 7 * (size_t)i + lane);
+	if (lane == 0) s.have = i;
+	__syncwarp();
+}
+
+__device__ __forceinline__ void load(const DevCtx& C, uint32_t i, Scratch& s, const Tables& T, Elem& E) {
+	E.lane = threadIdx.x & 31u;
+	E.T = &T;
+	if (s.have != i) {
+		asm volatile("cp.async.wait_all;" ::: "memory");  // a fetch that is not used after all
+		fetch(C, i, s, E.lane);
+	}
+	asm volatile("cp.async.wait_all;" ::: "memory");
 	__syncwarp();
 	E.R = reinterpret_cast<const float*>(s.rec);
 	E.O = E.D = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 	E.w = 0.0f;
 	E.dv = 0;
 	if (E.lane < 27) {
-		E.dv = __ldg(reinterpret_cast<const uint32_t*>(C.el_vid + 7 * (size_t)i) + E.lane);
+		E.dv = s.vid[E.lane];
 		ld_vertex(C.vert + 2 * (size_t)E.dv, E.O, E.D);
 		E.w = E.O.w;
 	}
 }
 
-// One H27 of a pass (the kinds of ElemPass), every lane of the warp.
+// One H27 of a pass (the kinds of ElemPass), every lane of the warp; next: the
+// element to fetch for the warp's next call (kNoElem: none).
 template <int KIND>
-__device__ __noinline__ void h27_pass(const DevCtx& C, uint32_t i, float inv_dt, float inv_dt2, float rd) {
-	Scratch& s = scratch();
+__device__ __noinline__ void h27_pass(const DevCtx& C, uint32_t i, uint32_t next, float inv_dt, float inv_dt2, float rd) {
+	Scratch& s = shared().s[threadIdx.x >> 5];
 	Elem E;
-	load(C, i, s, E);
+	load(C, i, s, shared().t, E);
 	const BodyParams& bp = C.bodies[__float_as_uint(__shfl_sync(kAll, E.D.w, 0)) >> 8];
 	const uint32_t e = __ldg(&bp.energy);
 	if (KIND != kVolume && (e == 11u || e == 12u)) return;  // SolveElementCube acts on 8-node hexes only
@@ -294,8 +417,8 @@ __device__ __noinline__ void h27_pass(const DevCtx& C, uint32_t i, float inv_dt,
 	float u0, u1;
 	if (KIND == kVolume) {
 		points<kHydro>(C, s, E, 0, bp, e, 1.0f, u0, u1);
-		const Vec3 g = root(E, gather(C, s.M1, E, 0));
-		const float U = wsum(u1);
+		const Vec3 g = root_u(E, gather(s.M1, E, 0), u1);
+		const float U = u1;
 		const float alpha = __ldg(&bp.compliance) * vol * inv_dt2;
 		move(E, (-2.0f * U) / fmaf(2.0f * U, alpha, wgg_of(E, g, g)), g);
 	} else if (e <= 2u) {
@@ -304,15 +427,15 @@ __device__ __noinline__ void h27_pass(const DevCtx& C, uint32_t i, float inv_dt,
 		if (e != 2u) {
 			const int hi = e == 0u;
 			points<kPixarFull>(C, s, E, hi, bp, e, __ldg(&bp.a), u0, u1);
-			g = root(E, gather(C, s.M0, E, hi));
-			U = wsum(u0);
+			g = root_u(E, gather(s.M0, E, hi), u0);
+			U = u0;
 		} else {
 			const float hw = __ldg(&bp.hw);
 			points<kHydro>(C, s, E, 0, bp, e, __ldg(&bp.a), u0, u1);
-			Vec3 gh = root(E, gather(C, s.M1, E, 0));
-			Vec3 gi;
-			const float UI = pref_i1(s, E, gi);
-			U = fmaf(hw, wsum(u1), UI);
+			Vec3 gh = gather(s.M1, E, 0), gi;
+			float UI = pref_row(s, E, gi);
+			root2_u(E, gh, u1, gi, UI);
+			U = fmaf(hw, u1, UI);
 			g = {fmaf(hw, gh.x, gi.x), fmaf(hw, gh.y, gi.y), fmaf(hw, gh.z, gi.z)};
 		}
 		const float comp = __ldg(&bp.compliance) / vol;
@@ -331,16 +454,24 @@ __device__ __noinline__ void h27_pass(const DevCtx& C, uint32_t i, float inv_dt,
 		Vec3 g0, g1 = {0.0f, 0.0f, 0.0f};
 		if (full) {
 			if (coupled && e != 6u) {
-				points<kDevHydro>(C, s, E, 1, bp, e, a, u0, u1);
-				g1 = root(E, gather(C, s.M1, E, 1));
-				U1 = wsum(u1);
+				points<kDevHydro>(C, s, E, 1, bp, e, a, u0, U1);
+				g0 = gather(s.M0, E, 1);
+				g1 = gather(s.M1, E, 1);
+				root2_u(E, g0, u0, g1, U1);
 			} else {
 				points<kDev>(C, s, E, 1, bp, e, a, u0, u1);
+				g0 = root_u(E, gather(s.M0, E, 1), u0);
 			}
-			g0 = root(E, gather(C, s.M0, E, 1));
-			U0 = fmaxf(0.0001f, wsum(u0));
+			U0 = fmaxf(0.0001f, u0);
 		} else {
-			U0 = pref_i1(s, E, g0);
+			U0 = pref_row(s, E, g0);
+			if (coupled) {
+				points<kHydro>(C, s, E, 0, bp, e, a, u0, U1);
+				g1 = gather(s.M1, E, 0);
+				root2_u(E, g0, U0, g1, U1);
+			} else {
+				g0 = root_u(E, g0, U0);
+			}
 			if (e == 7u) {
 				const float C0 = __ldg(&bp.yeoh[0]), C1 = __ldg(&bp.yeoh[1]), C2 = __ldg(&bp.yeoh[2]);
 				const float IM = U0 - 3.0f;
@@ -350,13 +481,13 @@ __device__ __noinline__ void h27_pass(const DevCtx& C, uint32_t i, float inv_dt,
 			}
 		}
 		if (coupled) {
-			if (!full || e == 6u) {
+			if (e == 6u) {
 				__syncwarp();
-				points<kHydro>(C, s, E, 0, bp, e, a, u0, u1);
-				g1 = root(E, gather(C, s.M1, E, 0));
-				U1 = wsum(u1);
+				points<kHydro>(C, s, E, 0, bp, e, a, u0, U1);
+				g1 = root_u(E, gather(s.M1, E, 0), U1);
 			}
-			const float wgg0 = wgg_of(E, g0, g0), wgg1 = wgg_of(E, g1, g0), wgg2 = wgg_of(E, g1, g1);
+			float wgg0, wgg1, wgg2;
+			wgg3_of(E, g0, g1, wgg0, wgg1, wgg2);
 			float l0, l1;
 			if (KIND == kRayleigh) {
 				if (sim) {
@@ -379,22 +510,21 @@ __device__ __noinline__ void h27_pass(const DevCtx& C, uint32_t i, float inv_dt,
 			move(E, lambda1_of(U0, wgg0, damp > 0.0f ? gD_of(E, g0) : 0.0f, alpha0, comp0, damp, limit, inv_dt), g0);
 			share_rel(s, E, false);
 			const int hi = full && e != 6u;
-			points<kHydro>(C, s, E, hi, bp, e, a, u0, u1);
-			g1 = root(E, gather(C, s.M1, E, hi));
-			U1 = wsum(u1);
+			points<kHydro>(C, s, E, hi, bp, e, a, u0, U1);
+			g1 = root_u(E, gather(s.M1, E, hi), U1);
 			const float wgg2 = wgg_of(E, g1, g1);
 			move(E, lambda1_of(U1, wgg2, damp > 0.0f ? gD_of(E, g1) : 0.0f, alpha1, comp1, damp, limit, inv_dt), g1);
 		}
 	}
-	__syncwarp();
+	if (next != kNoElem) fetch(C, next, s, E.lane);
 	if (E.lane < 27) st_vertex(C.vert + 2 * (size_t)E.dv, E.O, E.D);
 }
 
 // PbdDamp over the 27 nodes (XPBDFEM/Xpbd.h:306-346) on the canonical state
 // (O = X, D = V), the coefficient coeff / surfaceArea capped at 1.
-__device__ __forceinline__ void h27_pbd_in(const DevCtx& C, Scratch& s, uint32_t i, float coeff) {
+__device__ __forceinline__ void h27_pbd_in(const DevCtx& C, Scratch& s, const Tables& T, uint32_t i, float coeff) {
 	Elem E;
-	load(C, i, s, E);
+	load(C, i, s, T, E);
 	const bool node = E.lane < 27;
 	const float damping = fminf(1.0f, coeff / rec(E, kArea));
 	const float Wavg = (1.0e-8f + wsum(E.w)) * (1.0f / 27.0f), Wmin = 0.0001f * Wavg;
@@ -422,15 +552,23 @@ __device__ __forceinline__ void h27_pbd_in(const DevCtx& C, Scratch& s, uint32_t
 	if (node) st_vertex(C.vert + 2 * (size_t)E.dv, E.O, E.D);
 }
 
-__device__ __noinline__ void h27_pbd(const DevCtx& C, uint32_t i, float coeff) { h27_pbd_in(C, scratch(), i, coeff); }
+__device__ __noinline__ void h27_pbd(const DevCtx& C, uint32_t i, float coeff) {
+	h27_pbd_in(C, shared().s[threadIdx.x >> 5], shared().t, i, coeff);
+}
 
 struct H27Elem {
-	static constexpr bool kWarp = true;
+	static constexpr int kLanes = 32, kPbdLanes = 32;
 	static constexpr int kMinBlocks = 3;  // at most 85 registers: three 256-thread blocks per SM
 	static constexpr uint32_t kVid4 = 7;
+	static constexpr size_t smem() { return sizeof(Shared); }
+	__device__ static void init(const DevCtx& C) {
+		if ((threadIdx.x & 31u) == 0u) shared().s[threadIdx.x >> 5].have = kNoElem;
+		load_tables(C, shared().t);
+	}
 	template <int KIND>
-	__device__ static void pass(const DevCtx& C, uint32_t i, float inv_dt, float inv_dt2, float rd) {
-		h27_pass<KIND>(C, i, inv_dt, inv_dt2, rd);
+	__device__ static void pass(const DevCtx& C, uint32_t i, bool, float inv_dt, float inv_dt2, float rd,
+	                            uint32_t next = kNoElem) {
+		h27_pass<KIND>(C, i, next, inv_dt, inv_dt2, rd);
 	}
 	__device__ static void pbd(const DevCtx& C, uint32_t i, float coeff) { h27_pbd(C, i, coeff); }
 };

@@ -28,47 +28,45 @@ __device__ __forceinline__ bool in_slice_n(const DevCtx& C, const BodyParams& bp
 	return f >= n * m / 8u && f < n * (m + 1u) / 8u;
 }
 
-// One pass kind over the colours of one element kind (units: threads for
-// T10s, warps for H27s); false when a barrier gave up.
+constexpr int kPbd = 100;  // the PBD damping sweep (not a pass kind of the elements)
+
+// One pass kind over the colours of one element kind; false when a barrier
+// gave up.
 template <class E, int KIND>
-__device__ __forceinline__ bool sweep(const DevCtx& C, const DevCtx& B, uint32_t nthreads, float inv_dt, float inv_dt2,
-                                      uint32_t it, uint32_t tick, uint32_t& target) {
-	// a warp's worth of elements at a time to each block, as in k_elements
-	const uint32_t gwarp = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
-	const uint32_t unit = E::kWarp ? gwarp : gwarp * 32u + (threadIdx.x & 31u);
-	const uint32_t nunits = E::kWarp ? nthreads >> 5 : nthreads;
+__device__ __forceinline__ bool sweep(const DevCtx& C, const DevCtx& B, float inv_dt, float inv_dt2, uint32_t it,
+                                      uint32_t tick, uint32_t& target) {
 	for (uint32_t c = 0; c < C.el_colours; c++) {
 		const uint32_t b = __ldg(C.colour_el_begin + c), e = __ldg(C.colour_el_begin + c + 1);
-		for (uint32_t i = b + unit; i < e; i += nunits) {
-			if (KIND == kSolve) {
-				E::template pass<kSolve>(C, i, inv_dt, inv_dt2, 0.0f);
-				continue;
+		for_elements<KIND == kPbd ? E::kPbdLanes : E::kLanes>(b, e, [&](uint32_t i, bool live) {
+			if constexpr (KIND == kSolve) {
+				E::template pass<kSolve>(C, i, live, inv_dt, inv_dt2, 0.0f);
+			} else {
+				const BodyParams& bp = body_of_el<E>(C, i);
+				const uint32_t n = E::kVid4 == 7 ? __ldg(&bp.nhexes) : __ldg(&bp.ntets);
+				if constexpr (KIND == kVolume) {
+					live = live && it < __ldg(&bp.volume_passes);
+					if (any_live<E>(live)) E::template pass<kVolume>(C, i, live, inv_dt, inv_dt2, 0.0f);
+				} else if constexpr (KIND == kRayleigh) {
+					const uint32_t type = __ldg(&bp.rayleigh_type);
+					const float rd = __ldg(&bp.damping) * (type == 3u ? 8.0f : 1.0f);
+					live = live && type >= 2u && rd > 0.0f && in_slice_n(C, bp, i, n, tick);
+					if (any_live<E>(live)) E::template pass<kRayleigh>(C, i, live, inv_dt, inv_dt2, rd);
+				} else if (__ldg(&bp.pbd_on) && in_slice_n(C, bp, i, n, tick)) {
+					E::pbd(C, i, __ldg(&bp.rayleigh_type) == 3u ? __ldg(&bp.pbd_coeff_amortized) : __ldg(&bp.pbd_coeff));
+				}
 			}
-			const BodyParams& bp = body_of_el<E>(C, i);
-			const uint32_t n = E::kWarp ? __ldg(&bp.nhexes) : __ldg(&bp.ntets);
-			if (KIND == kVolume) {
-				if (it < __ldg(&bp.volume_passes)) E::template pass<kVolume>(C, i, inv_dt, inv_dt2, 0.0f);
-			} else if (KIND == kRayleigh) {
-				const uint32_t type = __ldg(&bp.rayleigh_type);
-				const float rd = __ldg(&bp.damping) * (type == 3u ? 8.0f : 1.0f);
-				if (type >= 2u && rd > 0.0f && in_slice_n(C, bp, i, n, tick))
-					E::template pass<kRayleigh>(C, i, inv_dt, inv_dt2, rd);
-			} else if (__ldg(&bp.pbd_on) && in_slice_n(C, bp, i, n, tick)) {
-				E::pbd(C, i, __ldg(&bp.rayleigh_type) == 3u ? __ldg(&bp.pbd_coeff_amortized) : __ldg(&bp.pbd_coeff));
-			}
-		}
+		});
 		if (!grid_sync(B, target)) return false;
 	}
 	return true;
 }
-
-constexpr int kPbd = 100;  // the PBD damping sweep (not a pass kind of the elements)
 
 __global__ void __launch_bounds__(256, 1) k_qmixed(DevCtx Ch, DevCtx Ct, uint32_t nsub, float dt) {
 	const float inv_dt = 1.0f / dt, inv_dt2 = 1.0f / (dt * dt);
 	const uint32_t gtid = blockIdx.x * blockDim.x + threadIdx.x, nthreads = gridDim.x * blockDim.x;
 	const uint32_t tick0 = __ldcg(Ch.tick);
 	const bool dmode = Ch.damp_kinds != 0u;
+	H27::init(Ch);
 	uint32_t target = Ch.bar_base;
 	for (uint32_t s = 0; s < nsub; s++) {
 		for (uint32_t v = gtid; v < Ch.nverts; v += nthreads) {
@@ -79,11 +77,11 @@ __global__ void __launch_bounds__(256, 1) k_qmixed(DevCtx Ch, DevCtx Ct, uint32_
 		}
 		if (!grid_sync(Ch, target)) return;
 		const uint32_t tick = tick0 + s;
-		if (!sweep<T10, kSolve>(Ct, Ch, nthreads, inv_dt, inv_dt2, 0, tick, target)) return;
-		if (!sweep<H27, kSolve>(Ch, Ch, nthreads, inv_dt, inv_dt2, 0, tick, target)) return;
+		if (!sweep<T10, kSolve>(Ct, Ch, inv_dt, inv_dt2, 0, tick, target)) return;
+		if (!sweep<H27, kSolve>(Ch, Ch, inv_dt, inv_dt2, 0, tick, target)) return;
 		for (uint32_t it = 0; it < Ch.nvol; it++) {
-			if (!sweep<T10, kVolume>(Ct, Ch, nthreads, inv_dt, inv_dt2, it, tick, target)) return;
-			if (!sweep<H27, kVolume>(Ch, Ch, nthreads, inv_dt, inv_dt2, it, tick, target)) return;
+			if (!sweep<T10, kVolume>(Ct, Ch, inv_dt, inv_dt2, it, tick, target)) return;
+			if (!sweep<H27, kVolume>(Ch, Ch, inv_dt, inv_dt2, it, tick, target)) return;
 		}
 		if (!dmode) continue;
 		for (uint32_t v = gtid; v < Ch.nverts; v += nthreads) {
@@ -94,12 +92,12 @@ __global__ void __launch_bounds__(256, 1) k_qmixed(DevCtx Ch, DevCtx Ct, uint32_
 		}
 		if (!grid_sync(Ch, target)) return;
 		if (Ch.damp_kinds & 1u) {
-			if (!sweep<T10, kRayleigh>(Ct, Ch, nthreads, inv_dt, inv_dt2, 0, tick, target)) return;
-			if (!sweep<H27, kRayleigh>(Ch, Ch, nthreads, inv_dt, inv_dt2, 0, tick, target)) return;
+			if (!sweep<T10, kRayleigh>(Ct, Ch, inv_dt, inv_dt2, 0, tick, target)) return;
+			if (!sweep<H27, kRayleigh>(Ch, Ch, inv_dt, inv_dt2, 0, tick, target)) return;
 		}
 		if (Ch.damp_kinds & 2u) {
-			if (!sweep<T10, kPbd>(Ct, Ch, nthreads, inv_dt, inv_dt2, 0, tick, target)) return;
-			if (!sweep<H27, kPbd>(Ch, Ch, nthreads, inv_dt, inv_dt2, 0, tick, target)) return;
+			if (!sweep<T10, kPbd>(Ct, Ch, inv_dt, inv_dt2, 0, tick, target)) return;
+			if (!sweep<H27, kPbd>(Ch, Ch, inv_dt, inv_dt2, 0, tick, target)) return;
 		}
 	}
 	if (!dmode) {
@@ -123,14 +121,16 @@ int launch_qmixed(const DevCtx& ch27, const DevCtx& ct10, int block, uint32_t ns
 	int dev = 0, sms = 0, per_sm = 0;
 	cudaError_t e = cudaGetDevice(&dev);
 	if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-	if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f, block, 0);
+	if (e == cudaSuccess)
+		e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)H27::smem());
+	if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f, block, H27::smem());
 	if (e != cudaSuccess) return (int)e;
 	if (per_sm <= 0) return (int)cudaErrorInvalidConfiguration;
 	e = reset_barrier(ch27, st);
 	if (e != cudaSuccess) return (int)e;
 	DevCtx a = ch27, b = ct10;
 	void* args[] = {&a, &b, &nsub, &dt};
-	return (int)cudaLaunchCooperativeKernel(f, dim3(per_sm * sms), dim3(block), args, 0, st);
+	return (int)cudaLaunchCooperativeKernel(f, dim3(per_sm * sms), dim3(block), args, H27::smem(), st);
 }
 
 }  // namespace xfem

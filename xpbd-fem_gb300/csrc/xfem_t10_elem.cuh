@@ -333,11 +333,13 @@ __device__ __noinline__ void q_pbd(const DevCtx& C, uint32_t i, float coeff) {
 }
 
 struct T10Elem {
-	static constexpr bool kWarp = false;
+	static constexpr int kLanes = 1, kPbdLanes = 1;
 	static constexpr int kMinBlocks = 1;
 	static constexpr uint32_t kVid4 = 3;
+	static constexpr size_t smem() { return 0; }
+	__device__ static void init(const DevCtx&) {}
 	template <int KIND>
-	__device__ static void pass(const DevCtx& C, uint32_t i, float inv_dt, float inv_dt2, float rd) {
+	__device__ static void pass(const DevCtx& C, uint32_t i, bool, float inv_dt, float inv_dt2, float rd) {
 		q_pass<KIND>(C, i, inv_dt, inv_dt2, rd);
 	}
 	__device__ static void pbd(const DevCtx& C, uint32_t i, float coeff) { q_pbd(C, i, coeff); }
