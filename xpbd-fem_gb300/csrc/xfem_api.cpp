@@ -864,6 +864,7 @@ int build_rings(xfem_body* h) {
 				}
 				// each node's corners (local element << 2 (tets), << 3 (hexes), << 4 (T10s) or << 5 (H27s) | corner), in
 				// element order
+				if (cwords.size() & 1u) cwords.push_back(0);  // 4-byte aligned: copied as words
 				clist.push_back((uint32_t)cwords.size());
 				const size_t ob = cwords.size();
 				cwords.resize(ob + nn + 1);
@@ -908,6 +909,7 @@ int build_rings(xfem_body* h) {
 	XCUDA(h->pbd_cb.alloc(pcb.size()));
 	XCUDA(h->pbd_cl.alloc(pcl.size()));
 	XCUDA(h->pbd_ent.alloc(pent.size()));
+	if (cwords.size() & 1u) cwords.push_back(0);
 	XCUDA(h->ring_clist.alloc(clist.size()));
 	XCUDA(h->ring_cwords.alloc(cwords.size()));
 	XCUDA(h->ring_hdr.alloc(hdr.size()));
@@ -1957,7 +1959,7 @@ int launch_mode(xfem_body* h, const DevCtx& ctx, uint32_t nsub, float dt) {
 		const int e = h->el_mode == kElHexes ? launch_hex_rings(ctx, 256, nsub, dt, h->stream)
 		              : h->el_mode == kElT10 ? launch_t10_rings(ctx, 128, nsub, dt, h->stream)
 		              : h->el_mode == kElH27 ? launch_h27_rings(ctx, 128, nsub, dt, h->stream)
-		                                     : launch_rings(ctx, 256, nsub, dt, h->stream);
+		                                     : launch_rings(ctx, nsub, dt, h->stream);
 		if (e) return fail(XFEM_ECUDA, std::string("ring launch: ") + cudaGetErrorString((cudaError_t)e));
 		return XFEM_OK;
 	}

@@ -524,7 +524,7 @@ int launch_volume(const float4* vert, const uint32_t* tets_dev, uint32_t nt, dou
 // One-ring mode (xfem_rings.cu): nsub substeps of the continuous-pressure
 // models, a cooperative persistent launch of `block` threads per block
 // (canonical (X, V) in and out).
-int launch_rings(const DevCtx& ctx, int block, uint32_t nsub, float dt, void* stream);
+int launch_rings(const DevCtx& ctx, uint32_t nsub, float dt, void* stream);
 // Hex mode (xfem_hexes.cu): nsub substeps of a hex mesh, a cooperative
 // persistent launch (canonical (X, V) in and out).
 int launch_hexes(const DevCtx& ctx, int block, uint32_t nsub, float dt, void* stream);
