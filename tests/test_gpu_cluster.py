@@ -83,3 +83,25 @@ def test_recording_forward_is_the_plain_one(dims):
     b.step_frames(1, 12, DT)
     assert np.array_equal(a.positions(), b.positions()) and np.array_equal(a.velocities(), b.velocities())
     assert np.array_equal(traj[-1], b.positions()[tips])
+
+
+# the reverse as one cluster: one block; one, two and three rounds of chunks per
+# block; one more than that (the grid form); two bodies; checkpointed segments
+@pytest.mark.parametrize("dims,every", [([(8, 2, 2)], 0), ([(8, 2, 2)], 3), ([(20, 9, 9)], 4), ([(32, 16, 12)], 0),
+                                        ([(32, 20, 16)], 0), ([(32, 21, 20)], 0), ([(5, 4, 3), (9, 2, 7)], 5)])
+@pytest.mark.parametrize("ground", [0, 1])
+def test_reverse_matches_the_one_lane_form(dims, every, ground, monkeypatch):
+    nsub = 7
+    s = _settings(ground=ground, ground_normal=(0.0, 1.0, 0.0), ground_offset=-0.5 * 0.1 * dims[0][1] + 0.01, friction=0.4)
+    rng = np.random.default_rng(3)
+    meshes = [xfem.generate_tet_block(*d, (0.1, 0.1, 0.1), 0, 0.2) + (1000.0,) for d in dims]
+    b = xfem.Body(meshes=meshes, settings=[s] * len(meshes))
+    nv = sum(c[0] for c in b.counts)
+    tips = np.uint32([0, nv // 2, nv - 1])
+    b.adjoint_forward(nsub, DT, tips, every)
+    g = rng.standard_normal((nsub, 3, 3)).astype(np.float32)
+    gx, gv = (rng.standard_normal((nv, 3)).astype(np.float32) for _ in range(2))
+    got = b.adjoint_backward(g, gx, gv)
+    monkeypatch.setenv("XFEM_REVERSE_FORM", "lane")
+    for x, y in zip(got, b.adjoint_backward(g, gx, gv)):
+        assert np.array_equal(x, y) and np.abs(x).max() > 0

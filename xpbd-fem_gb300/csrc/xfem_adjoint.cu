@@ -30,6 +30,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <stdlib.h>
+#include <string.h>
 
 #include "xfem_device.cuh"
 #include "xfem_internal.h"
@@ -199,25 +200,52 @@ __device__ __forceinline__ const float4* tape_at(const DevCtx& C, uint32_t s, ui
 	return C.tape_v + 2 * ((size_t)s * C.nverts + v);
 }
 
+// Where the kernels keep a vertex's adjoint state, Xb and Ob: in AdjCtx::abar,
+// or spread over the shared memory of a one-cluster launch.
+struct GlobalAdj {
+	float4* abar;
+	__device__ __forceinline__ Vec3 xb(uint32_t v) const { return v3(__ldcg(abar + 2 * (size_t)v)); }
+	__device__ __forceinline__ Vec3 ob(uint32_t v) const { return v3(__ldcg(abar + 2 * (size_t)v + 1)); }
+	__device__ __forceinline__ void set_xb(uint32_t v, const Vec3& a) const {
+		__stcg(abar + 2 * (size_t)v, make_float4(a.x, a.y, a.z, 0.0f));
+	}
+	__device__ __forceinline__ void set_ob(uint32_t v, const Vec3& a) const {
+		__stcg(abar + 2 * (size_t)v + 1, make_float4(a.x, a.y, a.z, 0.0f));
+	}
+};
+
+struct ClusterAdj {
+	ClusterVerts s;
+	__device__ __forceinline__ Vec3 xb(uint32_t v) const { return v3(ClusterVerts::get(s.at(v))); }
+	__device__ __forceinline__ Vec3 ob(uint32_t v) const { return v3(ClusterVerts::get(s.at(v) + 16u * s.per)); }
+	__device__ __forceinline__ void set_xb(uint32_t v, const Vec3& a) const {
+		ClusterVerts::put(s.at(v), make_float4(a.x, a.y, a.z, 0.0f));
+	}
+	__device__ __forceinline__ void set_ob(uint32_t v, const Vec3& a) const {
+		ClusterVerts::put(s.at(v) + 16u * s.per, make_float4(a.x, a.y, a.z, 0.0f));
+	}
+};
+
 // Reverse of the boundary between two substeps for one vertex: the finish
 // of the earlier one (its start O = Op, its swept D = Ds) and the predict of
 // the later one. xb: dL/d(predicted position of the later substep) with its
-// solves already reversed; run_sub: the run substep whose end position is the
-// later substep's O (the loss term). Leaves the earlier substep's state.
-__device__ __forceinline__ void boundary_reverse(const DevCtx& C, const AdjCtx& A, uint32_t v, const float4& Op,
-                                                 const float4& Ds, Vec3 xb, uint32_t run_sub) {
+// solves already reversed; tip: the loss at the end of the earlier substep, whose
+// end position is the later substep's O. Leaves the earlier substep's state.
+template <class AS>
+__device__ __forceinline__ void boundary_reverse(const DevCtx& C, const AS& ab, uint32_t v, const float4& Op,
+                                                 const float4& Ds, Vec3 xb, const Vec3& tip) {
 	const BodyParams& bp = C.bodies[__float_as_uint(Ds.w) >> 8];
 	// O of the later substep is read by its solves (through O + D), by the
 	// substeps after it and by the loss
-	const Vec3 os = vadd(vadd(v3(__ldcg(A.abar + 2 * (size_t)v + 1)), xb), tip_grad(C, A, v, run_sub));
+	const Vec3 os = vadd(vadd(ab.ob(v), xb), tip);
 	// O = Op + D', D_pred = (D' / dt + g dt) drag dt
 	const Vec3 dfin = vfma(xb, bp.drag_mul, os);
 	Vec3 ob = os;
 	const Vec3 dsb = finish_reverse(bp, Op, Ds, dfin, ob);
 	// the earlier substep's swept position is Op + Ds
 	ob = vsub(ob, dsb);
-	__stcg(A.abar + 2 * (size_t)v, make_float4(dsb.x, dsb.y, dsb.z, 0.0f));
-	__stcg(A.abar + 2 * (size_t)v + 1, make_float4(ob.x, ob.y, ob.z, 0.0f));
+	ab.set_xb(v, dsb);
+	ab.set_ob(v, ob);
 }
 
 // Reverse of advance_vertex at launch substep s for one owned vertex (xb as
@@ -226,59 +254,82 @@ __device__ __forceinline__ void boundary_reverse(const DevCtx& C, const AdjCtx& 
 // state: the previous segment's finalize reverse continues from it with the
 // same arithmetic as a boundary inside a launch, so checkpointed runs give
 // the full tape's results bit for bit.
-__device__ __forceinline__ void advance_reverse(const DevCtx& C, const AdjCtx& A, uint32_t v, uint32_t s, bool first,
+// t: what it reads of the tape and the loss, loaded by the caller (owned_tape).
+struct OwnedTape {
+	float4 Op, Ds;  // O of the substep before (not on the launch's first), D before the advance
+	Vec3 tip;       // the loss at the end of the substep before
+};
+
+__device__ __forceinline__ OwnedTape owned_tape(const DevCtx& C, const AdjCtx& A, uint32_t v, uint32_t s, bool first) {
+	OwnedTape t = {make_float4(0.0f, 0.0f, 0.0f, 0.0f), __ldcs(tape_at(C, s, v) + 1), {0.0f, 0.0f, 0.0f}};
+	if (!first) {
+		t.Op = __ldcg(tape_at(C, s - 1, v));
+		t.tip = tip_grad(C, A, v, C.sub_base + s - 1);
+	}
+	return t;
+}
+
+template <class AS>
+__device__ __forceinline__ void advance_reverse(const DevCtx& C, const AS& ab, uint32_t v, const OwnedTape& t, bool first,
                                                 float dt, Vec3 xb) {
 	if (first) {
 		if (C.sub_base > 0) {
-			__stcg(A.abar + 2 * (size_t)v, make_float4(xb.x, xb.y, xb.z, 0.0f));
+			ab.set_xb(v, xb);
 			return;
 		}
 		// O = X, D = ((V + g dt) drag) dt
-		const float4 Dl = __ldcs(tape_at(C, s, v) + 1);
-		const BodyParams& bp = C.bodies[__float_as_uint(Dl.w) >> 8];
-		const Vec3 os = vadd(v3(__ldcg(A.abar + 2 * (size_t)v + 1)), xb);
+		const BodyParams& bp = C.bodies[__float_as_uint(t.Ds.w) >> 8];
+		const Vec3 os = vadd(ab.ob(v), xb);
 		const Vec3 vb = vmul(xb, bp.drag_mul * dt);
-		__stcg(A.abar + 2 * (size_t)v, make_float4(os.x, os.y, os.z, 0.0f));
-		__stcg(A.abar + 2 * (size_t)v + 1, make_float4(vb.x, vb.y, vb.z, 0.0f));
+		ab.set_xb(v, os);
+		ab.set_ob(v, vb);
 		return;
 	}
-	boundary_reverse(C, A, v, __ldcg(tape_at(C, s - 1, v)), __ldcs(tape_at(C, s, v) + 1), xb, C.sub_base + s - 1);
+	boundary_reverse(C, ab, v, t.Op, t.Ds, xb, t.tip);
+}
+
+template <class AS>
+__device__ __forceinline__ void advance_reverse(const DevCtx& C, const AdjCtx& A, const AS& ab, uint32_t v, uint32_t s,
+                                                bool first, float dt, Vec3 xb) {
+	advance_reverse(C, ab, v, owned_tape(C, A, v, s, first), first, dt, xb);
 }
 
 // Reverse of finalize_vertex, the launch's closing finish. For the run's last
 // segment abar holds the canonical dL/dX, dL/dV at the end (plus the loss on
 // the final position); for an earlier segment it holds the next segment's
 // in-segment state, and the closing finish is reversed as a substep boundary.
-__device__ __forceinline__ void finalize_reverse(const DevCtx& C, const AdjCtx& A, uint32_t v, uint32_t nsub,
+template <class AS>
+__device__ __forceinline__ void finalize_reverse(const DevCtx& C, const AdjCtx& A, const AS& ab, uint32_t v, uint32_t nsub,
                                                  float inv_dt, bool last) {
 	const float4 Ds = __ldcg(C.tape_fin + v);
 	const float4 Op = __ldcg(tape_at(C, nsub - 1, v));
 	const uint32_t run_sub = C.sub_base + nsub - 1;
 	if (!last) {
-		boundary_reverse(C, A, v, Op, Ds, v3(__ldcg(A.abar + 2 * (size_t)v)), run_sub);
+		boundary_reverse(C, ab, v, Op, Ds, ab.xb(v), tip_grad(C, A, v, run_sub));
 		return;
 	}
 	const BodyParams& bp = C.bodies[__float_as_uint(Ds.w) >> 8];
-	const Vec3 xcb = v3(__ldcg(A.abar + 2 * (size_t)v));
-	const Vec3 vcb = v3(__ldcg(A.abar + 2 * (size_t)v + 1));
+	const Vec3 xcb = ab.xb(v);
+	const Vec3 vcb = ab.ob(v);
 	const Vec3 on = vadd(xcb, tip_grad(C, A, v, run_sub));
 	// X = O + D', V = D' / dt
 	const Vec3 dfin = vfma(vcb, inv_dt, on);
 	Vec3 ob = on;
 	const Vec3 dsb = finish_reverse(bp, Op, Ds, dfin, ob);
 	ob = vsub(ob, dsb);
-	__stcg(A.abar + 2 * (size_t)v, make_float4(dsb.x, dsb.y, dsb.z, 0.0f));
-	__stcg(A.abar + 2 * (size_t)v + 1, make_float4(ob.x, ob.y, ob.z, 0.0f));
+	ab.set_xb(v, dsb);
+	ab.set_ob(v, ob);
 }
 
 // Isolated vertices: no solve touches them; one thread reverses all the
 // segment's substeps of one vertex.
-__device__ __forceinline__ void isolated_reverse(const DevCtx& C, const AdjCtx& A, uint32_t begin, uint32_t step,
-                                                 uint32_t nsub, float dt) {
+template <class AS>
+__device__ __forceinline__ void isolated_reverse(const DevCtx& C, const AdjCtx& A, const AS& ab, uint32_t begin,
+                                                 uint32_t step, uint32_t nsub, float dt) {
 	for (uint32_t i = begin; i < C.nisolated; i += step) {
 		const uint32_t v = __ldg(C.isolated + i);
 		for (int s = (int)nsub - 1; s >= 0; s--)
-			advance_reverse(C, A, v, (uint32_t)s, s == 0, dt, v3(__ldcg(A.abar + 2 * (size_t)v)));
+			advance_reverse(C, A, ab, v, (uint32_t)s, s == 0, dt, ab.xb(v));
 	}
 }
 
@@ -354,7 +405,7 @@ __device__ __forceinline__ void cluster_reverse(const DevCtx& C, const AdjCtx& A
 	for (uint32_t k = 0; k < NV; k++) {
 		if (k < nv) {
 			if (mask & (1u << k))
-				advance_reverse(C, A, vid[k], s, first, dt, xb[k]);
+				advance_reverse(C, A, GlobalAdj{A.abar}, vid[k], s, first, dt, xb[k]);
 			else
 				__stcg(A.abar + 2 * (size_t)vid[k], make_float4(xb[k].x, xb[k].y, xb[k].z, 0.0f));
 		}
@@ -437,7 +488,7 @@ __device__ __forceinline__ void cluster_reverse_grouped(const DevCtx& C, const A
 		const uint32_t v = __ldg(vids + j * kLanes + cl);
 		const Vec3 x = xs[j];
 		if ((hdr >> (8 + j)) & 1u)
-			advance_reverse(C, A, v, s, first, dt, x);
+			advance_reverse(C, A, GlobalAdj{A.abar}, v, s, first, dt, x);
 		else
 			__stcg(A.abar + 2 * (size_t)v, make_float4(x.x, x.y, x.z, 0.0f));
 	}
@@ -458,9 +509,9 @@ __global__ void __launch_bounds__(256) k_reverse(DevCtx C, AdjCtx A, uint32_t ns
 	const uint32_t gwarp = wib * gridDim.x + blockIdx.x, nwarps = wpb * gridDim.x;
 	const uint32_t gtid = blockIdx.x * blockDim.x + threadIdx.x, nthreads = gridDim.x * blockDim.x;
 	uint32_t target = C.bar_base;
-	for (uint32_t v = gtid; v < C.nverts; v += nthreads) finalize_reverse(C, A, v, nsub, inv_dt, last != 0);
+	for (uint32_t v = gtid; v < C.nverts; v += nthreads) finalize_reverse(C, A, GlobalAdj{A.abar}, v, nsub, inv_dt, last != 0);
 	bool ok = grid_sync(C, target);
-	if (ok) isolated_reverse(C, A, gtid, nthreads, nsub, dt);
+	if (ok) isolated_reverse(C, A, GlobalAdj{A.abar}, gtid, nthreads, nsub, dt);
 	TetSlot* gsh = reinterpret_cast<TetSlot*>(rsmem) + (size_t)wib * 24 + (lane >> 3) * 6;
 	for (int s = (int)nsub - 1; s >= 0 && ok; s--) {
 		for (int c = (int)C.ncolours - 1; c >= 0 && ok; c--) {
@@ -494,6 +545,297 @@ __global__ void __launch_bounds__(256) k_reverse(DevCtx C, AdjCtx A, uint32_t ns
 	}
 }
 
+// ---- the reverse of a small all-cube handle as one thread-block cluster ---------
+//
+// As the forward's one-cluster form (xfem_cluster.cu): the adjoint state of
+// every vertex stays in the cluster's distributed shared memory and a pass ends
+// at the hardware cluster barrier. Only the chain of a cluster's six reverses
+// depends on the pass before; the solves' forward internals, the inverse
+// masses and what the advance reverse reads come from the tape. So a block of
+// eight warps works on one chunk at a time: warp 0 runs the chain, a lane per
+// cluster, while warps 1-6 recompute the internals of the block's next chunk, a
+// warp per tet, and warp 7 loads its vertices' tape; then the eight warps finish
+// the chunk's eight vertices side by side. Same functions, same order: the
+// gradients equal the grid form's bit for bit.
+//
+// 12,288 tets x 200 substeps (8 chunks per pass, 8 blocks): 11.8 ms in the grid
+// form (152 blocks, 8 lanes per cluster), 7.7 ms here (10.0 before the vertex
+// ids were kept in shared memory and the tape's next substep prefetched to L2).
+
+// A cluster's tet in shared memory: TetFw and the record words its reverse
+// reads, as 16 float4 per lane.
+struct TetWords {
+	TetFw f;
+	float q[8];  // QQ, QR
+};
+constexpr uint32_t kTetWords4 = 16;
+static_assert(sizeof(TetWords) == 16 * kTetWords4, "a tet's words are 16 float4");
+constexpr uint32_t kRevColours = 16;  // colours a handle of this form has at most
+
+// The chunk a block works on next: what its chain and finish read.
+struct RevStage {
+	float4 tet[6][kTetWords4][kLanes];
+	float4 Op[8][kLanes], Ds[8][kLanes], tip[8][kLanes];
+	float w[8][kLanes];
+};
+
+struct RevShared {
+	RevStage st[2];
+	float4 xb[8][kLanes];
+};
+
+// A chunk of the block's, kept for the launch: headers, vertex ids, first tet
+// row and the sums of -mu dL/dmu.
+struct RevChunk {
+	uint32_t hdr[kLanes], vid[8][kLanes];
+	float cbar[6][kLanes];
+	uint32_t off16, trow, pad[2];
+};
+
+// The cube's tets turn around its diagonal (solve_cube): in reverse, odd
+// tets (0, 3, N, P), then even ones (0, N, P, 3), the ring moved back by two
+// places per turn.
+__device__ __forceinline__ void reverse_cube(const RevStage& S, uint32_t lane, Vec3 xb[8], float* cbar) {
+	Vec3 r[6] = {xb[6], xb[7], xb[2], xb[1], xb[4], xb[5]};
+	float rw[6] = {S.w[6][lane], S.w[7][lane], S.w[2][lane], S.w[1][lane], S.w[4][lane], S.w[5][lane]};
+	const float w0 = S.w[0][lane], w3 = S.w[3][lane];
+	Vec3 x0 = xb[0], x3 = xb[3];
+	auto one = [&](int t, const float w[4], Vec3 x[4]) {
+		TetWords tw;
+		float4 words[kTetWords4];
+#pragma unroll
+		for (uint32_t k = 0; k < kTetWords4; k++) words[k] = S.tet[t][k][lane];
+		memcpy(&tw, words, sizeof(tw));
+		const TetRec tr = {make_float4(0.0f, 0.0f, 0.0f, 0.0f), make_float4(0.0f, 0.0f, 0.0f, 0.0f),
+		                   make_float4(0.0f, tw.q[0], tw.q[1], tw.q[2]), make_float4(tw.q[3], tw.q[4], tw.q[5], 0.0f)};
+		cbar[t * kLanes] += tet_reverse(tr, tw.f, w, x);
+	};
+#pragma unroll 1
+	for (int t = 4; t >= 0; t -= 2) {
+		{
+			const float w[4] = {w0, w3, rw[2], rw[1]};
+			Vec3 x[4] = {x0, x3, r[2], r[1]};
+			one(t + 1, w, x);
+			x0 = x[0], x3 = x[1], r[2] = x[2], r[1] = x[3];
+		}
+		{
+			const float w[4] = {w0, rw[1], rw[0], w3};
+			Vec3 x[4] = {x0, r[1], r[0], x3};
+			one(t, w, x);
+			x0 = x[0], r[1] = x[1], r[0] = x[2], x3 = x[3];
+		}
+		const Vec3 a = r[4], b = r[5];
+		const float wa = rw[4], wb = rw[5];
+#pragma unroll
+		for (int k = 5; k >= 2; k--) r[k] = r[k - 2], rw[k] = rw[k - 2];
+		r[0] = a, r[1] = b, rw[0] = wa, rw[1] = wb;
+	}
+	xb[0] = x0, xb[3] = x3;
+	// three turns back by two: the places of the first turn again
+	xb[6] = r[0], xb[7] = r[1], xb[2] = r[2], xb[1] = r[3], xb[4] = r[4], xb[5] = r[5];
+}
+
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
+// Warp `wib` (1-7) of the block prepares chunk R at launch substep s, and has
+// the same entries of the substep before it brought to L2 (the tape of a long
+// run comes from HBM).
+__device__ __forceinline__ void reverse_prepare(const DevCtx& C, const AdjCtx& A, RevStage& S, const RevChunk& R,
+                                                uint32_t s, bool first, uint32_t wib, uint32_t lane, float inv_dt2) {
+	const uint32_t hdr = R.hdr[lane];
+	if ((hdr & 15u) == 0u) return;
+	if (wib == 7u) {
+#pragma unroll 4
+		for (uint32_t k = 0; k < 8u; k++) {
+			const uint32_t v = R.vid[k][lane];
+			S.w[k][lane] = __ldcg(&tape_at(C, s, v)->w);
+			if (s > 0u) prefetch_l2(tape_at(C, s - 1u, v));
+			if ((hdr >> (8 + k)) & 1u) {
+				const OwnedTape t = owned_tape(C, A, v, s, first);
+				S.Op[k][lane] = t.Op;
+				S.Ds[k][lane] = t.Ds;
+				S.tip[k][lane] = make_float4(t.tip.x, t.tip.y, t.tip.z, 0.0f);
+			}
+		}
+		return;
+	}
+	const uint32_t j = wib - 1u;
+	const Mat mat = load_mat(C.bodies, hdr >> 16);
+	const float4* r = C.cblk + R.off16 + j * 4 * kLanes + lane;
+	const TetRec tr = {__ldg(r), __ldg(r + kLanes), __ldg(r + 2 * kLanes), __ldg(r + 3 * kLanes)};
+	const uint32_t sl = (uint32_t)(cube_slot((int)j, 0) | cube_slot((int)j, 1) << 4 | cube_slot((int)j, 2) << 8 |
+	                               cube_slot((int)j, 3) << 12);
+	float4 Ot[4];
+#pragma unroll
+	for (int k = 0; k < 4; k++) Ot[k] = __ldcg(tape_at(C, s, R.vid[(sl >> (4 * k)) & 15u][lane]));
+	Vec3 Din[4];
+	load_tet_input(C, s, R.trow + j, lane, Din);
+	if (s > 0u) {
+		const float4* p = C.tape_t + ((size_t)(s - 1u) * C.ntrows + R.trow + j) * 3 * kLanes + lane;
+		prefetch_l2(p);
+		prefetch_l2(p + kLanes);
+		prefetch_l2(p + 2 * kLanes);
+	}
+	TetWords tw;
+	tet_internals(mat, tr, inv_dt2, Ot, Din, tw.f);
+	const float q[8] = {tr.c.y, tr.c.z, tr.c.w, tr.d.x, tr.d.y, tr.d.z, 0.0f, 0.0f};
+#pragma unroll
+	for (int k = 0; k < 8; k++) tw.q[k] = q[k];
+	float4 words[kTetWords4];
+	memcpy(words, &tw, sizeof(tw));
+#pragma unroll
+	for (uint32_t k = 0; k < kTetWords4; k++) S.tet[j][k][lane] = words[k];
+}
+
+__global__ void __launch_bounds__(256, 1) k_reverse_cluster(DevCtx C, AdjCtx A, uint32_t nsub, float dt, int last,
+                                                            uint32_t rounds) {
+	extern __shared__ __align__(128) unsigned char rcmem[];
+	const float inv_dt = 1.0f / dt, inv_dt2 = 1.0f / (dt * dt);
+	const uint32_t lane = threadIdx.x & 31u, wib = threadIdx.x >> 5;
+	const uint32_t G = gridDim.x, rank = blockIdx.x;
+	RevShared& S = *reinterpret_cast<RevShared*>(rcmem);
+	float4* sv = reinterpret_cast<float4*>(rcmem + sizeof(RevShared));
+	const uint32_t per = cluster_verts(C.nverts, G);
+	RevChunk* chunks = reinterpret_cast<RevChunk*>(sv + 2 * (size_t)per);  // [colour][round]
+	const ClusterAdj ab = {ClusterVerts(smem_u32(sv), per)};
+	const uint32_t v0 = min(rank * per, C.nverts), v1 = min(v0 + per, C.nverts);
+	for (uint32_t v = v0 + threadIdx.x; v < v1; v += blockDim.x) {
+		sv[v - v0] = __ldcg(A.abar + 2 * (size_t)v);
+		sv[per + (v - v0)] = __ldcg(A.abar + 2 * (size_t)v + 1);
+		finalize_reverse(C, A, ab, v, nsub, inv_dt, last != 0);
+	}
+	// the block's chunks of each colour, in rounds: [first, end)
+	__shared__ uint32_t s_first[kRevColours], s_end[kRevColours];
+	if (threadIdx.x < C.ncolours) {
+		const uint32_t cb = __ldg(C.colour_chunk_begin + threadIdx.x), n = __ldg(C.colour_chunk_begin + threadIdx.x + 1) - cb;
+		s_first[threadIdx.x] = cb + n * rank / G;
+		s_end[threadIdx.x] = cb + n * (rank + 1u) / G;
+	}
+	__syncthreads();
+	for (uint32_t c = 0; c < C.ncolours; c++)
+		for (uint32_t k = 0; s_first[c] + k < s_end[c]; k++) {
+			RevChunk& R = chunks[c * rounds + k];
+			const uint4 m = __ldg(reinterpret_cast<const uint4*>(C.chunks) + s_first[c] + k);
+			const uint32_t* hdrs = reinterpret_cast<const uint32_t*>(C.cblk + m.x + 4 * kLanes * 6);
+			for (uint32_t i = threadIdx.x; i < 9u * kLanes; i += blockDim.x) (&R.hdr[0])[i] = __ldg(hdrs + i);
+			for (uint32_t i = threadIdx.x; i < 6u * kLanes; i += blockDim.x) (&R.cbar[0][0])[i] = A.cbar[(size_t)m.w * kLanes + i];
+			if (threadIdx.x == 0) R.off16 = m.x, R.trow = m.w;
+		}
+	cluster_barrier();
+	isolated_reverse(C, A, ab, rank * blockDim.x + threadIdx.x, G * blockDim.x, nsub, dt);
+
+	// the block's next chunk after (s, c, k), -1 when there is none
+	auto next_of = [&](int& s, int& c, uint32_t& k) {
+		if (s_first[c] + k + 1u < s_end[c]) {
+			k++;
+			return true;
+		}
+		for (;;) {
+			if (--c < 0) {
+				c = (int)C.ncolours - 1;
+				if (--s < 0) return false;
+			}
+			if (s_first[c] < s_end[c]) {
+				k = 0;
+				return true;
+			}
+		}
+	};
+	// the first chunk of the launch
+	int ns = (int)nsub - 1, nc = (int)C.ncolours - 1;
+	uint32_t nk = 0, it = 0;
+	bool more = s_first[nc] < s_end[nc] || next_of(ns, nc, nk);
+	if (more && wib > 0)
+		reverse_prepare(C, A, S.st[0], chunks[(uint32_t)nc * rounds + nk], (uint32_t)ns, ns == 0, wib, lane, inv_dt2);
+	for (int s = (int)nsub - 1; s >= 0; s--) {
+		for (int c = (int)C.ncolours - 1; c >= 0; c--) {
+			const uint32_t cf = s_first[c], n = s_end[c] - cf;
+			for (uint32_t k = 0; k < n; k++, it++) {
+				__syncthreads();  // the chunk is prepared, the last one finished
+				RevStage& st = S.st[it & 1u];
+				more = next_of(ns, nc, nk);
+				RevChunk& R = chunks[(uint32_t)c * rounds + k];
+				const uint32_t hdr = R.hdr[lane];
+				const bool live = (hdr & 15u) != 0u;
+				if (wib == 0) {
+					if (live) {
+						Vec3 xb[8];
+#pragma unroll
+						for (uint32_t j = 0; j < 8u; j++) xb[j] = ab.xb(R.vid[j][lane]);
+						reverse_cube(st, lane, xb, &R.cbar[0][lane]);
+#pragma unroll
+						for (uint32_t j = 0; j < 8u; j++) S.xb[j][lane] = make_float4(xb[j].x, xb[j].y, xb[j].z, 0.0f);
+					}
+				} else if (more) {
+					reverse_prepare(C, A, S.st[(it + 1u) & 1u], chunks[(uint32_t)nc * rounds + nk], (uint32_t)ns, ns == 0, wib, lane,
+					                inv_dt2);
+				}
+				__syncthreads();
+				// warp j finishes vertex j of each cluster: its advance reverse if
+				// the cluster owns it, else its adjoint
+				if (live) {
+					const uint32_t v = R.vid[wib][lane];
+					const Vec3 x = v3(S.xb[wib][lane]);
+					if ((hdr >> (8 + wib)) & 1u)
+						advance_reverse(C, ab, v, OwnedTape{st.Op[wib][lane], st.Ds[wib][lane], v3(st.tip[wib][lane])}, s == 0, dt, x);
+					else
+						ab.set_xb(v, x);
+				}
+			}
+			cluster_barrier();
+		}
+	}
+	for (uint32_t v = v0 + threadIdx.x; v < v1; v += blockDim.x) {
+		__stcg(A.abar + 2 * (size_t)v, sv[v - v0]);
+		__stcg(A.abar + 2 * (size_t)v + 1, sv[per + (v - v0)]);
+	}
+	for (uint32_t c = 0; c < C.ncolours; c++)
+		for (uint32_t k = 0; s_first[c] + k < s_end[c]; k++) {
+			const RevChunk& R = chunks[c * rounds + k];
+			for (uint32_t i = threadIdx.x; i < 6u * kLanes; i += blockDim.x)
+				A.cbar[(size_t)R.trow * kLanes + i] = (&R.cbar[0][0])[i];
+		}
+}
+
+// Blocks of the one-cluster reverse, 0 when the handle does not take it: all
+// clusters whole cubes, at most 16 colours and at most three chunks of a
+// colour per block (a chunk's chain is a third of a pass of the grid form,
+// which takes any number of chunks up to one per SM in the same time).
+cudaError_t reverse_cluster_blocks(const DevCtx& C, uint32_t max_colour_chunks, uint32_t* blocks, uint32_t* rounds,
+                                   size_t* smem) {
+	*blocks = 0;
+	if (C.vs_off != C.warp_smem || C.ncolours == 0 || C.ncolours > kRevColours || max_colour_chunks == 0) return cudaSuccess;
+	uint32_t G = 1;
+	while (G < 16u && G < max_colour_chunks) G *= 2;
+	*rounds = (max_colour_chunks + G - 1) / G;
+	if (*rounds > 3u) return cudaSuccess;
+	int dev = 0, optin = 0;
+	cudaError_t e = cudaGetDevice(&dev);
+	if (e == cudaSuccess) e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+	const void* f = (const void*)k_reverse_cluster;
+	cudaFuncAttributes fa{};
+	if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, f);
+	if (e != cudaSuccess) return e;
+	*smem = sizeof(RevShared) + 32u * (size_t)cluster_verts(C.nverts, G) + sizeof(RevChunk) * (size_t)C.ncolours * *rounds;
+	if (*smem + fa.sharedSizeBytes > (size_t)optin) return cudaSuccess;
+	e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)fa.sharedSizeBytes);
+	if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+	cudaLaunchAttribute at{};
+	at.id = cudaLaunchAttributeClusterDimension;
+	at.val.clusterDim.x = G;
+	at.val.clusterDim.y = at.val.clusterDim.z = 1;
+	cudaLaunchConfig_t lc{};
+	lc.gridDim = dim3(G);
+	lc.blockDim = dim3(256);
+	lc.dynamicSmemBytes = *smem;
+	lc.attrs = &at;
+	lc.numAttrs = 1;
+	int n = 0;
+	if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&n, f, &lc);
+	if (e == cudaSuccess && n > 0) *blocks = G;
+	return e;
+}
+
 }  // namespace
 
 int configure_adjoint_kernels(int, uint32_t) { return 0; }
@@ -502,6 +844,32 @@ int launch_reverse(const DevCtx& ctx, const AdjCtx& adj, int block, uint32_t, ui
                    float dt, bool last, void* stream) {
 	if (nsub == 0) return 0;
 	cudaStream_t st = (cudaStream_t)stream;
+	const char* form = getenv("XFEM_REVERSE_FORM");
+	// the hooks that make grid-barrier waits run out or wrap need that barrier
+	if (!form && !ctx.wait_miss && !ctx.bar_base) {
+		uint32_t G = 0, rounds = 0;
+		size_t bytes = 0;
+		const cudaError_t ec = reverse_cluster_blocks(ctx, max_colour_chunks, &G, &rounds, &bytes);
+		if (ec != cudaSuccess) return (int)ec;
+		if (G) {
+			cudaLaunchAttribute at{};
+			at.id = cudaLaunchAttributeClusterDimension;
+			at.val.clusterDim.x = G;
+			at.val.clusterDim.y = at.val.clusterDim.z = 1;
+			cudaLaunchConfig_t lc{};
+			lc.gridDim = dim3(G);
+			lc.blockDim = dim3(256);
+			lc.dynamicSmemBytes = bytes;
+			lc.stream = st;
+			lc.attrs = &at;
+			lc.numAttrs = 1;
+			DevCtx c = ctx;
+			AdjCtx a = adj;
+			int lastv = last ? 1 : 0;
+			void* args[] = {&c, &a, &nsub, &dt, &lastv, &rounds};
+			return (int)cudaLaunchKernelExC(&lc, (const void*)k_reverse_cluster, args);
+		}
+	}
 	int dev = 0, sms = 0, per_sm = 0;
 	// six forward-internal slots per 8-lane group, 4 groups per warp
 	const size_t smem = (size_t)(block / 32) * 24 * sizeof(TetSlot);
@@ -523,7 +891,7 @@ int launch_reverse(const DevCtx& ctx, const AdjCtx& adj, int block, uint32_t, ui
 	// the grouped form when one round of the grid's warps takes every part of
 	// the largest colour pass
 	int grouped = (uint64_t)max_colour_chunks * 8u <= (uint64_t)blocks * (uint32_t)(block / 32) ? 1 : 0;
-	if (const char* f = getenv("XFEM_REVERSE_FORM")) grouped = f[0] == 'g' ? 1 : f[0] == 'l' ? 0 : grouped;
+	if (form) grouped = form[0] == 'g' ? 1 : form[0] == 'l' ? 0 : grouped;
 	void* args[] = {&c, &a, &nsub, &dt, &lastv, &grouped};
 	return (int)cudaLaunchCooperativeKernel((const void*)k_reverse, dim3(blocks), dim3(block), args, smem, st);
 }

@@ -37,13 +37,6 @@ namespace {
 constexpr uint32_t kClusterBufs = 8;     // chunk buffers of a warp, at most
 constexpr uint32_t kClusterColours = 24;  // colours whose chunk descriptors sit in shared memory
 
-// Vertices each block holds (at least 2: ClusterVerts divides by a 32-bit
-// reciprocal).
-XFEM_HD uint32_t cluster_verts(uint32_t nverts, uint32_t blocks) {
-	const uint32_t per = (nverts + blocks - 1) / blocks;
-	return per < 2u ? 2u : per;
-}
-
 // A warp's shared memory: its chunk buffers, then the vertex slots.
 XFEM_HD uint32_t cluster_warp_bytes(uint32_t vs_off, uint32_t warp_smem, uint32_t bufs) {
 	return bufs * vs_off + (warp_smem - vs_off);
@@ -77,7 +70,7 @@ __global__ void __launch_bounds__(256) k_cluster(DevCtx C, ClusterPlan plan, uin
 	const uint32_t wbytes = cluster_warp_bytes(C.vs_off, C.warp_smem, nbuf);
 	float4* sv = reinterpret_cast<float4*>(smem + (size_t)plan.warps * wbytes);
 	const uint32_t per = cluster_verts(C.nverts, G);
-	const ClusterVerts vs = {smem_u32(sv), per, (uint32_t)((0x100000000ull + per - 1u) / per)};
+	const ClusterVerts vs(smem_u32(sv), per);
 	const uint32_t v0 = min(r * per, C.nverts), v1 = min(v0 + per, C.nverts);
 	for (uint32_t v = v0 + threadIdx.x; v < v1; v += blockDim.x) {
 		float4 O, D;

@@ -137,8 +137,17 @@ struct GlobalVerts {
 	}
 };
 
+// Vertices each block of a one-cluster launch holds (at least 2: ClusterVerts divides by a 32-bit
+// reciprocal).
+XFEM_HD uint32_t cluster_verts(uint32_t nverts, uint32_t blocks) {
+	const uint32_t per = (nverts + blocks - 1) / blocks;
+	return per < 2u ? 2u : per;
+}
+
 struct ClusterVerts {
 	uint32_t base, per, inv;  // shared address in every block, vertices per block, ceil(2^32 / per)
+	__device__ __forceinline__ ClusterVerts(uint32_t b, uint32_t p)
+	    : base(b), per(p), inv((uint32_t)((0x100000000ull + p - 1u) / p)) {}
 
 	__device__ __forceinline__ uint32_t at(uint32_t v) const {
 		const uint32_t r = __umulhi(v, inv);  // v / per: v * per < 2^32
