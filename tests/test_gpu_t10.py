@@ -230,3 +230,31 @@ def test_t10_errors():
         assert ex.value.code == xfem.EUNSUPPORTED
     b.step_frames(1, 4, DT)
     assert np.isfinite(b.positions()).all()
+
+
+@pytest.mark.parametrize("volume_passes", [0, 2])
+def test_bodies_of_every_energy_share_a_warp(volume_passes):
+    """Eight T10s of a colour share a warp, four lanes each, whatever their
+    bodies' energies: small bodies of every energy, coupled and serial, damped
+    in the solve, after it and not at all, in one handle step as alone."""
+    meshes, settings = [], []
+    for k, energy in enumerate((4, 0, 7, 3, 1, 6, 2, 5, 11, 4, 7, 3, 0, 31)):
+        dims = ((1, 1, 1), (2, 1, 1), (3, 2, 1))[k % 3]
+        nodes, idx = xfem.generate_tet_block(*dims, (0.1, 0.1, 0.1), k % 2, 0.2)
+        rtype = k % 4
+        s = xfem.default_settings(gravity=(0.3, -9.81, -2.0), compliance=4e-5 * (1 + k), poissons_ratio=0.45,
+                                  damping=0.0 if k % 3 == 0 else 0.003, pbd_damping=0.02 * (k % 2),
+                                  volume_and_time_corrected_pbd_damping=0.01,
+                                  amortized_volume_and_time_corrected_pbd_damping=0.05, volume_passes=volume_passes * (k % 2),
+                                  flags=xfem.ELEMENT_T10 | (energy << xfem.ENERGY_BIT) | (rtype << 20) | xfem.LOCK_LEFT |
+                                  ((k % 5 != 1) << xfem.XPBD_SOLVE_BIT))
+        meshes.append((nodes, idx, 1000.0))
+        settings.append(s)
+    batch = xfem.Body(meshes=meshes, settings=settings)
+    batch.step_frames(1, 11, DT)
+    for k, (m, s) in enumerate(zip(meshes, settings)):
+        one = xfem.Body(*m, s)
+        one.step_frames(1, 11, DT)
+        assert np.array_equal(one.positions(), batch.positions(k)), k
+        assert np.array_equal(one.velocities(), batch.velocities(k)), k
+        assert np.isfinite(one.positions()).all()

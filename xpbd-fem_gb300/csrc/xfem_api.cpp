@@ -1977,10 +1977,10 @@ int launch_mode(xfem_body* h, const DevCtx& ctx, uint32_t nsub, float dt) {
 		if (e) return fail(XFEM_ECUDA, std::string("element launch: ") + cudaGetErrorString((cudaError_t)e));
 		return XFEM_OK;
 	}
-	const int e = h->el_mode == kElH27     ? launch_h27(ctx, 256, nsub, dt, h->stream)
-	              : h->el_mode == kElT10   ? launch_t10(ctx, 256, nsub, dt, h->stream)
+	const int e = h->el_mode == kElH27     ? launch_h27(ctx, nsub, dt, h->stream)
+	              : h->el_mode == kElT10   ? launch_t10(ctx, nsub, dt, h->stream)
 	              : h->el_mode == kElMixed ? launch_mixed(ctx, 256, nsub, dt, h->stream)
-	                                       : launch_hexes(ctx, 256, nsub, dt, h->stream);
+	                                       : launch_hexes(ctx, nsub, dt, h->stream);
 	if (e) return fail(XFEM_ECUDA, std::string("element launch: ") + cudaGetErrorString((cudaError_t)e));
 	return XFEM_OK;
 }

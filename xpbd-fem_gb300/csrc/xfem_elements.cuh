@@ -210,14 +210,14 @@ __device__ __forceinline__ bool in_slice(const DevCtx& C, const BodyParams& bp, 
 	return f >= nh * m / 8u && f < nh * (m + 1u) / 8u;
 }
 
-// Calls f(i, live) on the elements [b, e) of a colour, LANES lanes of a warp
-// per element (32 / LANES elements per warp). Consecutive warps' worth of
-// elements go to consecutive blocks, so that a pass with fewer elements than
-// threads still spreads over every SM (230,400 T10s, about 10,000 per colour,
-// one lane each, sat on 39 of 152 SMs: 6,019 -> 4,202 us per frame; 262,144
-// hexes 1,042 -> 975; 28,800 H27s 3,089 -> 2,931). With 2 to 16 lanes per
-// element every lane of the warp calls f together, a group past the end with
-// the last element and live = false.
+// Calls f(i, last, live) on the elements [b, e) of a colour, LANES lanes of a
+// warp per element (32 / LANES elements per warp; last = e - 1). Consecutive
+// warps' worth of elements go to consecutive blocks, so that a pass with fewer
+// elements than threads still spreads over every SM (230,400 T10s, about
+// 10,000 per colour, one lane each, sat on 39 of 152 SMs: 6,019 -> 4,202 us per
+// frame; 262,144 hexes 1,042 -> 975; 28,800 H27s 3,089 -> 2,931). With 2 to 16
+// lanes per element every lane of the warp calls f together with the warp's
+// first element, live = whether its own group's is one of the colour.
 constexpr uint32_t kNoElem = 0xffffffffu;
 template <int LANES, class F>
 __device__ __forceinline__ void for_elements(uint32_t b, uint32_t e, F f) {
@@ -225,10 +225,19 @@ __device__ __forceinline__ void for_elements(uint32_t b, uint32_t e, F f) {
 	const uint32_t gwarp = (threadIdx.x >> 5) * gridDim.x + blockIdx.x, nwarps = (blockDim.x >> 5) * gridDim.x;
 	const uint32_t sub = (threadIdx.x & 31u) / LANES;
 	if constexpr (LANES == 1 || LANES == 32) {
-		for (uint32_t i = b + gwarp * n + sub; i < e; i += nwarps * n) f(i, true);
+		for (uint32_t i = b + gwarp * n + sub; i < e; i += nwarps * n) f(i, e - 1u, true);
 	} else {
-		for (uint32_t i0 = b + gwarp * n; i0 < e; i0 += nwarps * n) f(min(i0 + sub, e - 1u), i0 + sub < e);
+		for (uint32_t i0 = b + gwarp * n; i0 < e; i0 += nwarps * n) f(i0, e - 1u, i0 + sub < e);
 	}
+}
+
+// The element that a lane's group works on in f of for_elements.
+template <class E>
+__device__ __forceinline__ uint32_t elem_of(uint32_t i, uint32_t last) {
+	if constexpr (E::kLanes == 1 || E::kLanes == 32)
+		return i;
+	else
+		return min(i + (threadIdx.x & 31u) / E::kLanes, last);
 }
 
 template <class E>
@@ -249,11 +258,11 @@ __device__ __forceinline__ bool any_live(bool live) {
 
 // The persistent element kernel (cooperative launch, co-resident grid). E:
 // the element type (kVid4 uint4 of vertex ids per element; pass<KIND>(C, i,
-// live, ...) by kLanes lanes of a warp per element, pbd by kPbdLanes;
-// kMinBlocks: the blocks per SM the register budget is sized for; smem(), the
+// last, live, ...) by kLanes lanes of a warp per element, pbd by kPbdLanes;
+// kBlock threads, kMinBlocks blocks per SM: what registers are sized for; smem(), the
 // dynamic shared memory of a block, set up by init).
 template <class E>
-__global__ void __launch_bounds__(256, E::kMinBlocks) k_elements(DevCtx C, uint32_t nsub, float dt) {
+__global__ void __launch_bounds__(E::kBlock, E::kMinBlocks) k_elements(DevCtx C, uint32_t nsub, float dt) {
 	const float inv_dt = 1.0f / dt, inv_dt2 = 1.0f / (dt * dt);
 	const uint32_t gtid = blockIdx.x * blockDim.x + threadIdx.x, nthreads = gridDim.x * blockDim.x;
 	E::init(C);
@@ -270,29 +279,34 @@ __global__ void __launch_bounds__(256, E::kMinBlocks) k_elements(DevCtx C, uint3
 		if (!grid_sync(C, target)) return;
 		for (uint32_t c = 0; c < C.el_colours; c++) {
 			const uint32_t b = __ldg(C.colour_el_begin + c), e = __ldg(C.colour_el_begin + c + 1);
-			if constexpr (E::kLanes == 32) {
-				// one warp per element: its next element is fetched ahead
+			if constexpr (E::kLanes > 1) {
+				// several lanes per element: the warp's next elements are fetched ahead
+				constexpr uint32_t n = 32u / E::kLanes;
 				const uint32_t gwarp = (threadIdx.x >> 5) * gridDim.x + blockIdx.x, nwarps = nthreads >> 5;
-				for (uint32_t i = b + gwarp; i < e; i += nwarps) {
-					uint32_t next = i + nwarps;
+				for (uint32_t i = b + gwarp * n; i < e; i += nwarps * n) {
+					uint32_t next = i + nwarps * n, next_end = e;
 					if (next >= e) {
 						const uint32_t c2 = c + 1 < C.el_colours ? c + 1 : 0;
-						next = __ldg(C.colour_el_begin + c2) + gwarp;
-						if (next >= __ldg(C.colour_el_begin + c2 + 1) || (c2 == 0 && s + 1 == nsub)) next = kNoElem;
+						next = __ldg(C.colour_el_begin + c2) + gwarp * n;
+						next_end = __ldg(C.colour_el_begin + c2 + 1);
+						if (next >= next_end || (c2 == 0 && s + 1 == nsub)) next = kNoElem;
 					}
-					E::template pass<kSolve>(C, i, true, inv_dt, inv_dt2, 0.0f, next);
+					E::template pass<kSolve>(C, i, e - 1u, i + (threadIdx.x & 31u) / E::kLanes < e, inv_dt, inv_dt2, 0.0f, next,
+					                         next_end - 1u);
 				}
 			} else {
-				for_elements<E::kLanes>(b, e, [&](uint32_t i, bool live) { E::template pass<kSolve>(C, i, live, inv_dt, inv_dt2, 0.0f); });
+				for_elements<E::kLanes>(b, e, [&](uint32_t i, uint32_t last, bool live) {
+					E::template pass<kSolve>(C, i, last, live, inv_dt, inv_dt2, 0.0f);
+				});
 			}
 			if (!grid_sync(C, target)) return;
 		}
 		for (uint32_t it = 0; it < C.nvol; it++)
 			for (uint32_t c = 0; c < C.el_colours; c++) {
 				const uint32_t b = __ldg(C.colour_el_begin + c), e = __ldg(C.colour_el_begin + c + 1);
-				for_elements<E::kLanes>(b, e, [&](uint32_t i, bool live) {
-					live = live && it < __ldg(&body_of_el<E>(C, i).volume_passes);
-					if (any_live<E>(live)) E::template pass<kVolume>(C, i, live, inv_dt, inv_dt2, 0.0f);
+				for_elements<E::kLanes>(b, e, [&](uint32_t i, uint32_t last, bool live) {
+					live = live && it < __ldg(&body_of_el<E>(C, elem_of<E>(i, last)).volume_passes);
+					if (any_live<E>(live)) E::template pass<kVolume>(C, i, last, live, inv_dt, inv_dt2, 0.0f);
 				});
 				if (!grid_sync(C, target)) return;
 			}
@@ -308,19 +322,20 @@ __global__ void __launch_bounds__(256, E::kMinBlocks) k_elements(DevCtx C, uint3
 		if (C.damp_kinds & 1u)
 			for (uint32_t c = 0; c < C.el_colours; c++) {
 				const uint32_t b = __ldg(C.colour_el_begin + c), e = __ldg(C.colour_el_begin + c + 1);
-				for_elements<E::kLanes>(b, e, [&](uint32_t i, bool live) {
-					const BodyParams& bp = body_of_el<E>(C, i);
+				for_elements<E::kLanes>(b, e, [&](uint32_t i, uint32_t last, bool live) {
+					const uint32_t own = elem_of<E>(i, last);
+					const BodyParams& bp = body_of_el<E>(C, own);
 					const uint32_t type = __ldg(&bp.rayleigh_type);
 					const float rd = __ldg(&bp.damping) * (type == 3u ? 8.0f : 1.0f);
-					live = live && type >= 2u && rd > 0.0f && in_slice(C, bp, i, tick);
-					if (any_live<E>(live)) E::template pass<kRayleigh>(C, i, live, inv_dt, inv_dt2, rd);
+					live = live && type >= 2u && rd > 0.0f && in_slice(C, bp, own, tick);
+					if (any_live<E>(live)) E::template pass<kRayleigh>(C, i, last, live, inv_dt, inv_dt2, rd);
 				});
 				if (!grid_sync(C, target)) return;
 			}
 		if (C.damp_kinds & 2u)
 			for (uint32_t c = 0; c < C.el_colours; c++) {
 				const uint32_t b = __ldg(C.colour_el_begin + c), e = __ldg(C.colour_el_begin + c + 1);
-				for_elements<E::kPbdLanes>(b, e, [&](uint32_t i, bool) {
+				for_elements<E::kPbdLanes>(b, e, [&](uint32_t i, uint32_t, bool) {
 					const BodyParams& bp = body_of_el<E>(C, i);
 					if (__ldg(&bp.pbd_on) && in_slice(C, bp, i, tick))
 						E::pbd(C, i, __ldg(&bp.rayleigh_type) == 3u ? __ldg(&bp.pbd_coeff_amortized) : __ldg(&bp.pbd_coeff));
@@ -340,8 +355,9 @@ __global__ void __launch_bounds__(256, E::kMinBlocks) k_elements(DevCtx C, uint3
 }
 
 template <class E>
-int launch_elements(const DevCtx& ctx, int block, uint32_t nsub, float dt, void* stream) {
+int launch_elements(const DevCtx& ctx, uint32_t nsub, float dt, void* stream) {
 	if (nsub == 0) return 0;
+	constexpr int block = E::kBlock;
 	cudaStream_t st = (cudaStream_t)stream;
 	const void* f = (const void*)k_elements<E>;
 	int dev = 0, sms = 0, per_sm = 0;

@@ -263,9 +263,8 @@ int launch_h27_rings(const DevCtx& ctx, int block, uint32_t nsub, float dt, void
 	return (int)cudaLaunchCooperativeKernel(f, dim3(per_sm * sms), dim3(block), args, smem, st);
 }
 
-int launch_h27(const DevCtx& ctx, int block, uint32_t nsub, float dt, void* stream) {
-	if (block != 256) return (int)cudaErrorInvalidConfiguration;  // the per-warp scratch is sized for 8 warps
-	return launch_elements<h27e::H27Elem>(ctx, block, nsub, dt, stream);
+int launch_h27(const DevCtx& ctx, uint32_t nsub, float dt, void* stream) {
+	return launch_elements<h27e::H27Elem>(ctx, nsub, dt, stream);
 }
 
 }  // namespace xfem

@@ -354,13 +354,18 @@ __device__ __forceinline__ void move2(Elem& E, float l0, const Vec3& g0, float l
 	E.D.z = fmaf(s1, g1.z, fmaf(s0, g0.z, E.D.z));
 }
 
+// Where a block's dynamic shared memory holds this mode's part (after the
+// T10s' on meshes mixing both).
+#ifndef XFEM_H27_SMEM_AT
+#define XFEM_H27_SMEM_AT 0
+#endif
 struct Shared {
 	Tables t;
 	Scratch s[8];  // 256-thread blocks: 8 warps
 };
 __device__ __forceinline__ Shared& shared() {
 	extern __shared__ __align__(128) unsigned char h27_smem[];
-	return *reinterpret_cast<Shared*>(h27_smem);
+	return *reinterpret_cast<Shared*>(h27_smem + XFEM_H27_SMEM_AT);
 }
 
 // Starts the copy of element i's record and vertex ids into the warp's
@@ -558,6 +563,7 @@ __device__ __noinline__ void h27_pbd(const DevCtx& C, uint32_t i, float coeff) {
 
 struct H27Elem {
 	static constexpr int kLanes = 32, kPbdLanes = 32;
+	static constexpr int kBlock = 256;
 	static constexpr int kMinBlocks = 3;  // at most 85 registers: three 256-thread blocks per SM
 	static constexpr uint32_t kVid4 = 7;
 	static constexpr size_t smem() { return sizeof(Shared); }
@@ -566,8 +572,8 @@ struct H27Elem {
 		load_tables(C, shared().t);
 	}
 	template <int KIND>
-	__device__ static void pass(const DevCtx& C, uint32_t i, bool, float inv_dt, float inv_dt2, float rd,
-	                            uint32_t next = kNoElem) {
+	__device__ static void pass(const DevCtx& C, uint32_t i, uint32_t, bool, float inv_dt, float inv_dt2, float rd,
+	                            uint32_t next = kNoElem, uint32_t = 0) {
 		h27_pass<KIND>(C, i, next, inv_dt, inv_dt2, rd);
 	}
 	__device__ static void pbd(const DevCtx& C, uint32_t i, float coeff) { h27_pbd(C, i, coeff); }

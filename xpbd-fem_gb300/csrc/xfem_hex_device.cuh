@@ -557,12 +557,12 @@ __device__ __noinline__ void hex_pbd(const DevCtx& C, uint32_t i, float coeff) {
 
 struct HexElem {
 	static constexpr int kLanes = 1, kPbdLanes = 1;
-	static constexpr int kMinBlocks = 1;
+	static constexpr int kBlock = 256, kMinBlocks = 1;
 	static constexpr uint32_t kVid4 = 2;
 	static constexpr size_t smem() { return 0; }
 	__device__ static void init(const DevCtx&) {}
 	template <int KIND>
-	__device__ static void pass(const DevCtx& C, uint32_t i, bool, float inv_dt, float inv_dt2, float rd) {
+	__device__ static void pass(const DevCtx& C, uint32_t i, uint32_t, bool, float inv_dt, float inv_dt2, float rd) {
 		hex_pass<KIND>(C, i, inv_dt, inv_dt2, rd);
 	}
 	__device__ static void pbd(const DevCtx& C, uint32_t i, float coeff) { hex_pbd(C, i, coeff); }

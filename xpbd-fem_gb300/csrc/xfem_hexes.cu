@@ -273,8 +273,8 @@ __global__ void __launch_bounds__(256) k_hex_rings(DevCtx C, uint32_t nsub, floa
 
 }  // namespace
 
-int launch_hexes(const DevCtx& ctx, int block, uint32_t nsub, float dt, void* stream) {
-	return launch_elements<HexElem>(ctx, block, nsub, dt, stream);
+int launch_hexes(const DevCtx& ctx, uint32_t nsub, float dt, void* stream) {
+	return launch_elements<HexElem>(ctx, nsub, dt, stream);
 }
 
 int launch_hex_rings(const DevCtx& ctx, int block, uint32_t nsub, float dt, void* stream) {

@@ -527,7 +527,7 @@ int launch_volume(const float4* vert, const uint32_t* tets_dev, uint32_t nt, dou
 int launch_rings(const DevCtx& ctx, uint32_t nsub, float dt, void* stream);
 // Hex mode (xfem_hexes.cu): nsub substeps of a hex mesh, a cooperative
 // persistent launch (canonical (X, V) in and out).
-int launch_hexes(const DevCtx& ctx, int block, uint32_t nsub, float dt, void* stream);
+int launch_hexes(const DevCtx& ctx, uint32_t nsub, float dt, void* stream);
 // The continuous-pressure models on a hex mesh (xfem_hexes.cu): nsub
 // substeps of one-ring solves over the hexes, a cooperative persistent
 // launch (canonical (X, V) in and out).
@@ -536,7 +536,7 @@ int launch_hex_rings(const DevCtx& ctx, int block, uint32_t nsub, float dt, void
 // colour then every hex colour per sweep, a cooperative persistent launch.
 int launch_mixed(const DevCtx& ctx, int block, uint32_t nsub, float dt, void* stream);
 // Quadratic-tet mode (xfem_t10.cu): nsub substeps of a T10 mesh, likewise.
-int launch_t10(const DevCtx& ctx, int block, uint32_t nsub, float dt, void* stream);
+int launch_t10(const DevCtx& ctx, uint32_t nsub, float dt, void* stream);
 // The continuous-pressure models on a T10 mesh (xfem_t10.cu): nsub substeps
 // of one-ring solves over the T10s around the mesh vertices, a cooperative
 // persistent launch (canonical (X, V) in and out).
@@ -547,7 +547,7 @@ int launch_h27_rings(const DevCtx& ctx, int block, uint32_t nsub, float dt, void
 int launch_qmixed(const DevCtx& ch27, const DevCtx& ct10, int block, uint32_t nsub, float dt, void* stream);
 // Quadratic-hex mode (xfem_h27.cu): nsub substeps of an H27 mesh, one warp
 // per element (block must be 256).
-int launch_h27(const DevCtx& ctx, int block, uint32_t nsub, float dt, void* stream);
+int launch_h27(const DevCtx& ctx, uint32_t nsub, float dt, void* stream);
 // Per-tet material (n tets from the given per-tet tables): c0 of each record
 // and 1/mu; mu null = mu_uniform for all.
 int launch_set_c0(float4* cblk, const uint32_t* rec, const float* vol, const float* mu, float mu_uniform, uint32_t n,

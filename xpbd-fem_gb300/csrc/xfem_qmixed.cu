@@ -5,12 +5,13 @@
 // damping over the T10s then the H27s, then the PBD damping over the T10s
 // then the H27s, each over the amortized slice of its own order. Here each
 // kind keeps its own colouring and its own element arrays, so a sweep is the
-// T10 colours (one thread per T10, the T10 mode's code) followed by the H27
+// T10 colours (four lanes per T10, the T10 mode's code) followed by the H27
 // colours (one warp per H27, the H27 mode's code), each behind the grid
 // barrier. The kernel takes two contexts that differ only in their element
 // arrays: Ct holds the T10s, Ch the H27s.
-#include "xfem_h27_elem.cuh"
 #include "xfem_t10_elem.cuh"
+#define XFEM_H27_SMEM_AT sizeof(t10e::QuadShared)
+#include "xfem_h27_elem.cuh"
 
 namespace xfem {
 
@@ -28,6 +29,9 @@ __device__ __forceinline__ bool in_slice_n(const DevCtx& C, const BodyParams& bp
 	return f >= n * m / 8u && f < n * (m + 1u) / 8u;
 }
 
+// the T10s' shared memory, then the H27s' (their code finds its own at an offset)
+constexpr size_t kQMixedSmem = T10::smem() + H27::smem();
+
 constexpr int kPbd = 100;  // the PBD damping sweep (not a pass kind of the elements)
 
 // One pass kind over the colours of one element kind; false when a barrier
@@ -37,20 +41,21 @@ __device__ __forceinline__ bool sweep(const DevCtx& C, const DevCtx& B, float in
                                       uint32_t tick, uint32_t& target) {
 	for (uint32_t c = 0; c < C.el_colours; c++) {
 		const uint32_t b = __ldg(C.colour_el_begin + c), e = __ldg(C.colour_el_begin + c + 1);
-		for_elements<KIND == kPbd ? E::kPbdLanes : E::kLanes>(b, e, [&](uint32_t i, bool live) {
+		for_elements<KIND == kPbd ? E::kPbdLanes : E::kLanes>(b, e, [&](uint32_t i, uint32_t last, bool live) {
 			if constexpr (KIND == kSolve) {
-				E::template pass<kSolve>(C, i, live, inv_dt, inv_dt2, 0.0f);
+				E::template pass<kSolve>(C, i, last, live, inv_dt, inv_dt2, 0.0f);
 			} else {
-				const BodyParams& bp = body_of_el<E>(C, i);
+				const uint32_t own = KIND == kPbd ? i : elem_of<E>(i, last);
+				const BodyParams& bp = body_of_el<E>(C, own);
 				const uint32_t n = E::kVid4 == 7 ? __ldg(&bp.nhexes) : __ldg(&bp.ntets);
 				if constexpr (KIND == kVolume) {
 					live = live && it < __ldg(&bp.volume_passes);
-					if (any_live<E>(live)) E::template pass<kVolume>(C, i, live, inv_dt, inv_dt2, 0.0f);
+					if (any_live<E>(live)) E::template pass<kVolume>(C, i, last, live, inv_dt, inv_dt2, 0.0f);
 				} else if constexpr (KIND == kRayleigh) {
 					const uint32_t type = __ldg(&bp.rayleigh_type);
 					const float rd = __ldg(&bp.damping) * (type == 3u ? 8.0f : 1.0f);
-					live = live && type >= 2u && rd > 0.0f && in_slice_n(C, bp, i, n, tick);
-					if (any_live<E>(live)) E::template pass<kRayleigh>(C, i, live, inv_dt, inv_dt2, rd);
+					live = live && type >= 2u && rd > 0.0f && in_slice_n(C, bp, own, n, tick);
+					if (any_live<E>(live)) E::template pass<kRayleigh>(C, i, last, live, inv_dt, inv_dt2, rd);
 				} else if (__ldg(&bp.pbd_on) && in_slice_n(C, bp, i, n, tick)) {
 					E::pbd(C, i, __ldg(&bp.rayleigh_type) == 3u ? __ldg(&bp.pbd_coeff_amortized) : __ldg(&bp.pbd_coeff));
 				}
@@ -66,6 +71,7 @@ __global__ void __launch_bounds__(256, 1) k_qmixed(DevCtx Ch, DevCtx Ct, uint32_
 	const uint32_t gtid = blockIdx.x * blockDim.x + threadIdx.x, nthreads = gridDim.x * blockDim.x;
 	const uint32_t tick0 = __ldcg(Ch.tick);
 	const bool dmode = Ch.damp_kinds != 0u;
+	T10::init(Ct);
 	H27::init(Ch);
 	uint32_t target = Ch.bar_base;
 	for (uint32_t s = 0; s < nsub; s++) {
@@ -122,15 +128,15 @@ int launch_qmixed(const DevCtx& ch27, const DevCtx& ct10, int block, uint32_t ns
 	cudaError_t e = cudaGetDevice(&dev);
 	if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
 	if (e == cudaSuccess)
-		e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)H27::smem());
-	if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f, block, H27::smem());
+		e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kQMixedSmem);
+	if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f, block, kQMixedSmem);
 	if (e != cudaSuccess) return (int)e;
 	if (per_sm <= 0) return (int)cudaErrorInvalidConfiguration;
 	e = reset_barrier(ch27, st);
 	if (e != cudaSuccess) return (int)e;
 	DevCtx a = ch27, b = ct10;
 	void* args[] = {&a, &b, &nsub, &dt};
-	return (int)cudaLaunchCooperativeKernel(f, dim3(per_sm * sms), dim3(block), args, H27::smem(), st);
+	return (int)cudaLaunchCooperativeKernel(f, dim3(per_sm * sms), dim3(block), args, kQMixedSmem, st);
 }
 
 }  // namespace xfem

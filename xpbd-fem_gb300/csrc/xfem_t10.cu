@@ -5,13 +5,13 @@
 // :437-564 with Nodes = 10 and the 4-point rule, PointsLo = PointsHi = 4; the
 // cube models leave a tet alone), SolveVolumeOnly (:840-867), DampElement
 // (:910-928) and PbdDamp (XPBDFEM/Xpbd.h:306-346), in the element kernel of
-// xfem_elements.cuh with one thread per T10.
+// xfem_elements.cuh with four lanes of a warp per T10.
 //
-// Records: 15 float4 per T10 as a structure of arrays (float4 k of element i
+// Records: 14 float4 per T10 as a structure of arrays (float4 k of element i
 // at el_rec[k * nel + i]): Qi column-major, volume, surface area, the
 // prefactored QQ[9] and QR[36]. The map from the corners is linear, so one
 // Qi serves all four points; their shape-function gradients come from a
-// 120-float table (el_tab) that every thread reads at the same addresses.
+// 120-float table (el_tab).
 #include "xfem_ring_update.cuh"
 #include "xfem_t10_elem.cuh"
 
@@ -309,8 +309,8 @@ int launch_t10_rings(const DevCtx& ctx, int block, uint32_t nsub, float dt, void
 	return (int)cudaLaunchCooperativeKernel(f, dim3(per_sm * sms), dim3(block), args, smem, st);
 }
 
-int launch_t10(const DevCtx& ctx, int block, uint32_t nsub, float dt, void* stream) {
-	return launch_elements<t10e::T10Elem>(ctx, block, nsub, dt, stream);
+int launch_t10(const DevCtx& ctx, uint32_t nsub, float dt, void* stream) {
+	return launch_elements<t10e::T10Elem>(ctx, nsub, dt, stream);
 }
 
 }  // namespace xfem
