@@ -258,3 +258,28 @@ def test_bodies_of_every_energy_share_a_warp(volume_passes):
         assert np.array_equal(one.positions(), batch.positions(k)), k
         assert np.array_equal(one.velocities(), batch.velocities(k)), k
         assert np.isfinite(one.positions()).all()
+
+
+def test_a_colour_beyond_one_round_steps_like_a_small_one():
+    """Meshes whose largest colour needs a second round of four-lane warps take
+    a lane per T10 (xfem_t10_lane.cu): a batch large enough for that steps its
+    bodies as each alone (four lanes) does."""
+    meshes, settings = [], []
+    for k in range(48):
+        nodes, idx = xfem.generate_tet_block(12, 10, 9, (0.1, 0.1, 0.1), 0, 0.2)
+        s = xfem.default_settings(gravity=(0.3, -9.81, -2.0), compliance=4e-5 * (1 + k % 3), poissons_ratio=0.45,
+                                  damping=0.002 * (k == 1), volume_passes=int(k == 2), pbd_damping=0.02 * (k == 3),
+                                  volume_and_time_corrected_pbd_damping=0.01,
+                                  flags=xfem.ELEMENT_T10 | ((4, 7, 3)[k % 3] << xfem.ENERGY_BIT) | (2 << 20) |
+                                  xfem.LOCK_LEFT | ((k != 5) << xfem.XPBD_SOLVE_BIT))
+        meshes.append((nodes, idx, 1000.0))
+        settings.append(s)
+    batch = xfem.Body(meshes=meshes, settings=settings)
+    sched = np.diff(batch.t10_schedule()["colour_t10_begin"]).max() * len(meshes)
+    assert sched > 8 * 12 * 160
+    batch.step_frames(1, 3, DT)
+    for k in range(6):
+        one = xfem.Body(*meshes[k], settings[k])
+        one.step_frames(1, 3, DT)
+        assert np.array_equal(one.positions(), batch.positions(k)), k
+        assert np.array_equal(one.velocities(), batch.velocities(k)), k

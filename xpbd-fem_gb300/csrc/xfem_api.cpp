@@ -1045,6 +1045,7 @@ static int build_element_set(xfem_body* h, uint32_t kind, bool qt) {
 	} else {
 		h->ctx.el_colours = ncol;
 		h->ctx.nel = nel;
+		for (uint32_t c = 0; c < ncol; c++) h->ctx.max_colour_el = std::max(h->ctx.max_colour_el, cb[c + 1] - cb[c]);
 	}
 	h->device_bytes += vid.size() * 16 + rec.size() * 16 + cb.size() * 4 + flat.size() * 4 + g4.size() * 4;
 	return XFEM_OK;

@@ -366,6 +366,7 @@ struct DevCtx {
 	const uint4* el_vid;
 	const float4* el_rec;
 	const uint32_t* colour_el_begin;  // el_colours + 1
+	uint32_t max_colour_el;           // elements of the largest colour
 	const uint32_t* el_flat;
 	uint32_t nel;
 	uint32_t mt_colours;
@@ -537,6 +538,7 @@ int launch_hex_rings(const DevCtx& ctx, int block, uint32_t nsub, float dt, void
 int launch_mixed(const DevCtx& ctx, int block, uint32_t nsub, float dt, void* stream);
 // Quadratic-tet mode (xfem_t10.cu): nsub substeps of a T10 mesh, likewise.
 int launch_t10(const DevCtx& ctx, uint32_t nsub, float dt, void* stream);
+int launch_t10_lane(const DevCtx& ctx, uint32_t nsub, float dt, void* stream);  // one lane per T10
 // The continuous-pressure models on a T10 mesh (xfem_t10.cu): nsub substeps
 // of one-ring solves over the T10s around the mesh vertices, a cooperative
 // persistent launch (canonical (X, V) in and out).
