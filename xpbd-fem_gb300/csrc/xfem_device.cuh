@@ -689,12 +689,12 @@ __device__ __forceinline__ float2 solve_tet(const Mat& bp, const TetRec& r, floa
 	return make_float2(l0, l1);
 }
 
-// The six solves of a whole-cube cluster in sequence, on the cluster's eight
-// vertices (local slots; only D's xyz changes). The cube's tets turn around
-// its diagonal (slots 0 and 3): tet t shares one vertex P with the tet before
-// it and brings one vertex N of the ring 2 1 4 5 6 7 (2), in the slots
-// (0, N, P, 3) for even t and (0, 3, N, P) for odd t. So the six run as three
-// turns of one loop of two solves, the ring moved by two places per turn.
+// Calls f(t, Ot, Dt) on the six tets of a whole-cube cluster in sequence, on the
+// cluster's eight vertices (local slots; f changes only Dt's xyz). The cube's
+// tets turn around its diagonal (slots 0 and 3): tet t shares one vertex P with
+// the tet before it and brings one vertex N of the ring 2 1 4 5 6 7 (2), in the
+// slots (0, N, P, 3) for even t and (0, 3, N, P) for odd t. So the six run as
+// three turns of one loop of two, the ring moved by two places per turn.
 // A pass is one warp's chain of instructions, and six solves unrolled (34 KB
 // of code with the advance behind it) waited for instruction fetch 1.85 of
 // every 4.7 cycles on the 192-tet cantilever; the loop waits 0.44. Its 42 moves
@@ -702,31 +702,24 @@ __device__ __forceinline__ float2 solve_tet(const Mat& bp, const TetRec& r, floa
 // 1.57 M-tet mesh, 2,403 -> 2,188 us on 608,256 damped tets. Turning the
 // vertex advance into a loop as well lost (1,009 -> 1,163 us): it moves all
 // eight vertices eight times.
-// before(t, Dt) and after(t, multipliers) see each tet.
-template <bool EXT, class Before, class After>
-__device__ __forceinline__ void solve_cube(const Mat& mat, const float4* rec, float inv_dt, float inv_dt2, float4 O[8],
-                                           float4 D[8], Before before, After after) {
+template <class F>
+__device__ __forceinline__ void turn_cube(float4 O[8], float4 D[8], F f) {
 	float4 ro[6] = {O[2], O[1], O[4], O[5], O[6], O[7]};
 	Vec3 rd[6] = {v3(D[2]), v3(D[1]), v3(D[4]), v3(D[5]), v3(D[6]), v3(D[7])};
 	auto f4 = [](const Vec3& a) { return make_float4(a.x, a.y, a.z, 0.0f); };
 	Vec3 d0 = v3(D[0]), d3 = v3(D[3]);
 #pragma unroll 1
 	for (int t = 0; t < 6; t += 2) {
-		const float4* r = rec + t * 4 * kLanes;
 		{
-			const TetRec tr = {r[0], r[kLanes], r[2 * kLanes], r[3 * kLanes]};
 			const float4 Ot[4] = {O[0], ro[1], ro[0], O[3]};
 			float4 Dt[4] = {f4(d0), f4(rd[1]), f4(rd[0]), f4(d3)};
-			before(t, Dt);
-			after(t, solve_tet<EXT>(mat, tr, inv_dt, inv_dt2, Ot, Dt));
+			f(t, Ot, Dt);
 			d0 = v3(Dt[0]), rd[1] = v3(Dt[1]), rd[0] = v3(Dt[2]), d3 = v3(Dt[3]);
 		}
 		{
-			const TetRec tr = {r[4 * kLanes], r[5 * kLanes], r[6 * kLanes], r[7 * kLanes]};
 			const float4 Ot[4] = {O[0], O[3], ro[2], ro[1]};
 			float4 Dt[4] = {f4(d0), f4(d3), f4(rd[2]), f4(rd[1])};
-			before(t + 1, Dt);
-			after(t + 1, solve_tet<EXT>(mat, tr, inv_dt, inv_dt2, Ot, Dt));
+			f(t + 1, Ot, Dt);
 			d0 = v3(Dt[0]), d3 = v3(Dt[1]), rd[2] = v3(Dt[2]), rd[1] = v3(Dt[3]);
 		}
 		const float4 o0 = ro[0], o1 = ro[1];
@@ -740,6 +733,23 @@ __device__ __forceinline__ void solve_cube(const Mat& mat, const float4* rec, fl
 	auto back = [](float4& a, const Vec3& b) { a.x = b.x, a.y = b.y, a.z = b.z; };
 	back(D[0], d0), back(D[3], d3), back(D[2], rd[0]), back(D[1], rd[1]), back(D[4], rd[2]), back(D[5], rd[3]),
 	    back(D[6], rd[4]), back(D[7], rd[5]);
+}
+
+// Tet t's record of the calling lane's cluster (rec: the lane's first).
+__device__ __forceinline__ TetRec cluster_rec(const float4* rec, int t) {
+	const float4* r = rec + t * 4 * kLanes;
+	return {r[0], r[kLanes], r[2 * kLanes], r[3 * kLanes]};
+}
+
+// The six solves of a whole-cube cluster. before(t, Dt) and after(t,
+// multipliers) see each tet.
+template <bool EXT, class Before, class After>
+__device__ __forceinline__ void solve_cube(const Mat& mat, const float4* rec, float inv_dt, float inv_dt2, float4 O[8],
+                                           float4 D[8], Before before, After after) {
+	turn_cube(O, D, [&](int t, const float4* Ot, float4* Dt) {
+		before(t, Dt);
+		after(t, solve_tet<EXT>(mat, cluster_rec(rec, t), inv_dt, inv_dt2, Ot, Dt));
+	});
 }
 
 // PbdDamp (XPBDFEM/Xpbd.h:307-346): moves the tet's velocities towards its
