@@ -167,7 +167,8 @@ struct xfem_body {
 	// brick launch form (sync_mode 4; built when every chunk is a cube chunk)
 	DevBuf<float4> bcblk;
 	DevBuf<uint32_t> tet_brec_dev;  // per tet (all bodies): its c0 word in the brick chunks
-	DevBuf<uint32_t> bcb, bwait, bcnb_begin, bcnb, bpriv_begin, bpriv_vid, bfin_begin, bfin_vid, bnb_begin, bnb, bflag;
+	DevBuf<uint32_t> bcb, bwait, bcnb_begin, bcnb, bpriv_begin, bpriv_vid, bfin_begin, bfin_vid, bnb_begin, bnb, bflag, blastmask, btflat;
+	DevBuf<float> btarea;
 	// meshes mixing tets and hexes (kElMixed): the tets as elements of their own colouring
 	DevBuf<uint4> mt_vid;
 	DevBuf<float4> mt_rec;
@@ -305,6 +306,17 @@ bool ext_any_of(const std::vector<BodyHost>& bodies) {
 		if (b.settings.damping > 0.0f || b.settings.pbd_damping > 0.0f || model == kModelNeoClamp ||
 		    model >= kModelPixar || b.settings.volume_passes)
 			return true;
+	}
+	return false;
+}
+
+// Whether some body's solve is more than the plain kernels' (the counterpart of
+// the kernels' plain_solve): in-solve damping, Mixed's clamp, a Pixar or a cube model.
+bool ext_solve_of(const std::vector<BodyHost>& bodies) {
+	for (const BodyHost& b : bodies) {
+		const uint32_t model = model_of((b.settings.flags >> XFEM_ENERGY_BIT) & XFEM_ENERGY_MASK);
+		const uint32_t type = (b.settings.flags >> XFEM_RAYLEIGH_TYPE_BIT) & 3u;
+		if ((model != kModelNeo && model != kModelYeoh) || (type < XFEM_RAYLEIGH_POST && b.settings.damping > 0.0f)) return true;
 	}
 	return false;
 }
@@ -1120,7 +1132,8 @@ int build_mixed_tets(xfem_body* h) {
 // and the clusters are those of the other launch forms.
 int build_bricks(xfem_body* h, const std::vector<uint32_t>& ccb, const std::vector<float4>& cblk,
                  const std::vector<ChunkMeta>& meta, const std::vector<uint32_t>& lane_dv,
-                 const std::vector<uint8_t>& lane_nv) {
+                 const std::vector<uint8_t>& lane_nv, const std::vector<uint32_t>& lastmask,
+                 const std::vector<uint32_t>& flat, const std::vector<float>& area) {
 	const uint32_t ncol = h->ncolours, nch = (uint32_t)meta.size();
 	int sms = 0, optin = 0, per_sm_smem = 0;
 	XCUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device));
@@ -1270,10 +1283,18 @@ int build_bricks(xfem_body* h, const std::vector<uint32_t>& ccb, const std::vect
 	// (plane 3 of its record) sits in the brick chunks, so that material
 	// changes reach both layouts
 	std::vector<uint32_t> brec_of_slot((size_t)h->nrows * kLanes, 0);
+	std::vector<uint32_t> blast((size_t)nbc * kLanes, 0), bflat((size_t)nbc * kLanes * 6, 0);
+	std::vector<float> barea((size_t)nbc * kLanes * 6, 0.0f);
 	parallel_for((uint32_t)bc.size(), [&](uint32_t q) {
 		for (size_t j = 0; j < bc[q].size(); j++) {
 			const uint32_t i = bc[q][j], k = i / kLanes, a = i % kLanes;
 			const uint32_t dch = bcb[q] + (uint32_t)(j / kLanes), dl = (uint32_t)(j % kLanes);
+			blast[(size_t)dch * kLanes + dl] = lastmask[i];
+			for (uint32_t t = 0; t < 6; t++) {
+				const size_t from = ((size_t)meta[k].trow + t) * kLanes + a, to = ((size_t)dch * 6 + t) * kLanes + dl;
+				bflat[to] = flat[from];
+				barea[to] = area[from];
+			}
 			const float4* src = &cblk[meta[k].off16];
 			float4* dst = &blk[(size_t)dch * per16];
 			for (uint32_t t = 0; t < 6; t++)
@@ -1295,6 +1316,9 @@ int build_bricks(xfem_body* h, const std::vector<uint32_t>& ccb, const std::vect
 	XCUDA(h->tet_brec_dev.alloc(brec.size()));
 	XCUDA(h->bcblk.alloc(blk.size()));
 	XCUDA(h->bcb.alloc(bcb.size()));
+	XCUDA(h->blastmask.alloc(blast.size()));
+	XCUDA(h->btflat.alloc(bflat.size()));
+	XCUDA(h->btarea.alloc(barea.size()));
 	XCUDA(h->bwait.alloc(bwait.size()));
 	XCUDA(h->bcnb_begin.alloc(cnb_begin.size()));
 	XCUDA(h->bcnb.alloc(std::max<size_t>(1, cnb.size())));
@@ -1311,6 +1335,9 @@ int build_bricks(xfem_body* h, const std::vector<uint32_t>& ccb, const std::vect
 	XCUDA(up(h->bcblk.p, blk.data(), blk.size() * sizeof(float4)));
 	XCUDA(up(h->tet_brec_dev.p, brec.data(), brec.size() * 4));
 	XCUDA(up(h->bcb.p, bcb.data(), bcb.size() * 4));
+	XCUDA(up(h->blastmask.p, blast.data(), blast.size() * 4));
+	XCUDA(up(h->btflat.p, bflat.data(), bflat.size() * 4));
+	XCUDA(up(h->btarea.p, barea.data(), barea.size() * 4));
 	XCUDA(up(h->bwait.p, bwait.data(), bwait.size() * 4));
 	XCUDA(up(h->bcnb_begin.p, cnb_begin.data(), cnb_begin.size() * 4));
 	XCUDA(up(h->bcnb.p, cnb.data(), cnb.size() * 4));
@@ -1323,6 +1350,9 @@ int build_bricks(xfem_body* h, const std::vector<uint32_t>& ccb, const std::vect
 	XCUDA(cudaStreamSynchronize(h->stream));
 	DevCtx& c = h->ctx;
 	c.bcblk = h->bcblk.p;
+	c.blastmask = h->blastmask.p;
+	c.btflat = h->btflat.p;
+	c.btarea = h->btarea.p;
 	c.bchunk_begin = h->bcb.p;
 	c.bchunk_wait_end = h->bwait.p;
 	c.bcnb_begin = h->bcnb_begin.p;
@@ -1336,7 +1366,7 @@ int build_bricks(xfem_body* h, const std::vector<uint32_t>& ccb, const std::vect
 	c.bflag = h->bflag.p;
 	c.nbricks = nb;
 	c.bpriv_max = pmax;
-	h->device_bytes += blk.size() * 16 + (brec.size() + bcb.size() + bwait.size() + cnb_begin.size() + cnb.size() + pbeg.size() + pvid.size() + fbeg.size() + fvid.size() +
+	h->device_bytes += blk.size() * 16 + (brec.size() + blast.size() + bflat.size() + barea.size() + bcb.size() + bwait.size() + cnb_begin.size() + cnb.size() + pbeg.size() + pvid.size() + fbeg.size() + fvid.size() +
 	                                      nbeg.size() + nbv.size() + (size_t)nb * kBrickFlagStride) * 4;
 	if (getenv("XFEM_SETUP_TIMING"))
 		fprintf(stderr, "xfem bricks: %u bricks, %u chunks, %zu private and %zu shared vertices, at most %u private "
@@ -1450,6 +1480,8 @@ int build_device(xfem_body* h) {
 	clk.lap("chunk shapes");
 	std::vector<float4> cblk((size_t)total16, make_float4(0, 0, 0, 0));
 	std::vector<uint32_t> lastmask(nlanes, 0);
+	std::vector<uint32_t> flat;  // per tet row: the tet's index in its body's order
+	std::vector<float> area;     // and its surface area
 	for (auto& b : h->bodies) {
 		b.tet_slot.assign(b.nt, 0xffffffffu);
 		b.tet_rec.assign(b.nt, 0);
@@ -1627,8 +1659,8 @@ int build_device(xfem_body* h) {
 		XCUDA(up(h->tet_inv_mu.p, inv_mu.data(), inv_mu.size() * 4));
 		// per tet row: the index in the body's flattened order (the amortized
 		// damping slices) and the surface area (PBD damping)
-		std::vector<uint32_t> flat((size_t)trows * kLanes, 0);
-		std::vector<float> area((size_t)trows * kLanes, 1.0f);
+		flat.assign((size_t)trows * kLanes, 0);
+		area.assign((size_t)trows * kLanes, 1.0f);
 		for (const BodyHost& b : h->bodies) {
 			const Schedule& sc = b.sched;
 			uint32_t o = 0;
@@ -1705,6 +1737,7 @@ int build_device(xfem_body* h) {
 	c.timeout_ns = h->opt.wait_timeout_ms ? (uint64_t)h->opt.wait_timeout_ms * 1000000ull : kDefaultTimeoutNs;
 	h->cfg.lambdas = h->opt.keep_lambdas != 0;
 	h->cfg.ext = c.ext != 0u;
+	h->cfg.ext_solve = ext_solve_of(h->bodies);
 	c.ring_hdr = h->ring_hdr.p;
 	c.ring_node = h->ring_node.p;
 	c.ring_ent = h->ring_ent.p;
@@ -1729,20 +1762,23 @@ int build_device(xfem_body* h) {
 	h->cfg.total_chunks = nch;
 	h->cfg.colour_chunk_begin_host = ccb;
 	if (all_cube && !h->ring_mode && !h->el_mode && nch && (h->opt.sync_mode == 0 || h->opt.sync_mode == 4)) {
-		const int rb = build_bricks(h, ccb, cblk, meta, lane_dv, lane_nv);
+		const int rb = build_bricks(h, ccb, cblk, meta, lane_dv, lane_nv, lastmask, flat, area);
 		if (rb) return rb;
 		clk.lap("bricks");
 	}
 	return update_right_targets(h);
 }
 
-// Whether the persistent form (sync_mode 1) of this handle runs as one
-// thread-block cluster, and of how many blocks (cluster_plan). Returns a
-// cudaError_t value.
+// How the persistent form (sync_mode 1) of this handle runs: as one thread-block
+// cluster (cluster_plan), with the extended kernel on the bricks
+// (brick_ext_fits), or as one grid. Returns a cudaError_t value.
 int pick_cluster(xfem_body* h) {
 	h->cfg.cluster = ClusterPlan();
+	h->cfg.brick_ext = false;
 	if (h->cfg.sync_mode != 1 || h->cfg.lambdas || !h->nchunks) return 0;
-	return cluster_plan(h->ctx, h->max_colour_chunks, h->cfg.block, false, h->cfg.ext, &h->cfg.cluster);
+	const int e = cluster_plan(h->ctx, h->max_colour_chunks, h->cfg.block, false, h->cfg.ext_level(), &h->cfg.cluster);
+	if (e || h->cfg.cluster.blocks || h->cfg.ext_level() != 1) return e;
+	return brick_ext_fits(h->ctx, h->cfg.block, &h->cfg.brick_ext);
 }
 
 int set_config(xfem_body* h, int sync_mode, int block) {
@@ -2234,13 +2270,14 @@ int xfem_set_settings(xfem_body* h, uint32_t body, const xfem_settings* s) {
 	XCUDA(cudaMemcpyAsync(h->pass_on.p, pt.data(), pt.size(), cudaMemcpyHostToDevice, h->stream));
 	XCUDA(cudaStreamSynchronize(h->stream));
 	const uint32_t kinds = damp_kinds_of(h->bodies);
-	const bool ext = ext_any_of(h->bodies);
+	const bool ext = ext_any_of(h->bodies), ext_solve = ext_solve_of(h->bodies);
 	const uint32_t nvol = nvol_of(h->bodies);
-	if (kinds != h->ctx.damp_kinds || ext != h->cfg.ext || nvol != h->ctx.nvol) {
+	if (kinds != h->ctx.damp_kinds || ext != h->cfg.ext || ext_solve != h->cfg.ext_solve || nvol != h->ctx.nvol) {
 		h->ctx.damp_kinds = kinds;
 		h->ctx.ext = ext ? 1u : 0u;
 		h->ctx.nvol = nvol;
 		h->cfg.ext = ext;
+		h->cfg.ext_solve = ext_solve;
 		if (h->graph) {  // the captured launches follow the old sweeps
 			cudaGraphExecDestroy(h->graph);
 			h->graph = nullptr;

@@ -42,16 +42,8 @@ XFEM_HD uint32_t cluster_warp_bytes(uint32_t vs_off, uint32_t warp_smem, uint32_
 	return bufs * vs_off + (warp_smem - vs_off);
 }
 
-template <bool ONE>
-__device__ __forceinline__ auto body_params(const DevCtx& C) {
-	if constexpr (ONE)
-		return OneBody{C.bodies[0], load_mat(C.bodies, 0)};
-	else
-		return AnyBody{};
-}
-
 // ONE: a single body, its parameters in registers.
-template <bool TAPE, bool EXT, bool ONE>
+template <bool TAPE, int LEVEL, bool ONE>
 __global__ void __launch_bounds__(256) k_cluster(DevCtx C, ClusterPlan plan, uint32_t nsub, float dt) {
 	extern __shared__ __align__(128) uint8_t smem[];
 	__shared__ uint64_t s_mbar[8][kClusterBufs];
@@ -61,6 +53,7 @@ __global__ void __launch_bounds__(256) k_cluster(DevCtx C, ClusterPlan plan, uin
 	const uint32_t lane = threadIdx.x & 31u, wib = threadIdx.x >> 5;
 	const uint32_t G = gridDim.x, r = blockIdx.x;
 	const uint32_t gtid = blockIdx.x * blockDim.x + threadIdx.x, nthreads = gridDim.x * blockDim.x;
+	constexpr bool EXT = LEVEL != 0;
 	const bool dmode = EXT && C.damp_kinds != 0u;
 	const uint32_t ncol = C.ncolours, P = (EXT ? pass_kinds(C) : 1u) * ncol, nbuf = plan.bufs;
 	const uint32_t tick0 = __ldcg(C.tick);  // read before the first barrier; block 0 advances it at the end
@@ -153,8 +146,8 @@ __global__ void __launch_bounds__(256) k_cluster(DevCtx C, ClusterPlan plan, uin
 				if (!ok)
 					;
 				else if (!EXT || kind == 0)
-					run_chunk<false, TAPE, EXT>(C, vs, bps, st, (uint32_t)ch, -1, lane, dmode || s == 0, dt, inv_dt, inv_dt2,
-					                            s, dmode);
+					run_chunk<false, TAPE, EXT, LEVEL == 2>(C, vs, bps, st, (uint32_t)ch, -1, lane, dmode || s == 0, dt,
+					                                                    inv_dt, inv_dt2, s, dmode);
 				else if (kind <= C.nvol)
 					run_vol_chunk(C, vs, st, (uint32_t)ch, -1, lane, inv_dt, inv_dt2, kind, dmode);
 				else
@@ -177,10 +170,11 @@ __global__ void __launch_bounds__(256) k_cluster(DevCtx C, ClusterPlan plan, uin
 	if (gtid == 0) *C.tick = tick0 + nsub;
 }
 
-const void* cluster_fn(bool tape, bool ext, bool one) {
-	if (tape) return one ? (const void*)k_cluster<true, false, true> : (const void*)k_cluster<true, false, false>;
-	if (ext) return one ? (const void*)k_cluster<false, true, true> : (const void*)k_cluster<false, true, false>;
-	return one ? (const void*)k_cluster<false, false, true> : (const void*)k_cluster<false, false, false>;
+const void* cluster_fn(bool tape, int ext, bool one) {
+	if (tape) return one ? (const void*)k_cluster<true, 0, true> : (const void*)k_cluster<true, 0, false>;
+	if (ext == 2) return one ? (const void*)k_cluster<false, 2, true> : (const void*)k_cluster<false, 2, false>;
+	if (ext == 1) return one ? (const void*)k_cluster<false, 1, true> : (const void*)k_cluster<false, 1, false>;
+	return one ? (const void*)k_cluster<false, 0, true> : (const void*)k_cluster<false, 0, false>;
 }
 
 size_t cluster_smem(const DevCtx& C, const ClusterPlan& p) {
@@ -207,7 +201,7 @@ void cluster_config(const DevCtx& C, const ClusterPlan& p, int block, cudaLaunch
 // 192 tets 753 us against 494), every vertex in shared memory. Of the cluster
 // sizes that allow it: the smallest whose blocks hold all their records with
 // at most one chunk warp per scheduler, else the largest.
-int cluster_plan(const DevCtx& C, uint32_t max_colour_chunks, int block, bool tape, bool ext, ClusterPlan* plan) {
+int cluster_plan(const DevCtx& C, uint32_t max_colour_chunks, int block, bool tape, int ext, ClusterPlan* plan) {
 	*plan = ClusterPlan();
 	if (block > 256 || block % 32 || C.nverts == 0 || C.ncolours == 0) return 0;
 	int dev = 0, optin = 0;
@@ -246,7 +240,7 @@ int cluster_plan(const DevCtx& C, uint32_t max_colour_chunks, int block, bool ta
 }
 
 // Not a cooperative launch: the blocks of a cluster are always resident together.
-int launch_cluster(const DevCtx& ctx, const ClusterPlan& plan, int block, bool tape, bool ext, uint32_t nsub, float dt,
+int launch_cluster(const DevCtx& ctx, const ClusterPlan& plan, int block, bool tape, int ext, uint32_t nsub, float dt,
                    void* stream) {
 	cudaLaunchAttribute at{};
 	cudaLaunchConfig_t lc{};

@@ -340,6 +340,14 @@ struct OneBody {
 	}
 };
 
+template <bool ONE>
+__device__ __forceinline__ auto body_params(const DevCtx& C) {
+	if constexpr (ONE)
+		return OneBody{C.bodies[0], load_mat(C.bodies, 0)};
+	else
+		return AnyBody{};
+}
+
 // Hydrostatic term at the single point (XPBDFEM/Fem.cpp:539-549 with the
 // adjugate :284-300, F :311-323 and the gradient :338-354). J is formed as
 // the reference forms it, det(F) of F = Qi Ds (rows of Ds: P0, P1, P2) through
@@ -505,9 +513,10 @@ __device__ __forceinline__ void volume_tet(const Mat& bp, const TetRec& r, float
 // its current positions, then RayleighDamp (XPBDFEM/Xpbd.h:217-263) on its
 // velocities: one constraint for the Pixar models, the pair for the others,
 // nothing for the cube models. damp: the Rayleigh ratio (x 8 when amortized).
+template <bool XSOLVE = true>
 __device__ __forceinline__ void rayleigh_tet(const Mat& bp, const TetRec& r, const float4 X[4], float4 V[4],
                                              float inv_dt, float damp) {
-	if (bp.model == kModelNone) return;  // SolveElementCube damps quads and hexes only
+	if (XSOLVE && bp.model == kModelNone) return;  // SolveElementCube damps quads and hexes only
 	const float q[3][3] = {{r.a.x, r.a.y, r.a.z}, {r.a.w, r.b.x, r.b.y}, {r.b.z, r.b.w, r.c.x}};
 	const float QQ[3] = {r.c.y, r.c.z, r.c.w};
 	const float QR[3] = {r.d.x, r.d.y, r.d.z};
@@ -517,7 +526,7 @@ __device__ __forceinline__ void rayleigh_tet(const Mat& bp, const TetRec& r, con
 	for (int i = 0; i < 3; i++) P[i] = {X[i].x - X[3].x, X[i].y - X[3].y, X[i].z - X[3].z};
 	Vec3 g0[4], g1[4];
 	const float ib0 = r.d.w * inv_dt / damp, ib1 = ib0 * bp.ratio;  // comp / (dt damping)
-	if (bp.model == kModelPixar) {
+	if (XSOLVE && bp.model == kModelPixar) {
 		// SolveElementPixar with DampingMode::On (XPBDFEM/Fem.cpp:429-430): one constraint
 		const float U = pixar_energy(bp, q, QQ, QR, P, g0, g1);
 		float gV = 0.0f;
@@ -533,7 +542,7 @@ __device__ __forceinline__ void rayleigh_tet(const Mat& bp, const TetRec& r, con
 		}
 		return;
 	}
-	const float U0 = deviatoric<true>(bp, QQ, QR, P, g0);
+	const float U0 = deviatoric<XSOLVE>(bp, QQ, QR, P, g0);
 	const float U1 = hydrostatic(q, P, bp.a, g1);
 	if (bp.simultaneous) {
 		float b0 = 0.0f, b1 = 0.0f;

@@ -409,6 +409,9 @@ struct DevCtx {
 	uint32_t* bflag;
 	uint32_t nbricks, bpriv_max;
 	uint32_t nbodies;
+	const uint32_t* blastmask;  // lastmask, tflat and tarea of the brick chunks (six tet rows each)
+	const uint32_t* btflat;
+	const float* btarea;
 };
 
 // Brick chunk block: records (6 x 4 x 32 float4), header (32 u32), vertex
@@ -464,10 +467,14 @@ struct LaunchCfg {
 	int block = 256;
 	int blocks = 0;        // persistent grid size
 	ClusterPlan cluster;   // sync_mode 1: the one-cluster form, when the handle takes it
+	bool brick_ext = false;  // sync_mode 1, extended: on the bricks (k_bricks_ext)
 	int sync_mode = 1;     // 1 persistent + grid barrier, 2 per-colour launches (CUDA graph), 3 persistent dataflow,
 	                       // 4 persistent bricks (k_bricks: brick-resident vertices, neighbour waits)
 	bool lambdas = false;
 	bool ext = false;      // launch the extended instantiations (DevCtx::ext)
+	bool ext_solve = false;  // ext: some body's solve is not the plain one
+	// 0 the plain kernels, 1 with damping and volume sweeps, 2 with the extended solves too
+	int ext_level() const { return !ext ? 0 : ext_solve ? 2 : 1; }
 	uint32_t warp_smem = 0;
 	uint32_t total_chunks = 0;
 	std::vector<uint32_t> colour_chunk_begin_host;
@@ -483,8 +490,8 @@ int configure_kernels(const LaunchCfg& cfg);
 int persistent_grid(const LaunchCfg& cfg, int* blocks_out);
 // The one-cluster form's plan for a handle and a block size, and its launch
 // (tape: the recording forward). Both return a cudaError_t value.
-int cluster_plan(const DevCtx& ctx, uint32_t max_colour_chunks, int block, bool tape, bool ext, ClusterPlan* plan);
-int launch_cluster(const DevCtx& ctx, const ClusterPlan& plan, int block, bool tape, bool ext, uint32_t nsub, float dt,
+int cluster_plan(const DevCtx& ctx, uint32_t max_colour_chunks, int block, bool tape, int ext, ClusterPlan* plan);
+int launch_cluster(const DevCtx& ctx, const ClusterPlan& plan, int block, bool tape, int ext, uint32_t nsub, float dt,
                    void* stream);
 // Dynamic shared memory bytes per block of the brick kernel, and whether
 // `nbricks` blocks of `block` threads fit on the device at once (the
@@ -492,6 +499,10 @@ int launch_cluster(const DevCtx& ctx, const ClusterPlan& plan, int block, bool t
 // value; *fits is set on success.
 size_t brick_smem_bytes(int block, uint32_t bpriv_max);
 int brick_grid_fits(int block, uint32_t bpriv_max, uint32_t nbricks, bool* fits);
+// The extended kernel on the bricks (xfem_bricks_ext.cu): whether this block
+// size fits, and its launch. Both return a cudaError_t value.
+int brick_ext_fits(const DevCtx& ctx, int block, bool* fits);
+int launch_bricks_ext(const DevCtx& ctx, int block, uint32_t nsub, float dt, void* stream);
 // Dynamic shared memory bytes per block of the solve kernels.
 size_t solve_smem_bytes(int block, uint32_t warp_smem);
 

@@ -124,10 +124,6 @@ __global__ void __launch_bounds__(256) k_persistent(DevCtx C, uint32_t nsub, flo
 	if (gtid == 0) *C.tick = tick0 + nsub;
 }
 
-__device__ __forceinline__ void st_release_gpu(uint32_t* p, uint32_t v) {
-	asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-
 // Bounded wait until every neighbour chunk of `ch` has done its share of
 // substep s: chunks of a lower colour must have completed s + 1 substeps,
 // chunks of a higher colour s substeps (the previous one). One lane per
@@ -222,39 +218,6 @@ __global__ void __launch_bounds__(256) k_dataflow(DevCtx C, uint32_t nsub, float
 // a brick it shares vertices with. The colour order, the clusters and the
 // arithmetic are those of k_persistent, so the results are bit-identical.
 
-// The calling warp's brick chunk buffer and mbarrier.
-__device__ __forceinline__ Stage brick_stage_init(uint32_t lane) {
-	extern __shared__ __align__(128) uint8_t smem[];
-	__shared__ uint64_t bmbars[32];
-	const uint32_t w = threadIdx.x >> 5;
-	Stage st = {smem + (size_t)w * kBrickChunkBytes, nullptr, &bmbars[w], 0u, -1, make_uint4(0u, 0u, 0u, 0u)};
-	if (lane == 0) mbar_init(st.mbar);
-	__syncwarp();
-	return st;
-}
-
-__device__ __forceinline__ void brick_issue(const DevCtx& C, Stage& st, uint32_t chunk, uint32_t lane) {
-	__syncwarp();
-	if (lane == 0)
-		bulk_copy_g2s(st.buf, C.bcblk + (size_t)chunk * (kBrickChunkBytes / 16u), kBrickChunkBytes, st.mbar);
-	st.inflight = (int)chunk;
-}
-
-// Makes brick chunk `chunk` resident in the warp's buffer; false on timeout.
-__device__ __forceinline__ bool brick_acquire(const DevCtx& C, Stage& st, uint32_t chunk, uint32_t lane) {
-	if (st.inflight != (int)chunk) {
-		if (st.inflight >= 0) {
-			if (!mbar_wait(C, st.mbar, st.parity)) return false;
-			st.parity ^= 1u;
-		}
-		brick_issue(C, st, chunk, lane);
-	}
-	const bool ok = mbar_wait(C, st.mbar, st.parity);
-	st.parity ^= 1u;
-	st.inflight = -1;
-	return ok;
-}
-
 // The warp's next brick chunk after `ch` (colour c of substep s; bcb: the
 // brick's colour chunk offsets), -1 when the launch has no more for it.
 __device__ __forceinline__ int next_brick_chunk(const uint32_t* bcb, uint32_t ncol, uint32_t s, uint32_t nsub,
@@ -335,43 +298,6 @@ __device__ __forceinline__ void run_chunk_brick(const DevCtx& C, Stage& st, int 
 			}
 		}
 	}
-}
-
-// Bounded wait, by the calling threads (`first` of them striding by
-// `stride`), until every brick of list[nb0, nb1) has published at least
-// `target` passes. Returns false when a wait ran out or another
-// block reported an error. The polls are relaxed loads and one acquire
-// fence follows them (the acquire pattern of the PTX memory model): an
-// acquire load on every poll, or an acquire-release fence, made the
-// throughput frame 1.7% and 11% slower.
-__device__ bool brick_wait(const DevCtx& C, const uint32_t* list, uint32_t nb0, uint32_t nb1, uint32_t target,
-                           uint32_t first, uint32_t stride) {
-	target += C.wait_miss;
-	bool bad = false;
-	for (uint32_t i = nb0 + first; i < nb1 && !bad; i += stride) {
-		const uint32_t* f = C.bflag + (size_t)__ldg(list + i) * kBrickFlagStride;
-		uint32_t spins = 0;
-		uint64_t t0 = 0;
-		while ((int32_t)(ld_relaxed_gpu(f) - target) < 0) {
-			if (++spins == 256) {
-				spins = 0;
-				if (*(volatile int*)C.err) {
-					bad = true;
-					break;
-				}
-				const uint64_t t = global_ns();
-				if (t0 == 0) {
-					t0 = t;
-				} else if (t - t0 > C.timeout_ns) {
-					atomicCAS(C.err, 0, kErrBarrierTimeout);
-					bad = true;
-					break;
-				}
-			}
-		}
-	}
-	asm volatile("fence.acquire.gpu;" ::: "memory");
-	return !bad;
 }
 
 // Persistent brick kernel: one block per brick (grid = nbricks, cooperative
@@ -723,9 +649,11 @@ int launch_substeps(const DevCtx& ctx, const LaunchCfg& cfg, uint32_t nsub, floa
 		}
 		return 0;
 	}
+	if (cfg.sync_mode == 1 && cfg.brick_ext && !ctx.bar_base)
+		return launch_bricks_ext(ctx, cfg.block, nsub, dt, stream);
 	// the hooks that make grid-barrier waits run out or wrap need that barrier
 	if (cfg.sync_mode == 1 && cfg.cluster.blocks && !ctx.wait_miss && !ctx.bar_base)
-		return launch_cluster(ctx, cfg.cluster, cfg.block, false, cfg.ext, nsub, dt, stream);
+		return launch_cluster(ctx, cfg.cluster, cfg.block, false, cfg.ext_level(), nsub, dt, stream);
 	if (cfg.sync_mode == 1 || cfg.sync_mode == 3) {
 		e = reset_barrier(ctx, st);
 		if (e == cudaSuccess && cfg.sync_mode == 3) e = cudaMemsetAsync(ctx.done, 0, sizeof(uint32_t) * ctx.nchunks, st);
@@ -782,10 +710,10 @@ int launch_substeps_tape(const DevCtx& ctx, int block, uint32_t warp_smem, uint3
 	cudaStream_t st = (cudaStream_t)stream;
 	ClusterPlan plan;
 	if (!ctx.wait_miss && !ctx.bar_base) {
-		const int ec = cluster_plan(ctx, max_colour_chunks, block, true, false, &plan);
+		const int ec = cluster_plan(ctx, max_colour_chunks, block, true, 0, &plan);
 		if (ec) return ec;
 	}
-	if (plan.blocks) return launch_cluster(ctx, plan, block, true, false, nsub, dt, stream);
+	if (plan.blocks) return launch_cluster(ctx, plan, block, true, 0, nsub, dt, stream);
 	const void* f = (const void*)k_persistent<false, true>;
 	const size_t smem = solve_smem_bytes(block, warp_smem);
 	cudaError_t e = set_smem_attr(f, smem);
