@@ -1158,9 +1158,12 @@ int build_bricks(xfem_body* h, const std::vector<uint32_t>& ccb, const std::vect
 	// one brick per SM (or xfem_options.bricks), about one chunk per brick and colour at least.
 	// Two bricks per SM, each with blocks of 192 threads, when each still gets three chunks
 	// per colour or more: one brick's neighbour waits and barrier then overlap the other's
-	// solves (the throughput mesh, 3.4 chunks per brick and colour: 0.979 ms per frame
-	// against 0.990 with one brick of 256 threads). Their private vertices are capped so
-	// that two blocks of six chunk buffers fit one SM.
+	// solves, and a brick whose colours need more chunks than its eight warps take them in
+	// two rounds. Measured, pairs against one brick of 256 threads per SM, us per frame:
+	// 196,608 cubes (2.5 chunks per brick and colour) 862 and 819, 262,144 912 and 904,
+	// 268,800 944 and 1,180, 294,912 947 and 1,261; with damping, 196,608 1,503 and 1,470,
+	// 262,144 1,437 and 1,608. Their private vertices are capped so that two blocks of six
+	// chunk buffers fit one SM.
 	const bool pairs = !h->opt.bricks && L >= 3ull * 2 * (uint64_t)sms * kLanes * ncol;
 	if (pairs) {
 		const int64_t cap2 = ((int64_t)per_sm_smem / 2 - 1024 - 6 * (int64_t)kBrickChunkBytes - 4096) / kBrickVertexBytes;

@@ -13,7 +13,8 @@
 // 8,800 for a damping pass (the brick has 2.6 chunks of a colour, on as many
 // warps), and 2,000 to 4,500 until the neighbours' pass counts are there.
 // Measured, a frame of 20 substeps with the interactive damping settings, grid
-// form before: 608,256 tets 1,872 -> 1,515 us.
+// form before: 608,256 tets 1,872 -> 1,457 us, 3,145,728 tets (two bricks per SM)
+// 3,808 -> 2,510.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -26,43 +27,6 @@
 namespace xfem {
 
 namespace {
-
-__device__ __forceinline__ float4 ld_any(const float4* p) {
-	float4 v;
-	asm volatile("ld.cg.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p) : "memory");
-	return v;
-}
-
-__device__ __forceinline__ void st_any(float4* p, const float4& v) {
-	asm volatile("st.cg.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
-}
-
-// A brick chunk's vertex words: a device vertex, or kPrivate | the slot of the
-// block's shared memory (O at sv[p], D at sv[pmax + p], device id spid[p]). One
-// access through a generic address, past L1, for both: a warp whose lanes have
-// both takes no branch per vertex.
-struct BrickVerts {
-	float4* sv;
-	const uint32_t* spid;
-	uint32_t pmax;
-
-	__device__ __forceinline__ float4* o(const DevCtx& C, uint32_t w) const {
-		return (w & kPrivate) ? sv + (w & ~kPrivate) : C.vert + 2 * (size_t)w;
-	}
-	__device__ __forceinline__ float4* d(const DevCtx& C, uint32_t w) const {
-		return (w & kPrivate) ? sv + pmax + (w & ~kPrivate) : C.vert + 2 * (size_t)w + 1;
-	}
-	__device__ __forceinline__ void ld(const DevCtx& C, uint32_t w, float4& O, float4& D) const {
-		O = ld_any(o(C, w));
-		D = ld_any(d(C, w));
-	}
-	__device__ __forceinline__ void st(const DevCtx& C, uint32_t w, const float4& O, const float4& D) const {
-		st_any(o(C, w), O);
-		st_any(d(C, w), D);
-	}
-	__device__ __forceinline__ void st_d(const DevCtx& C, uint32_t w, const float4& D) const { st_any(d(C, w), D); }
-	__device__ __forceinline__ uint32_t id(uint32_t w) const { return (w & kPrivate) ? spid[w & ~kPrivate] : w; }
-};
 
 // Element sweeps of a substep, in their order.
 enum class Sweep { kSolve, kVolume, kRayleigh, kPbd };
@@ -77,9 +41,9 @@ __device__ __forceinline__ Sweep sweep_of(const DevCtx& C, uint32_t kind) {
 // damp_chunk, but one load of the eight vertices and one write-back for all of
 // them. With those three inlined or called side by side the kernel kept its
 // registers on the stack (1,040 bytes, 160 of them spilled) and a damped frame of
-// 608,256 tets took 1,773 us; so, with no stack, 1,515.
-template <class BP>
-__device__ __forceinline__ void sweep_cube(const DevCtx& C, const BrickVerts& vs, const BP& bps, Stage& st, uint32_t chunk, int next,
+// 608,256 tets took 1,773 us; so, with no stack, 1,515 then.
+template <class VS, class BP>
+__device__ __forceinline__ void sweep_cube(const DevCtx& C, const VS& vs, const BP& bps, Stage& st, uint32_t chunk, int next,
                                            uint32_t lane, Sweep sweep, uint32_t k, bool first, bool finish, float dt,
                                            float inv_dt, float inv_dt2, uint32_t tick) {
 	const uint32_t trow = chunk * 6u;
@@ -145,10 +109,7 @@ __device__ __forceinline__ void sweep_cube(const DevCtx& C, const BrickVerts& vs
 #pragma unroll
 		for (int s = 0; s < 8; s++) {
 			if (last & (1u << s)) bps.finalize(C, vs.id(vid[s]), O[s], D[s], inv_dt);
-			if ((mask | last) & (1u << s))
-				vs.st(C, vid[s], O[s], D[s]);
-			else
-				vs.st_d(C, vid[s], D[s]);
+			vs.st(C, vid[s], O[s], D[s], ((mask | last) & (1u << s)) != 0u);
 		}
 	}
 }
@@ -168,7 +129,7 @@ __global__ void __launch_bounds__(PAIR ? 192 : 256, PAIR ? 2 : 1) k_bricks_ext(c
 	Stage st = brick_stage_init(lane);
 	float4* sv = reinterpret_cast<float4*>(smem + (size_t)wpb * kBrickChunkBytes);
 	uint32_t* spid = reinterpret_cast<uint32_t*>(sv + 2 * (size_t)C.bpriv_max);
-	const BrickVerts vs = {sv, spid, C.bpriv_max};
+	const BrickVerts<!PAIR> vs = {sv, spid, C.bpriv_max};
 	const auto bps = body_params<ONE>(C);
 	for (uint32_t i = threadIdx.x; i <= ncol; i += blockDim.x) {
 		s_bcb[i] = __ldg(C.bchunk_begin + (size_t)b * ncol + i);

@@ -117,7 +117,7 @@ __device__ __forceinline__ void run_chunk_cube(const DevCtx& C, const VS& vs, co
 		if (XSOLVE && !plain_solve(mat))
 			solve_cube<XSOLVE>(mat, rec + lane, inv_dt, inv_dt2, O, D, before, after);
 		else
-			solve_cube<false>(mat, rec + lane, inv_dt, inv_dt2, O, D, before, after);
+			solve_cube<false, VS::kAhead && !TAPE>(mat, rec + lane, inv_dt, inv_dt2, O, D, before, after);
 	}
 	if (next >= 0) stage_issue_m(C, st, (uint32_t)next, mnext, lane);  // buffer consumed: prefetch
 	if (live) {
@@ -461,6 +461,63 @@ __device__ __forceinline__ bool pass_runs(const DevCtx& C, uint32_t q, uint32_t 
 }
 
 // ---- bricks: what the plain and the extended brick kernel share -------------------
+__device__ __forceinline__ float4 ld_any(const float4* p) {
+	float4 v;
+	asm volatile("ld.cg.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p) : "memory");
+	return v;
+}
+
+__device__ __forceinline__ void st_any(float4* p, const float4& v) {
+	asm volatile("st.cg.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
+}
+
+// A brick chunk's vertex words: a device vertex, or kPrivate | the slot of the
+// block's shared memory (O at sv[p], D at sv[pmax + p], device id spid[p]).
+// GENERIC: one access through a generic address, past L1, for both, so that a
+// warp whose lanes have both takes no branch per vertex; else a branch. With one
+// brick per SM the former is faster (a batch of 96 uneven bodies: 3,695 us per four
+// frames against 3,815), with two bricks per SM the latter (1,572,864 tets: 902 us
+// per frame against 1,073).
+template <bool GENERIC>
+struct BrickVerts {
+	float4* sv;
+	const uint32_t* spid;
+	uint32_t pmax;
+
+	__device__ __forceinline__ float4* o(const DevCtx& C, uint32_t w) const {
+		return (w & kPrivate) ? sv + (w & ~kPrivate) : C.vert + 2 * (size_t)w;
+	}
+	__device__ __forceinline__ float4* d(const DevCtx& C, uint32_t w) const {
+		return (w & kPrivate) ? sv + pmax + (w & ~kPrivate) : C.vert + 2 * (size_t)w + 1;
+	}
+	__device__ __forceinline__ void ld(const DevCtx& C, uint32_t w, float4& O, float4& D) const {
+		if (GENERIC) {
+			O = ld_any(o(C, w));
+			D = ld_any(d(C, w));
+		} else if (w & kPrivate) {
+			O = sv[w & ~kPrivate];
+			D = sv[pmax + (w & ~kPrivate)];
+		} else {
+			ld_vertex(C.vert + 2 * (size_t)w, O, D);
+		}
+	}
+	// o_too: O changed as well
+	__device__ __forceinline__ void st(const DevCtx& C, uint32_t w, const float4& O, const float4& D, bool o_too) const {
+		if (GENERIC) {
+			if (o_too) st_any(o(C, w), O);
+			st_any(d(C, w), D);
+		} else if (w & kPrivate) {
+			if (o_too) sv[w & ~kPrivate] = O;
+			sv[pmax + (w & ~kPrivate)] = D;
+		} else if (o_too) {
+			st_vertex(C.vert + 2 * (size_t)w, O, D);
+		} else {
+			__stcg(C.vert + 2 * (size_t)w + 1, D);
+		}
+	}
+	__device__ __forceinline__ uint32_t id(uint32_t w) const { return (w & kPrivate) ? spid[w & ~kPrivate] : w; }
+};
+
 __device__ __forceinline__ void st_release_gpu(uint32_t* p, uint32_t v) {
 	asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }

@@ -237,17 +237,16 @@ __device__ __forceinline__ int next_brick_chunk(const uint32_t* bcb, uint32_t nc
 }
 
 // One resident brick chunk (every lane a whole cube, as run_chunk_cube).
-// Vertex word w of a lane: a device vertex in vert, or kPrivate | p for the
-// brick's shared-memory slot p (O at sv[p], D at sv[bpriv_max + p], device id
-// spid[p]; O and D in two arrays so that the 16-byte accesses of a warp, whose
-// lanes hold nearby slots, fall in different bank groups).
+// Its vertex words are BrickVerts'; a brick's O and D are two arrays so that the
+// 16-byte accesses of a warp, whose lanes hold nearby slots, fall in different
+// bank groups.
 // bodies: the body parameters (a shared-memory copy when the handle has few).
 // ONE: a single body, whose parameters bp1 and material mat1 the kernel holds
 // in registers.
-template <bool ONE>
+template <bool ONE, bool PAIR>
 __device__ __forceinline__ void run_chunk_brick(const DevCtx& C, Stage& st, int next, uint32_t lane, bool first,
-                                                float dt, float inv_dt, float inv_dt2, float4* sv,
-                                                const uint32_t* spid, const BodyParams* bodies, bool bshared,
+                                                float dt, float inv_dt, float inv_dt2, const BrickVerts<!PAIR>& vs,
+                                                const BodyParams* bodies, bool bshared,
                                                 const BodyParams& bp1, const Mat& mat1) {
 	const float4* rec = reinterpret_cast<const float4*>(st.buf);
 	const uint32_t* hdrs = reinterpret_cast<const uint32_t*>(st.buf + 2048u * 6u);
@@ -262,41 +261,23 @@ __device__ __forceinline__ void run_chunk_brick(const DevCtx& C, Stage& st, int 
 #pragma unroll
 		for (int s = 0; s < 8; s++) vw[s] = vws[s * kLanes + lane];
 #pragma unroll
-		for (int s = 0; s < 8; s++) {
-			if (vw[s] & kPrivate) {
-				const uint32_t p = vw[s] & ~kPrivate;
-				O[s] = sv[p];
-				D[s] = sv[C.bpriv_max + p];
-			} else {
-				ld_vertex(C.vert + 2 * (size_t)vw[s], O[s], D[s]);
-			}
-		}
+		for (int s = 0; s < 8; s++) vs.ld(C, vw[s], O[s], D[s]);
 #pragma unroll
 		for (int s = 0; s < 8; s++)
 			if (mask & (1u << s)) {
-				const uint32_t v = (vw[s] & kPrivate) ? spid[vw[s] & ~kPrivate] : vw[s];
+				const uint32_t v = vs.id(vw[s]);
 				if (ONE)
 					advance_vertex_bp(C, bp1, v, O[s], D[s], first, dt, inv_dt);
 				else
 					advance_vertex(C, v, O[s], D[s], first, dt, inv_dt, bodies);
 			}
-		solve_cube<false>(
+		solve_cube<false, !PAIR>(
 		    mat, rec + lane, inv_dt, inv_dt2, O, D, [](int, const float4*) {}, [](int, const float2&) {});
 	}
 	if (next >= 0) brick_issue(C, st, (uint32_t)next, lane);  // buffer consumed: prefetch
 	if (live) {
 #pragma unroll
-		for (int s = 0; s < 8; s++) {
-			if (vw[s] & kPrivate) {
-				const uint32_t p = vw[s] & ~kPrivate;
-				if (mask & (1u << s)) sv[p] = O[s];
-				sv[C.bpriv_max + p] = D[s];
-			} else if (mask & (1u << s)) {
-				st_vertex(C.vert + 2 * (size_t)vw[s], O[s], D[s]);
-			} else {
-				__stcg(C.vert + 2 * (size_t)vw[s] + 1, D[s]);
-			}
-		}
+		for (int s = 0; s < 8; s++) vs.st(C, vw[s], O[s], D[s], (mask & (1u << s)) != 0u);
 	}
 }
 
@@ -304,8 +285,14 @@ __device__ __forceinline__ void run_chunk_brick(const DevCtx& C, Stage& st, int 
 // launch so that every brick is resident), the plain solve only (no damping,
 // volume passes or multiplier output). The state between substeps stays
 // (O, D), and each brick finalizes its own vertices at the end.
-template <bool ONE>
-__global__ void __launch_bounds__(256) k_bricks(DevCtx C, uint32_t nsub, float dt) {
+// PAIR: two bricks per SM, of 192 threads at most and so of 168 registers a
+// thread. Told that bound, the compiler schedules within it (a frame of 1,572,864
+// tets: 928 us before, 902 so; reading records ahead would spill: 939). One brick
+// per SM has registers left, and reads a tet's record while the one before is
+// solved (four frames of a batch of 96 uneven bodies: 4,086 -> 3,815 us, and 3,695
+// with the vertices through generic addresses).
+template <bool ONE, bool PAIR>
+__global__ void __launch_bounds__(PAIR ? 192 : 256, PAIR ? 2 : 1) k_bricks(DevCtx C, uint32_t nsub, float dt) {
 	extern __shared__ __align__(128) uint8_t smem[];
 	__shared__ uint32_t s_bcb[65], s_bwait[64];
 	__shared__ BodyParams s_bodies[kBrickBodies];
@@ -317,6 +304,7 @@ __global__ void __launch_bounds__(256) k_bricks(DevCtx C, uint32_t nsub, float d
 	Stage st = brick_stage_init(lane);
 	float4* sv = reinterpret_cast<float4*>(smem + (size_t)wpb * kBrickChunkBytes);
 	uint32_t* spid = reinterpret_cast<uint32_t*>(sv + 2 * (size_t)C.bpriv_max);
+	const BrickVerts<!PAIR> vs = {sv, spid, C.bpriv_max};
 	for (uint32_t i = threadIdx.x; i <= ncol; i += blockDim.x) {
 		s_bcb[i] = __ldg(C.bchunk_begin + (size_t)b * ncol + i);
 		if (i < ncol) s_bwait[i] = __ldg(C.bchunk_wait_end + (size_t)b * ncol + i);
@@ -375,7 +363,7 @@ __global__ void __launch_bounds__(256) k_bricks(DevCtx C, uint32_t nsub, float d
 					break;
 				}
 				const int next = next_brick_chunk(s_bcb, ncol, s, nsub, c, ch, wib, wpb);
-				run_chunk_brick<ONE>(C, st, next, lane, s == 0, dt, inv_dt, inv_dt2, sv, spid, bodies, bshared, bp1,
+				run_chunk_brick<ONE, PAIR>(C, st, next, lane, s == 0, dt, inv_dt, inv_dt2, vs, bodies, bshared, bp1,
 				                     mat1);
 			}
 			if (__syncthreads_or(bad ? 1 : 0)) {
@@ -595,20 +583,25 @@ size_t brick_smem_bytes(int block, uint32_t bpriv_max) {
 	return (size_t)(block / 32) * kBrickChunkBytes + (size_t)bpriv_max * kBrickVertexBytes;
 }
 
+const void* bricks_fn(bool one, bool pair) {
+	if (pair) return one ? (const void*)k_bricks<true, true> : (const void*)k_bricks<false, true>;
+	return one ? (const void*)k_bricks<true, false> : (const void*)k_bricks<false, false>;
+}
+
 int brick_grid_fits(int block, uint32_t bpriv_max, uint32_t nbricks, bool* fits) {
 	const size_t smem = brick_smem_bytes(block, bpriv_max);
-	cudaError_t e = set_smem_attr((const void*)k_bricks<true>, smem);
-	if (e == cudaSuccess) e = set_smem_attr((const void*)k_bricks<false>, smem);
-	int dev = 0, sms = 0, per_sm = 0;
-	if (e == cudaSuccess) e = cudaGetDevice(&dev);
+	int dev = 0, sms = 0, per_sm = 1 << 20;
+	cudaError_t e = cudaGetDevice(&dev);
 	if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-	int per_sm1 = 0;
-	if (e == cudaSuccess)
-		e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)k_bricks<false>, block, smem);
-	if (e == cudaSuccess)
-		e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm1, (const void*)k_bricks<true>, block, smem);
+	for (int one = 0; one < 2 && e == cudaSuccess; one++) {
+		const void* f = bricks_fn(one != 0, nbricks > (uint32_t)sms);
+		int n = 0;
+		e = set_smem_attr(f, smem);
+		if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, f, block, smem);
+		per_sm = std::min(per_sm, n);
+	}
 	if (e != cudaSuccess) return (int)e;
-	*fits = (uint64_t)std::min(per_sm, per_sm1) * (uint64_t)sms >= nbricks && nbricks > 0;
+	*fits = (uint64_t)per_sm * (uint64_t)sms >= nbricks && nbricks > 0;
 	return 0;
 }
 
@@ -635,6 +628,10 @@ int launch_substeps(const DevCtx& ctx, const LaunchCfg& cfg, uint32_t nsub, floa
 		// pass counters start at 0; one launch counts at most 2^30 passes
 		const size_t smem_b = brick_smem_bytes(cfg.block, ctx.bpriv_max);
 		const uint32_t per = std::max(1u, (1u << 30) / std::max(1u, ctx.ncolours));
+		int dev = 0, sms = 0;
+		e = cudaGetDevice(&dev);
+		if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+		if (e != cudaSuccess) return (int)e;
 		for (uint32_t done = 0; done < nsub;) {
 			uint32_t n = std::min(per, nsub - done);
 			e = cudaMemsetAsync(ctx.bflag, 0, sizeof(uint32_t) * kBrickFlagStride * ctx.nbricks, st);
@@ -642,7 +639,7 @@ int launch_substeps(const DevCtx& ctx, const LaunchCfg& cfg, uint32_t nsub, floa
 			DevCtx c = ctx;
 			float dtv = dt;
 			void* args[] = {&c, &n, &dtv};
-			const void* f = ctx.nbodies == 1 ? (const void*)k_bricks<true> : (const void*)k_bricks<false>;
+			const void* f = bricks_fn(ctx.nbodies == 1, ctx.nbricks > (uint32_t)sms);
 			e = cudaLaunchCooperativeKernel(f, dim3(ctx.nbricks), dim3(cfg.block), args, smem_b, st);
 			if (e != cudaSuccess) return (int)e;
 			done += n;
