@@ -139,6 +139,7 @@ struct xfem_body {
 	DevBuf<float2> tlam;
 	DevBuf<int> err;
 	int* err_host = nullptr;  // pinned: the error word's read-back at every synchronising call
+	int* err_mapped = nullptr;  // its device address
 	DevBuf<float> stage;
 	DevBuf<double> vol;
 	// per tet, caller order (all bodies): record index of c0, volume, output
@@ -420,6 +421,14 @@ int device_error(int e) {
 	}
 }
 
+// Error word e of the device: cleared there and reported.
+int report_error(xfem_body* h, int e) {
+	if (e == 0) return XFEM_OK;
+	XCUDA(cudaMemsetAsync(h->err.p, 0, sizeof(int), h->stream));
+	XCUDA(cudaStreamSynchronize(h->stream));
+	return device_error(e);
+}
+
 int check_device_error(xfem_body* h) {
 	int e = 0;
 	if (h->err_host) {  // pinned: an asynchronous copy, no staging
@@ -430,12 +439,14 @@ int check_device_error(xfem_body* h) {
 		XCUDA(cudaMemcpyAsync(&e, h->err.p, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
 		XCUDA(cudaStreamSynchronize(h->stream));
 	}
-	if (e != 0) {
-		XCUDA(cudaMemsetAsync(h->err.p, 0, sizeof(int), h->stream));
-		XCUDA(cudaStreamSynchronize(h->stream));
-		return device_error(e);
-	}
-	return XFEM_OK;
+	return report_error(h, e);
+}
+
+// After a gather that brought the error word along (or not: check_device_error).
+int check_gathered_error(xfem_body* h, bool brought) {
+	if (!brought) return check_device_error(h);
+	XCUDA(cudaStreamSynchronize(h->stream));
+	return report_error(h, *h->err_host);
 }
 
 int prepare_mesh(const xfem_mesh& m, BodyHost& b) {
@@ -1617,6 +1628,7 @@ int build_device(xfem_body* h) {
 	XCUDA(h->err.alloc(1));
 	if (!h->err_host) XCUDA(cudaHostAlloc((void**)&h->err_host, sizeof(int), cudaHostAllocDefault));
 	*h->err_host = 0;
+	XCUDA(cudaHostGetDevicePointer((void**)&h->err_mapped, h->err_host, 0));
 	uint32_t maxnv = 1;
 	for (auto& b : h->bodies) maxnv = std::max(maxnv, b.nv);
 	XCUDA(h->stage.alloc(3 * (size_t)maxnv));
@@ -2078,20 +2090,21 @@ int get_xyz(xfem_body* h, uint32_t body, int which, float* out) {
 	if (!b) return XFEM_EINVAL;
 	if (!out) return fail(XFEM_EINVAL, "null output");
 	XCUDA(cudaSetDevice(h->device));
+	int* err_out = b->nv ? h->err_mapped : nullptr;  // no vertices, no gather
 	if (which <= 1) {
 		// positions or velocities into page-locked memory: the gather writes
 		// them there itself (no staging copy)
 		if (float* direct = static_cast<float*>(mapped_host(out))) {
-			const int e = launch_gather_xyz(h->vert.p, which, h->dev_of_vert.p + b->vbase, b->nv, direct, h->stream);
+			const int e = launch_gather_xyz(h->vert.p, which, h->dev_of_vert.p + b->vbase, b->nv, direct, h->err.p, err_out, h->stream);
 			if (e) return fail(XFEM_ECUDA, "gather launch failed");
-			return check_device_error(h);
+			return check_gathered_error(h, err_out != nullptr);
 		}
 	}
-	const int e = launch_gather_xyz(h->vert.p, which, h->dev_of_vert.p + b->vbase, b->nv, h->stage.p, h->stream);
+	const int e = launch_gather_xyz(h->vert.p, which, h->dev_of_vert.p + b->vbase, b->nv, h->stage.p, h->err.p, err_out, h->stream);
 	if (e) return fail(XFEM_ECUDA, "gather launch failed");
 	const size_t n = which >= 2 ? b->nv : 3 * (size_t)b->nv;
 	XCUDA(cudaMemcpyAsync(out, h->stage.p, n * sizeof(float), cudaMemcpyDeviceToHost, h->stream));
-	return check_device_error(h);
+	return check_gathered_error(h, err_out != nullptr);
 }
 
 // Queues the upload of one body's positions (which 0) or velocities (1) on
@@ -3170,9 +3183,9 @@ int xfem_adjoint_backward(xfem_body* h, const float* grad_tip_traj, const float*
 		XCUDA(cudaMemcpyAsync(h->vert.p, a.ckpt.p + 2 * nv * a.nseg, 2 * nv * sizeof(float4), cudaMemcpyDeviceToDevice,
 		                      h->stream));
 	// outputs in caller order, gathered on the device
-	if (dx0 && launch_gather_xyz(a.abar.p, 0, h->dev_of_vert.p, (uint32_t)nv, h->io.p, h->stream))
+	if (dx0 && launch_gather_xyz(a.abar.p, 0, h->dev_of_vert.p, (uint32_t)nv, h->io.p, nullptr, nullptr, h->stream))
 		return fail(XFEM_ECUDA, "gather launch failed");
-	if (dv0 && launch_gather_xyz(a.abar.p, 1, h->dev_of_vert.p, (uint32_t)nv, h->io.p + 3 * nv, h->stream))
+	if (dv0 && launch_gather_xyz(a.abar.p, 1, h->dev_of_vert.p, (uint32_t)nv, h->io.p + 3 * nv, nullptr, nullptr, h->stream))
 		return fail(XFEM_ECUDA, "gather launch failed");
 	if (dmu && launch_gather_dmu(a.cbar.p, h->tet_slot_dev.p, h->tet_inv_mu.p, h->ntets, h->io.p + 6 * nv, h->stream))
 		return fail(XFEM_ECUDA, "gather launch failed");

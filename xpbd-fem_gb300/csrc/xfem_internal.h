@@ -527,9 +527,10 @@ int launch_reverse(const DevCtx& ctx, const AdjCtx& adj, int block, uint32_t war
                    uint32_t nsub, float dt, bool last, void* stream);
 int configure_adjoint_kernels(int block, uint32_t warp_smem);
 
-// Transfer helpers (caller order <-> device order), run on `stream`.
+// Transfer helpers (caller order <-> device order), run on `stream`. The gather
+// also copies *err to *err_out, unless that is null.
 int launch_gather_xyz(const float4* vert, int which, const uint32_t* dev_of_caller, uint32_t n, float* out,
-                      void* stream);
+                      const int* err, int* err_out, void* stream);
 int launch_scatter_xyz(float4* vert, int which, const uint32_t* dev_of_caller, uint32_t n, const float* in,
                        void* stream);
 int launch_volume(const float4* vert, const uint32_t* tets_dev, uint32_t nt, double* out, void* stream);

