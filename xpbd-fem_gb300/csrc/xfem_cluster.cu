@@ -20,7 +20,7 @@
 // 98,304 tets, 16 blocks of 4 chunk warps, 1,172 -> 1,033 us; 78,336 tets in
 // clusters of every shape (20 colours) 2,427 -> 2,008 us; 6,144 damped tets, a
 // launch per substep, 967 -> 702 us for ten; the recording forward of 12,288
-// tets x 200 substeps 9.7 -> 6.9 ms.
+// tets x 200 substeps 9.7 -> 6.1 ms.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
