@@ -554,13 +554,16 @@ __global__ void __launch_bounds__(256) k_reverse(DevCtx C, AdjCtx A, uint32_t ns
 // masses and what the advance reverse reads come from the tape. So a block of
 // eight warps works on one chunk at a time: warp 0 runs the chain, a lane per
 // cluster, while warps 1-6 recompute the internals of the block's next chunk, a
-// warp per tet, and warp 7 loads its vertices' tape; then the eight warps finish
+// warp per tet, and warps 1-7 load its vertices' tape; then the eight warps finish
 // the chunk's eight vertices side by side. Same functions, same order: the
 // gradients equal the grid form's bit for bit.
 //
 // 12,288 tets x 200 substeps (8 chunks per pass, 8 blocks): 11.8 ms in the grid
-// form (152 blocks, 8 lanes per cluster), 7.7 ms here (10.0 before the vertex
-// ids were kept in shared memory and the tape's next substep prefetched to L2).
+// form (152 blocks, 8 lanes per cluster), 6.0 ms here (10.0 before the vertex
+// ids were kept in shared memory and the tape's next substep prefetched to L2,
+// 7.7 while warp 7 loaded all of a chunk's vertices). A pass of 7,500 cycles: the
+// chain 5,100, with the other warps' preparation of 2,500 to 4,800 beside it, the
+// finish 350, the barrier 1,900.
 
 // A cluster's tet in shared memory: TetFw and the record words its reverse
 // reads, as 16 float4 per lane.
@@ -637,29 +640,10 @@ __device__ __forceinline__ void reverse_cube(const RevStage& S, uint32_t lane, V
 
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
-// Warp `wib` (1-7) of the block prepares chunk R at launch substep s, and has
-// the same entries of the substep before it brought to L2 (the tape of a long
-// run comes from HBM).
-__device__ __forceinline__ void reverse_prepare(const DevCtx& C, const AdjCtx& A, RevStage& S, const RevChunk& R,
-                                                uint32_t s, bool first, uint32_t wib, uint32_t lane, float inv_dt2) {
-	const uint32_t hdr = R.hdr[lane];
-	if ((hdr & 15u) == 0u) return;
-	if (wib == 7u) {
-#pragma unroll 4
-		for (uint32_t k = 0; k < 8u; k++) {
-			const uint32_t v = R.vid[k][lane];
-			S.w[k][lane] = __ldcg(&tape_at(C, s, v)->w);
-			if (s > 0u) prefetch_l2(tape_at(C, s - 1u, v));
-			if ((hdr >> (8 + k)) & 1u) {
-				const OwnedTape t = owned_tape(C, A, v, s, first);
-				S.Op[k][lane] = t.Op;
-				S.Ds[k][lane] = t.Ds;
-				S.tip[k][lane] = make_float4(t.tip.x, t.tip.y, t.tip.z, 0.0f);
-			}
-		}
-		return;
-	}
-	const uint32_t j = wib - 1u;
+// Tet j of chunk R: its internals at launch substep s, and the same tape entry of
+// the substep before to L2.
+__device__ __forceinline__ void reverse_prepare_tet(const DevCtx& C, RevStage& S, const RevChunk& R, uint32_t s, uint32_t j,
+                                                    uint32_t lane, uint32_t hdr, float inv_dt2) {
 	const Mat mat = load_mat(C.bodies, hdr >> 16);
 	const float4* r = C.cblk + R.off16 + j * 4 * kLanes + lane;
 	const TetRec tr = {__ldg(r), __ldg(r + kLanes), __ldg(r + 2 * kLanes), __ldg(r + 3 * kLanes)};
@@ -685,6 +669,41 @@ __device__ __forceinline__ void reverse_prepare(const DevCtx& C, const AdjCtx& A
 	memcpy(words, &tw, sizeof(tw));
 #pragma unroll
 	for (uint32_t k = 0; k < kTetWords4; k++) S.tet[j][k][lane] = words[k];
+}
+
+// Warp `wib` (1-7) of the block prepares chunk R at launch substep s, and has
+// the same entries of the substep before it brought to L2 (the tape of a long
+// run comes from HBM).
+__device__ __forceinline__ void reverse_prepare(const DevCtx& C, const AdjCtx& A, RevStage& S, const RevChunk& R,
+                                                uint32_t s, bool first, uint32_t wib, uint32_t lane, float inv_dt2) {
+	const uint32_t hdr = R.hdr[lane];
+	if ((hdr & 15u) == 0u) return;
+	// What the finish reads of vertex wib - 1 (warp 7: also of vertex 7) is loaded
+	// ahead of the tet. All eight by warp 7 took it 6,700 cycles, 1,800 longer than
+	// the chain.
+	float vw[2];
+	OwnedTape own[2];
+#pragma unroll
+	for (uint32_t i = 0; i < 2u; i++) {
+		const uint32_t k = wib - 1u + i;
+		if (i == 1u && wib != 7u) break;
+		const uint32_t v = R.vid[k][lane];
+		vw[i] = __ldcg(&tape_at(C, s, v)->w);
+		if ((hdr >> (8 + k)) & 1u) own[i] = owned_tape(C, A, v, s, first);
+		if (s > 0u) prefetch_l2(tape_at(C, s - 1u, v));
+	}
+	if (wib < 7u) reverse_prepare_tet(C, S, R, s, wib - 1u, lane, hdr, inv_dt2);
+#pragma unroll
+	for (uint32_t i = 0; i < 2u; i++) {
+		const uint32_t k = wib - 1u + i;
+		if (i == 1u && wib != 7u) break;
+		S.w[k][lane] = vw[i];
+		if ((hdr >> (8 + k)) & 1u) {
+			S.Op[k][lane] = own[i].Op;
+			S.Ds[k][lane] = own[i].Ds;
+			S.tip[k][lane] = make_float4(own[i].tip.x, own[i].tip.y, own[i].tip.z, 0.0f);
+		}
+	}
 }
 
 __global__ void __launch_bounds__(256, 1) k_reverse_cluster(DevCtx C, AdjCtx A, uint32_t nsub, float dt, int last,
