@@ -56,8 +56,9 @@ __device__ bool grid_sync(const DevCtx& C, uint32_t& target) {
 	target += gridDim.x + C.wait_miss;
 	if (threadIdx.x == 0) {
 		int ok = 1;
-		__threadfence();
-		atomicAdd(C.bar_count, 1u);
+		// a release is enough on arrival: a full fence, which also drops L1, cost the
+		// element kernels 0 to 2.4% of a frame (48 x 25 x 24 H27s: 1,827 -> 1,782 us)
+		asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(C.bar_count) : "memory");
 		uint32_t spins = 0;
 		uint64_t t0 = 0;
 		while ((int32_t)(ld_relaxed_gpu(C.bar_count) - target) < 0) {
