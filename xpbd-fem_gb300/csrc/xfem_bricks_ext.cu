@@ -13,7 +13,7 @@
 // 8,800 for a damping pass (the brick has 2.6 chunks of a colour, on as many
 // warps), and 2,000 to 4,500 until the neighbours' pass counts are there.
 // Measured, a frame of 20 substeps with the interactive damping settings, grid
-// form before: 608,256 tets 1,872 -> 1,457 us, 3,145,728 tets (two bricks per SM)
+// form before: 608,256 tets 1,872 -> 1,417 us, 3,145,728 tets (two bricks per SM)
 // 3,808 -> 2,510.
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -169,17 +169,17 @@ __global__ void __launch_bounds__(PAIR ? 192 : 256, PAIR ? 2 : 1) k_bricks_ext(c
 			const uint32_t wend = s_bwait[c];
 			bool bad = false, waited = false;
 			for (uint32_t ch = s_bcb[c] + wib; ch < s_bcb[c + 1] && !bad; ch += wpb) {
+				if (!brick_acquire(C, st, ch, lane)) {
+					bad = true;
+					break;
+				}
+				const int next = next_of(ch, q, s);
 				if (ch < wend && !waited) {
 					bad = __any_sync(0xffffffffu, !brick_wait(C, C.bnb, nb0, nb1, epoch, lane, 32u));
 					__syncwarp();  // orders every lane's loads after the lanes' acquires
 					waited = true;
 					if (bad) break;
 				}
-				if (!brick_acquire(C, st, ch, lane)) {
-					bad = true;
-					break;
-				}
-				const int next = next_of(ch, q, s);
 				sweep_cube(C, vs, bps, st, ch, next, lane, sweep_of(C, kind), kind, dmode || s == 0, dmode, dt, inv_dt, inv_dt2,
 				           tick0 + s);
 			}
