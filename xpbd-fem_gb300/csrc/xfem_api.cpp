@@ -1132,10 +1132,90 @@ int build_mixed_tets(xfem_body* h) {
 	return XFEM_OK;
 }
 
+// Brick of each cluster (`lanes`: sorted keys, lowest device vertex << 32 | lane):
+// the clusters of one body are halved across their longest side, in proportion
+// to the bricks on either side, until each part is one brick. The clusters level
+// with the cut (within 0.4 of a cluster's size) are divided in Morton order, so
+// that a jittered layer is not scattered over both sides. A range of several
+// bodies is cut in order.
+void split_bricks(const xfem_body* h, const std::vector<uint64_t>& lanes, uint32_t nb, const std::vector<uint32_t>& lane_dv,
+                  const std::vector<uint8_t>& lane_nv, std::vector<uint32_t>& brick_of) {
+	std::vector<float> pos(3 * (size_t)h->nverts);
+	for (const BodyHost& b : h->bodies)
+		for (uint32_t v = 0; v < b.nv; v++)
+			for (int k = 0; k < 3; k++) pos[3 * (size_t)(b.vbase + b.sched.vert_rank[v]) + k] = b.nodes[3 * (size_t)v + k];
+	struct Cluster {
+		float c[3], ext[3];
+		uint32_t lane, order, body;
+	};
+	std::vector<Cluster> cl(lanes.size());
+	parallel_for((uint32_t)lanes.size(), [&](uint32_t j) {
+		Cluster& c = cl[j];
+		c.lane = (uint32_t)lanes[j];
+		c.order = j;
+		const uint32_t n = lane_nv[c.lane];
+		for (int k = 0; k < 3; k++) {
+			float lo = INFINITY, hi = -INFINITY;
+			for (uint32_t sl = 0; sl < n; sl++) {
+				const float x = pos[3 * (size_t)lane_dv[(size_t)c.lane * kMaxClusterVerts + sl] + k];
+				lo = std::min(lo, x), hi = std::max(hi, x);
+			}
+			const float mid = 0.5f * (lo + hi);
+			c.c[k] = isfinite(mid) ? mid : 0.0f, c.ext[k] = isfinite(hi - lo) ? hi - lo : 0.0f;
+		}
+		const uint32_t v = (uint32_t)(lanes[j] >> 32);
+		c.body = 0;
+		for (uint32_t lo = 0, hi = (uint32_t)h->bodies.size(); hi - lo > 1;) {
+			const uint32_t mid = (lo + hi) / 2;
+			(h->bodies[mid].vbase <= v ? lo : hi) = mid;
+			c.body = lo;
+		}
+	});
+	struct Range {
+		uint32_t b, e, k0, k1;  // clusters [b, e) are bricks [k0, k1)
+	};
+	std::vector<Range> level = {{0, (uint32_t)cl.size(), 0, nb}}, below;
+	while (!level.empty()) {
+		below.assign(2 * level.size(), Range{0, 0, 0, 0});
+		parallel_for((uint32_t)level.size(), [&](uint32_t i) {
+			const Range r = level[i];
+			if (r.k1 - r.k0 == 1) {
+				for (uint32_t j = r.b; j < r.e; j++) brick_of[cl[j].lane] = r.k0;
+				return;
+			}
+			const uint32_t nl = (r.k1 - r.k0) / 2, cut = r.b + (uint32_t)((uint64_t)(r.e - r.b) * nl / (r.k1 - r.k0));
+			if (cl[r.b].body == cl[r.e - 1].body) {
+				float lo[3], hi[3], ext[3] = {0, 0, 0};
+				for (int k = 0; k < 3; k++) lo[k] = INFINITY, hi[k] = -INFINITY;
+				for (uint32_t j = r.b; j < r.e; j++)
+					for (int k = 0; k < 3; k++) {
+						lo[k] = std::min(lo[k], cl[j].c[k]), hi[k] = std::max(hi[k], cl[j].c[k]);
+						ext[k] += cl[j].ext[k];
+					}
+				int a = 0;
+				for (int k = 1; k < 3; k++)
+					if (hi[k] - lo[k] > hi[a] - lo[a]) a = k;
+				const float level_with = 0.4f * ext[a] / (float)(r.e - r.b);
+				auto at = [&](uint32_t j) { return cl.begin() + j; };
+				std::nth_element(at(r.b), at(cut), at(r.e), [&](const Cluster& x, const Cluster& y) { return x.c[a] < y.c[a]; });
+				const float from = cl[cut].c[a] - level_with, to = cl[cut].c[a] + level_with;
+				const auto g = std::partition(at(r.b), at(r.e), [&](const Cluster& x) { return x.c[a] < from; });
+				const auto ge = std::partition(g, at(r.e), [&](const Cluster& x) { return x.c[a] <= to; });
+				std::sort(g, ge, [](const Cluster& x, const Cluster& y) { return x.order < y.order; });
+			}
+			below[2 * i] = {r.b, cut, r.k0, r.k0 + nl};
+			below[2 * i + 1] = {cut, r.e, r.k0 + nl, r.k1};
+		});
+		level.clear();
+		for (const Range& r : below)
+			if (r.k1 > r.k0) level.push_back(r);
+	}
+}
+
 // The brick layout of the launch form sync_mode 4 (k_bricks), built from the
-// packed cube chunks. Clusters are sorted by their lowest device vertex (a
-// Morton rank, so nearby clusters sort together) and cut into `nbricks`
-// runs of equal length: the bricks. A brick's clusters of one colour form its
+// packed cube chunks. The clusters are divided into `nbricks` runs along the
+// Morton curve (by lowest device vertex), or by split_bricks, of equal length
+// each: the bricks. A brick's clusters of one colour form its
 // chunks of that colour, in the colour's own order. A vertex whose clusters
 // all lie in one brick gets a slot in that brick's shared memory (up to
 // `slot_cap` per brick; the rest stay in vert). Bricks are neighbours when
@@ -1186,6 +1266,20 @@ int build_bricks(xfem_body* h, const std::vector<uint32_t>& ccb, const std::vect
 	const uint32_t nb = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(want, L / ((uint64_t)kLanes * ncol)));
 	std::vector<uint32_t> brick_of((size_t)nch * kLanes, 0xffffffffu);
 	for (uint64_t j = 0; j < L; j++) brick_of[(uint32_t)lanes[j]] = (uint32_t)(j * nb / L);
+	// Runs along the Morton curve, or the parts of split_bricks? The runs (aligned blocks of a
+	// grid, with as many cubes of each colour), unless some colour of a run has more than one
+	// chunk beyond one for each of the brick's warps, as the thin slabs beyond a power of two do.
+	// Measured, runs and parts, us per frame: 128 x 64 x 32 cubes 887 and 930, 64 x 48 x 48 724
+	// and 734, 83 x 41 x 30 642 and 647, 51 x 50 x 49 681 and 663; 127 x 65 x 33 (up to eight
+	// chunks on six warps) 1,188 and 962, with damping 2,402 and 1,917. (The parts have the
+	// smaller surface, 48% of the cubes on it instead of 62%, but less even colours.)
+	bool parts = false;
+	std::vector<uint32_t> of_colour((size_t)nb * ncol, 0);
+	for (const uint64_t key : lanes)
+		parts = ++of_colour[(size_t)brick_of[(uint32_t)key] * ncol + chunk_colour[(uint32_t)key / kLanes]] >
+		            kLanes * ((uint32_t)h->brick_block / 32u + 1u) ||
+		        parts;
+	if (parts) split_bricks(h, lanes, nb, lane_dv, lane_nv, brick_of);
 	// (vertex, brick) incidences
 	// every cluster touching each vertex, as colour << 16 | brick; chunks are
 	// colour-major, so each vertex's touches come in ascending colour order
