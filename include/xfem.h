@@ -160,7 +160,8 @@ typedef struct xfem_options {
 	                          (xfem_info.cluster_mode tells which). The layout fixes the colour
 	                          order, so the choice changes results within rounding */
 	uint32_t no_morton;    /* 1 = keep the caller's vertex order on the device */
-	uint32_t sync_mode;    /* 0 = auto (autotuned), 1 = persistent kernel + grid barrier, 2 = CUDA graph,
+	uint32_t sync_mode;    /* 0 = auto (autotuned), 1 = persistent kernel + grid barrier (small handles: one
+	                          thread-block cluster; 0 only: damping and volume sweeps over bricks), 2 = CUDA graph,
 	                          3 = persistent kernel, chunks wait only on neighbouring chunks (dataflow),
 	                          4 = persistent kernel over bricks: each block owns a compact brick of cube
 	                          clusters whose own vertices stay in shared memory, and waits only on the
