@@ -13,7 +13,7 @@
 // 8,800 for a damping pass (the brick has 2.6 chunks of a colour, on as many
 // warps), and 2,000 to 4,500 until the neighbours' pass counts are there.
 // Measured, a frame of 20 substeps with the interactive damping settings, grid
-// form before: 608,256 tets 1,872 -> 1,417 us, 3,145,728 tets (two bricks per SM)
+// form before: 608,256 tets 1,872 -> 1,396 us, 3,145,728 tets (two bricks per SM)
 // 3,808 -> 2,510.
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -43,23 +43,19 @@ __device__ __forceinline__ Sweep sweep_of(const DevCtx& C, uint32_t kind) {
 // registers on the stack (1,040 bytes, 160 of them spilled) and a damped frame of
 // 608,256 tets took 1,773 us; so, with no stack, 1,515 then.
 template <class VS, class BP>
-__device__ __forceinline__ void sweep_cube(const DevCtx& C, const VS& vs, const BP& bps, Stage& st, uint32_t chunk, int next,
+__device__ __forceinline__ void sweep_cube(const DevCtx& C, const VS& vs, const BP& bps, Stage& st, const BrickLane& bl, uint32_t chunk, int next,
                                            uint32_t lane, Sweep sweep, uint32_t k, bool first, bool finish, float dt,
                                            float inv_dt, float inv_dt2, uint32_t tick) {
 	const uint32_t trow = chunk * 6u;
 	const float4* rec = reinterpret_cast<const float4*>(st.buf);
-	const uint32_t* hdrs = reinterpret_cast<const uint32_t*>(st.buf + 2048u * 6u);
-	const uint32_t* vids = hdrs + kLanes;
-	const uint32_t hdr = hdrs[lane];
+	const uint32_t hdr = bl.hdr;
+	const uint32_t* vid = bl.vw;
 	const bool live = (hdr & 15u) != 0, solve = sweep == Sweep::kSolve;
 	const uint32_t mask = solve ? (hdr >> 8) & 0xffu : 0u;
-	uint32_t vid[8];
 	float4 O[8], D[8];  // a damping sweep's X and V
 	uint32_t last = 0;  // the vertices that this pass finishes, with damping sweeps
 	uint32_t some = 0;  // bit t: tet t has work
 	if (live) {
-#pragma unroll
-		for (int s = 0; s < 8; s++) vid[s] = vids[s * kLanes + lane];
 #pragma unroll
 		for (int s = 0; s < 8; s++) vs.ld(C, vid[s], O[s], D[s]);
 		const Mat mat = bps.mat(C, hdr >> 16);
@@ -174,13 +170,16 @@ __global__ void __launch_bounds__(PAIR ? 192 : 256, PAIR ? 2 : 1) k_bricks_ext(c
 					break;
 				}
 				const int next = next_of(ch, q, s);
+				BrickLane bl;
+				if (!PAIR) bl = brick_lane(st, lane);
 				if (ch < wend && !waited) {
 					bad = __any_sync(0xffffffffu, !brick_wait(C, C.bnb, nb0, nb1, epoch, lane, 32u));
 					__syncwarp();  // orders every lane's loads after the lanes' acquires
 					waited = true;
 					if (bad) break;
 				}
-				sweep_cube(C, vs, bps, st, ch, next, lane, sweep_of(C, kind), kind, dmode || s == 0, dmode, dt, inv_dt, inv_dt2,
+				if (PAIR) bl = brick_lane(st, lane);
+				sweep_cube(C, vs, bps, st, bl, ch, next, lane, sweep_of(C, kind), kind, dmode || s == 0, dmode, dt, inv_dt, inv_dt2,
 				           tick0 + s);
 			}
 			if (__syncthreads_or(bad ? 1 : 0)) {

@@ -563,6 +563,23 @@ __device__ __forceinline__ bool brick_acquire(const DevCtx& C, Stage& st, uint32
 	return ok;
 }
 
+// What a lane needs of its resident brick chunk before its vertices. With one brick
+// per SM it is read ahead of the wait for the neighbours (a damped frame of 608,256
+// tets: 1,418 -> 1,396 us; with two per SM after it: 2,510 us against 2,525 for
+// 3,145,728).
+struct BrickLane {
+	uint32_t hdr, vw[8];
+};
+
+__device__ __forceinline__ BrickLane brick_lane(const Stage& st, uint32_t lane) {
+	const uint32_t* p = reinterpret_cast<const uint32_t*>(st.buf + 2048u * 6u) + lane;
+	BrickLane l;
+	l.hdr = p[0];
+#pragma unroll
+	for (int s = 0; s < 8; s++) l.vw[s] = p[(s + 1) * kLanes];
+	return l;
+}
+
 // Bounded wait, by the calling threads (`first` of them striding by
 // `stride`), until every brick of list[nb0, nb1) (ALL: every brick in [nb0,
 // nb1), without a list) has published at least

@@ -244,22 +244,18 @@ __device__ __forceinline__ int next_brick_chunk(const uint32_t* bcb, uint32_t nc
 // ONE: a single body, whose parameters bp1 and material mat1 the kernel holds
 // in registers.
 template <bool ONE, bool PAIR>
-__device__ __forceinline__ void run_chunk_brick(const DevCtx& C, Stage& st, int next, uint32_t lane, bool first,
+__device__ __forceinline__ void run_chunk_brick(const DevCtx& C, Stage& st, const BrickLane& bl, int next, uint32_t lane, bool first,
                                                 float dt, float inv_dt, float inv_dt2, const BrickVerts<!PAIR>& vs,
                                                 const BodyParams* bodies, bool bshared,
                                                 const BodyParams& bp1, const Mat& mat1) {
 	const float4* rec = reinterpret_cast<const float4*>(st.buf);
-	const uint32_t* hdrs = reinterpret_cast<const uint32_t*>(st.buf + 2048u * 6u);
-	const uint32_t* vws = hdrs + kLanes;
-	const uint32_t hdr = hdrs[lane];
+	const uint32_t hdr = bl.hdr;
+	const uint32_t* vw = bl.vw;
 	const bool live = (hdr & 15u) != 0;
 	const uint32_t mask = (hdr >> 8) & 0xffu;
-	uint32_t vw[8];
 	float4 O[8], D[8];
 	if (live) {
 		const Mat mat = ONE ? mat1 : bshared ? load_mat_shared(bodies, hdr >> 16) : load_mat(bodies, hdr >> 16);
-#pragma unroll
-		for (int s = 0; s < 8; s++) vw[s] = vws[s * kLanes + lane];
 #pragma unroll
 		for (int s = 0; s < 8; s++) vs.ld(C, vw[s], O[s], D[s]);
 #pragma unroll
@@ -358,6 +354,8 @@ __global__ void __launch_bounds__(PAIR ? 192 : 256, PAIR ? 2 : 1) k_bricks(DevCt
 					break;
 				}
 				const int next = next_brick_chunk(s_bcb, ncol, s, nsub, c, ch, wib, wpb);
+				BrickLane bl;
+				if (!PAIR) bl = brick_lane(st, lane);
 				if (ch < wend && !waited) {
 					const uint32_t q = b * ncol + c;
 					bad = __any_sync(0xffffffffu, !brick_wait(C, C.bcnb, __ldg(C.bcnb_begin + q),
@@ -366,7 +364,8 @@ __global__ void __launch_bounds__(PAIR ? 192 : 256, PAIR ? 2 : 1) k_bricks(DevCt
 					waited = true;
 					if (bad) break;
 				}
-				run_chunk_brick<ONE, PAIR>(C, st, next, lane, s == 0, dt, inv_dt, inv_dt2, vs, bodies, bshared, bp1,
+				if (PAIR) bl = brick_lane(st, lane);
+				run_chunk_brick<ONE, PAIR>(C, st, bl, next, lane, s == 0, dt, inv_dt, inv_dt2, vs, bodies, bshared, bp1,
 				                     mat1);
 			}
 			if (__syncthreads_or(bad ? 1 : 0)) {
