@@ -191,7 +191,10 @@ typedef struct xfem_mesh {
 typedef struct xfem_info {
 	uint32_t bodies, vertices, tets, clusters, colours;
 	uint32_t isolated;        /* vertices in no tet */
-	uint32_t chunks, tet_rows, block_size, blocks;
+	uint32_t chunks, tet_rows, block_size;
+	uint32_t blocks;          /* the grid of the form that sync_mode names, which the allocation-free
+	                             call runs too (a small or damped handle may step in another form:
+	                             xfem_get_launch) */
 	uint32_t sync_mode;       /* 1 persistent + grid barrier, 2 CUDA graph, 3 persistent dataflow,
 	                             4 persistent bricks */
 	uint32_t cluster_mode;    /* 1 one tet per cluster, 2 edge stars */
@@ -199,6 +202,26 @@ typedef struct xfem_info {
 	uint32_t bricks;          /* bricks of the brick layout (0: none built) */
 	uint64_t device_bytes;
 } xfem_info;
+
+/* How a call ran on the device (xfem_get_launch). */
+enum {
+	XFEM_FORM_NONE = 0,       /* no such call yet */
+	XFEM_FORM_GRID = 1,       /* persistent kernel + grid barrier */
+	XFEM_FORM_GRAPH = 2,      /* CUDA graph of colour launches (blocks: those of the largest) */
+	XFEM_FORM_DATAFLOW = 3,   /* persistent kernel, waits on neighbouring chunks */
+	XFEM_FORM_BRICKS = 4,     /* persistent kernel over bricks */
+	XFEM_FORM_CLUSTER = 5,    /* one thread-block cluster */
+	XFEM_FORM_BRICKS_EXT = 6, /* damping and volume sweeps over bricks */
+	XFEM_FORM_ELEMENTS = 7,   /* hexes, T10s, H27s and meshes mixing them */
+	XFEM_FORM_RINGS = 8       /* the continuous-pressure models */
+};
+typedef struct xfem_launch {
+	uint32_t form;            /* XFEM_FORM_* */
+	uint32_t blocks, threads; /* of the kernel launch */
+	uint32_t lanes;           /* lanes of a warp per cluster of tets, element (T10s where T10s and H27s
+	                             mix) or ring */
+} xfem_launch;
+enum { XFEM_LAUNCH_STEP = 0, XFEM_LAUNCH_RECORD = 1, XFEM_LAUNCH_REVERSE = 2 };
 
 typedef struct xfem_body xfem_body;
 
@@ -239,6 +262,10 @@ int xfem_batch_create(uint32_t nbodies, const xfem_mesh* meshes, const xfem_sett
                       const xfem_options* options, xfem_body** out);
 int xfem_destroy(xfem_body* b);
 int xfem_get_info(const xfem_body* b, xfem_info* out);
+/* How the handle's last stepping call, adjoint forward or adjoint backward
+ * (which: XFEM_LAUNCH_*) ran: the forms give the same results at different
+ * speeds, and which one a handle takes follows from its size and settings. */
+int xfem_get_launch(const xfem_body* b, uint32_t which, xfem_launch* out);
 
 /* ---- parameters ---------------------------------------------------------- */
 /* Replaces the UpdateSettings export (wasm/main.cpp:80-95) for one body. */

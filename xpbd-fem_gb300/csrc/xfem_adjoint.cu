@@ -886,6 +886,7 @@ int launch_reverse(const DevCtx& ctx, const AdjCtx& adj, int block, uint32_t, ui
 			AdjCtx a = adj;
 			int lastv = last ? 1 : 0;
 			void* args[] = {&c, &a, &nsub, &dt, &lastv, &rounds};
+			note_launch(XFEM_FORM_CLUSTER, G, 256, 1);
 			return (int)cudaLaunchKernelExC(&lc, (const void*)k_reverse_cluster, args);
 		}
 	}
@@ -912,6 +913,7 @@ int launch_reverse(const DevCtx& ctx, const AdjCtx& adj, int block, uint32_t, ui
 	int grouped = (uint64_t)max_colour_chunks * 8u <= (uint64_t)blocks * (uint32_t)(block / 32) ? 1 : 0;
 	if (form) grouped = form[0] == 'g' ? 1 : form[0] == 'l' ? 0 : grouped;
 	void* args[] = {&c, &a, &nsub, &dt, &lastv, &grouped};
+	note_launch(XFEM_FORM_GRID, blocks, (uint32_t)block, grouped ? 8 : 1);
 	return (int)cudaLaunchCooperativeKernel((const void*)k_reverse, dim3(blocks), dim3(block), args, smem, st);
 }
 

@@ -189,9 +189,11 @@ struct xfem_body {
 	float tune_ms = 0.0f;  // the autotuner's best trial time (3 calls), when it timed any
 	// cached CUDA graph (graph mode)
 	cudaGraphExec_t graph = nullptr;
+	xfem_launch graph_launch{};  // of the captured launches
 	uint32_t graph_nsub = 0;
 	float graph_dt = 0.0f;
 	uint64_t device_bytes = 0;
+	xfem_launch launched[3]{};  // by XFEM_LAUNCH_*
 
 	~xfem_body() {
 		if (err_host) cudaFreeHost(err_host);
@@ -1945,6 +1947,7 @@ int run(xfem_body* h, uint32_t nsub, float dt) {
 	if (h->cfg.sync_mode == 1 || h->cfg.sync_mode == 3 || h->cfg.sync_mode == 4) {
 		const int e = launch_substeps(h->ctx, h->cfg, nsub, dt, h->stream);
 		if (e) return fail(XFEM_ECUDA, std::string("persistent launch: ") + cudaGetErrorString((cudaError_t)e));
+		h->launched[XFEM_LAUNCH_STEP] = t_launched;
 		return XFEM_OK;
 	}
 	if (!h->graph || h->graph_nsub != nsub || h->graph_dt != dt) {
@@ -1963,8 +1966,10 @@ int run(xfem_body* h, uint32_t nsub, float dt) {
 		if (ei != cudaSuccess) return fail(XFEM_ECUDA, std::string("graph instantiate: ") + cudaGetErrorString(ei));
 		h->graph_nsub = nsub;
 		h->graph_dt = dt;
+		h->graph_launch = t_launched;
 	}
 	XCUDA(cudaGraphLaunch(h->graph, h->stream));
+	h->launched[XFEM_LAUNCH_STEP] = h->graph_launch;
 	return XFEM_OK;
 }
 
@@ -2107,6 +2112,7 @@ int launch_mode(xfem_body* h, const DevCtx& ctx, uint32_t nsub, float dt) {
 		              : h->el_mode == kElH27 ? launch_h27_rings(ctx, 128, nsub, dt, h->stream)
 		                                     : launch_rings(ctx, nsub, dt, h->stream);
 		if (e) return fail(XFEM_ECUDA, std::string("ring launch: ") + cudaGetErrorString((cudaError_t)e));
+		h->launched[XFEM_LAUNCH_STEP] = t_launched;
 		return XFEM_OK;
 	}
 	if (h->el_mode == kElQMixed) {
@@ -2121,6 +2127,7 @@ int launch_mode(xfem_body* h, const DevCtx& ctx, uint32_t nsub, float dt) {
 		ct.nel = h->q_nel;
 		const int e = launch_qmixed(ctx, ct, 256, nsub, dt, h->stream);
 		if (e) return fail(XFEM_ECUDA, std::string("element launch: ") + cudaGetErrorString((cudaError_t)e));
+		h->launched[XFEM_LAUNCH_STEP] = t_launched;
 		return XFEM_OK;
 	}
 	const int e = h->el_mode == kElH27     ? launch_h27(ctx, nsub, dt, h->stream)
@@ -2128,6 +2135,7 @@ int launch_mode(xfem_body* h, const DevCtx& ctx, uint32_t nsub, float dt) {
 	              : h->el_mode == kElMixed ? launch_mixed(ctx, 256, nsub, dt, h->stream)
 	                                       : launch_hexes(ctx, nsub, dt, h->stream);
 	if (e) return fail(XFEM_ECUDA, std::string("element launch: ") + cudaGetErrorString((cudaError_t)e));
+	h->launched[XFEM_LAUNCH_STEP] = t_launched;
 	return XFEM_OK;
 }
 
@@ -2356,6 +2364,13 @@ int xfem_get_info(const xfem_body* b, xfem_info* out) {
 	return XFEM_OK;
 }
 
+int xfem_get_launch(const xfem_body* b, uint32_t which, xfem_launch* out) {
+	if (!b || !out) return fail(XFEM_EINVAL, "null argument");
+	if (which > XFEM_LAUNCH_REVERSE) return fail(XFEM_EINVAL, "XFEM_LAUNCH_STEP, _RECORD or _REVERSE");
+	*out = b->launched[which];
+	return XFEM_OK;
+}
+
 int xfem_set_settings(xfem_body* h, uint32_t body, const xfem_settings* s) {
 	BodyHost* b = body_of(h, body);
 	if (!b) return XFEM_EINVAL;
@@ -2479,6 +2494,7 @@ int xfem_step_frames_noalloc(xfem_body* h, uint32_t frames, uint32_t substeps, f
 		return fail(XFEM_ELIMIT, "one call's grid-barrier arrivals (substeps x passes per substep x persistent "
 		                         "blocks) must stay below 2^31; split the call");
 	if (e) return fail(XFEM_ECUDA, std::string("allocation-free launch: ") + cudaGetErrorString((cudaError_t)e));
+	h->launched[XFEM_LAUNCH_STEP] = t_launched;
 	if (dev_err) return device_error(dev_err);
 	return XFEM_OK;
 }
@@ -3212,6 +3228,7 @@ int xfem_adjoint_forward(xfem_body* h, uint32_t nsub, float dt, uint32_t checkpo
 		const int e = launch_substeps_tape(tape_ctx(h, j), block, h->cfg.warp_smem, h->max_colour_chunks, seg_len(a, j), dt, h->stream);
 		if (e) return fail(XFEM_ECUDA, std::string("recording launch: ") + cudaGetErrorString((cudaError_t)e));
 	}
+	h->launched[XFEM_LAUNCH_RECORD] = t_launched;
 	if (nseg > 1)
 		XCUDA(cudaMemcpyAsync(a.ckpt.p + 2 * nv * nseg, h->vert.p, 2 * nv * sizeof(float4), cudaMemcpyDeviceToDevice,
 		                      h->stream));
@@ -3273,6 +3290,7 @@ int xfem_adjoint_backward(xfem_body* h, const float* grad_tip_traj, const float*
 		                             j == (int)a.nseg - 1, h->stream);
 		if (e) return fail(XFEM_ECUDA, std::string("reverse launch: ") + cudaGetErrorString((cudaError_t)e));
 	}
+	h->launched[XFEM_LAUNCH_REVERSE] = t_launched;
 	if (a.nseg > 1)
 		XCUDA(cudaMemcpyAsync(h->vert.p, a.ckpt.p + 2 * nv * a.nseg, 2 * nv * sizeof(float4), cudaMemcpyDeviceToDevice,
 		                      h->stream));

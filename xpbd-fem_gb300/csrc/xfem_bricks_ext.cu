@@ -271,6 +271,7 @@ int launch_bricks_ext(const DevCtx& ctx, int block, uint32_t nsub, float dt, voi
 		DevCtx c = ctx;
 		float dtv = dt;
 		void* args[] = {&c, &n, &dtv};
+		note_launch(XFEM_FORM_BRICKS_EXT, ctx.nbricks, (uint32_t)block, 1);
 		e = cudaLaunchCooperativeKernel(f, dim3(ctx.nbricks), dim3(block), args, smem, st);
 		if (e != cudaSuccess) return (int)e;
 		done += n;

@@ -249,6 +249,7 @@ int launch_cluster(const DevCtx& ctx, const ClusterPlan& plan, int block, bool t
 	DevCtx c = ctx;
 	ClusterPlan p = plan;
 	void* args[] = {&c, &p, &nsub, &dt};
+	note_launch(XFEM_FORM_CLUSTER, plan.blocks, (uint32_t)block, 1);
 	return (int)cudaLaunchKernelExC(&lc, cluster_fn(tape, ext, ctx.nbodies == 1), args);
 }
 

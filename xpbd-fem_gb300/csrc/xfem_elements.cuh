@@ -372,6 +372,7 @@ int launch_elements(const DevCtx& ctx, uint32_t nsub, float dt, void* stream) {
 	if (e != cudaSuccess) return (int)e;
 	DevCtx c = ctx;
 	void* args[] = {&c, &nsub, &dt};
+	note_launch(XFEM_FORM_ELEMENTS, (uint32_t)(per_sm * sms), (uint32_t)block, (uint32_t)E::kLanes);
 	return (int)cudaLaunchCooperativeKernel(f, dim3(per_sm * sms), dim3(block), args, E::smem(), st);
 }
 

@@ -293,6 +293,7 @@ int launch_hex_rings(const DevCtx& ctx, int block, uint32_t nsub, float dt, void
 	if (e != cudaSuccess) return (int)e;
 	DevCtx c = ctx;
 	void* args[] = {&c, &nsub, &dt};
+	note_launch(XFEM_FORM_RINGS, (uint32_t)(per_sm * sms), (uint32_t)block, 32);
 	return (int)cudaLaunchCooperativeKernel(f, dim3(per_sm * sms), dim3(block), args, smem, st);
 }
 

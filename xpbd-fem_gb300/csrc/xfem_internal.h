@@ -7,6 +7,7 @@
 
 #include <vector>
 
+#include "xfem.h"
 #include "xfem_rest.h"
 
 namespace xfem {
@@ -462,6 +463,13 @@ constexpr uint64_t kDefaultTimeoutNs = 2000000000ull;
 struct ClusterPlan {
 	uint32_t blocks = 0, warps = 0, bufs = 0;
 };
+
+// The last kernel launch of the calling thread, for xfem_get_launch: every
+// launcher of a stepping, recording or reverse kernel notes it.
+inline thread_local xfem_launch t_launched = {};
+inline void note_launch(uint32_t form, uint32_t blocks, uint32_t threads, uint32_t lanes) {
+	t_launched = {form, blocks, threads, lanes};
+}
 
 struct LaunchCfg {
 	int block = 256;

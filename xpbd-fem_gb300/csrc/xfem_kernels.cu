@@ -653,6 +653,7 @@ int launch_substeps(const DevCtx& ctx, const LaunchCfg& cfg, uint32_t nsub, floa
 			float dtv = dt;
 			void* args[] = {&c, &n, &dtv};
 			const void* f = bricks_fn(ctx.nbodies == 1, ctx.nbricks > (uint32_t)sms);
+			note_launch(XFEM_FORM_BRICKS, ctx.nbricks, (uint32_t)cfg.block, 1);
 			e = cudaLaunchCooperativeKernel(f, dim3(ctx.nbricks), dim3(cfg.block), args, smem_b, st);
 			if (e != cudaSuccess) return (int)e;
 			done += n;
@@ -673,6 +674,7 @@ int launch_substeps(const DevCtx& ctx, const LaunchCfg& cfg, uint32_t nsub, floa
 		const void* f = cfg.sync_mode == 1
 		                    ? persistent_fn(cfg.lambdas, cfg.ext)
 		                    : (cfg.lambdas ? (const void*)k_dataflow<true> : (const void*)k_dataflow<false>);
+		note_launch(cfg.sync_mode == 1 ? XFEM_FORM_GRID : XFEM_FORM_DATAFLOW, (uint32_t)cfg.blocks, (uint32_t)cfg.block, 1);
 		e = cudaLaunchCooperativeKernel(f, dim3(cfg.blocks), dim3(cfg.block), args, smem, st);
 		return (int)e;
 	}
@@ -682,6 +684,7 @@ int launch_substeps(const DevCtx& ctx, const LaunchCfg& cfg, uint32_t nsub, floa
 	const uint32_t warps_per_block = cfg.block / 32;
 	const bool dmode = cfg.ext && ctx.damp_kinds != 0u;
 	const uint32_t kinds = cfg.ext ? 1u + ctx.nvol + (uint32_t)__builtin_popcount(ctx.damp_kinds) : 1u;
+	uint32_t largest = 0;
 	for (uint32_t s = 0; s < nsub; s++) {
 		for (uint32_t kind = 0; kind < kinds; kind++) {
 			for (uint32_t c = 0; c < ctx.ncolours; c++) {
@@ -691,6 +694,7 @@ int launch_substeps(const DevCtx& ctx, const LaunchCfg& cfg, uint32_t nsub, floa
 				if (s == 0 && kind == 0 && c == 0 && ctx.nisolated) extra = (ctx.nisolated + cfg.block - 1) / cfg.block;
 				const uint32_t grid = sb + extra;
 				if (grid == 0) continue;
+				largest = std::max(largest, grid);
 				DevCtx cc = ctx;
 				uint32_t colour = c, ns = nsub, kd = kind, sub = s;
 				int first = (dmode || s == 0) ? 1 : 0;
@@ -701,6 +705,7 @@ int launch_substeps(const DevCtx& ctx, const LaunchCfg& cfg, uint32_t nsub, floa
 			}
 		}
 	}
+	note_launch(XFEM_FORM_GRAPH, largest, (uint32_t)cfg.block, 1);
 	const uint32_t fb = (ctx.nverts + 255) / 256;
 	if (fb && !dmode) {
 		k_finalize<<<fb, 256, 0, st>>>(ctx, dt);
@@ -711,7 +716,7 @@ int launch_substeps(const DevCtx& ctx, const LaunchCfg& cfg, uint32_t nsub, floa
 	return (int)cudaGetLastError();
 }
 
-// The recording forward: k_persistent with the tape writes compiled in. The
+// The recording forward: k_cluster or, for larger handles, k_persistent with the tape writes compiled in. The
 // arithmetic is the same inlined code as the plain launch, so the trajectory
 // is the plain launch's bit for bit.
 int launch_substeps_tape(const DevCtx& ctx, int block, uint32_t warp_smem, uint32_t max_colour_chunks, uint32_t nsub,
@@ -737,6 +742,7 @@ int launch_substeps_tape(const DevCtx& ctx, int block, uint32_t warp_smem, uint3
 	if (e != cudaSuccess) return (int)e;
 	DevCtx c = ctx;
 	void* args[] = {&c, &nsub, &dt};
+	note_launch(XFEM_FORM_GRID, (uint32_t)(per_sm * sms), (uint32_t)block, 1);
 	return (int)cudaLaunchCooperativeKernel(f, dim3(per_sm * sms), dim3(block), args, smem, st);
 }
 
@@ -839,6 +845,7 @@ int launch_substeps_noalloc(const DevCtx& ctx, int block, uint32_t warp_smem, bo
 	c.bar_count = p;
 	c.err = reinterpret_cast<int*>(p + 1);
 	void* args[] = {&c, &nsub, &dt};
+	note_launch(XFEM_FORM_GRID, blocks, (uint32_t)block, 1);
 	e = cudaLaunchCooperativeKernel(f, dim3(blocks), dim3(block), args, smem, st);
 	if (e != cudaSuccess) return (int)e;
 	e = cudaMemcpyAsync(device_error, p + 1, sizeof(int), cudaMemcpyDeviceToHost, st);

@@ -136,6 +136,7 @@ int launch_qmixed(const DevCtx& ch27, const DevCtx& ct10, int block, uint32_t ns
 	if (e != cudaSuccess) return (int)e;
 	DevCtx a = ch27, b = ct10;
 	void* args[] = {&a, &b, &nsub, &dt};
+	note_launch(XFEM_FORM_ELEMENTS, (uint32_t)(per_sm * sms), (uint32_t)block, (uint32_t)T10::kLanes);
 	return (int)cudaLaunchCooperativeKernel(f, dim3(per_sm * sms), dim3(block), args, kQMixedSmem, st);
 }
 

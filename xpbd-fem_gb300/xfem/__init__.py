@@ -88,6 +88,15 @@ class Info(C.Structure):
                                           "cluster_mode", "max_chunk_deps", "bricks")] + [("device_bytes", C.c_uint64)]
 
 
+class Launch(C.Structure):
+    _fields_ = [(n, C.c_uint32) for n in ("form", "blocks", "threads", "lanes")]
+
+
+# XFEM_FORM_*, in order
+FORMS = ("none", "grid", "graph", "dataflow", "bricks", "cluster", "bricks_ext", "elements", "rings")
+LAUNCH_STEP, LAUNCH_RECORD, LAUNCH_REVERSE = 0, 1, 2
+
+
 # every symbol include/xfem.h declares
 EXPORTS = [
     "xfem_settings_default", "xfem_create", "xfem_create_ex", "xfem_batch_create", "xfem_destroy",
@@ -103,7 +112,7 @@ EXPORTS = [
     "xfem_body_t10_count", "xfem_get_t10_rest_state", "xfem_get_t10_schedule", "xfem_compute_t10_edges",
     "xfem_compute_t10_rest_state", "xfem_compute_t10_schedule", "xfem_body_h27_count", "xfem_get_h27_rest_state",
     "xfem_get_h27_schedule", "xfem_compute_h27_mesh", "xfem_compute_h27_rest_state", "xfem_compute_h27_schedule",
-    "xfem_test_hook", "xfem_get_mixed_tet_schedule", "xfem_compute_mixed_rest_state", "xfem_compute_mixed_schedule",
+    "xfem_test_hook", "xfem_get_launch", "xfem_get_mixed_tet_schedule", "xfem_compute_mixed_rest_state", "xfem_compute_mixed_schedule",
 ]
 HEX_EP = 120  # floats per hex rest-state record (ElementParamsLinearHex flattened)
 T10_EP = 56  # floats per T10 rest-state record (ElementParamsQuadraticTet flattened)
@@ -135,6 +144,7 @@ def lib():
         L.xfem_batch_create.argtypes = [u32, P, P, P, P]
         L.xfem_destroy.argtypes = [P]
         L.xfem_get_info.argtypes = [P, P]
+        L.xfem_get_launch.argtypes = [P, u32, P]
         L.xfem_set_settings.argtypes = [P, u32, P]
         L.xfem_set_lock_mask.argtypes = [P, u32, P]
         L.xfem_set_tet_mu.argtypes = [P, u32, P]
@@ -498,6 +508,13 @@ class Body:
         i = Info()
         _check(lib().xfem_get_info(self._h, C.byref(i)))
         return {n: getattr(i, n) for n, _ in Info._fields_}
+
+    def launch(self, which=LAUNCH_STEP):
+        """How the last stepping call (or adjoint forward, adjoint backward) ran:
+        its form (FORMS), blocks, threads per block and lanes."""
+        r = Launch()
+        _check(lib().xfem_get_launch(self._h, which, C.byref(r)))
+        return dict(form=FORMS[r.form], blocks=r.blocks, threads=r.threads, lanes=r.lanes)
 
     # -- parameters
     def set_settings(self, s, body=0):
