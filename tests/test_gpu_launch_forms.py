@@ -111,6 +111,32 @@ def test_sweeps_on_bricks(dims, block):
     assert a.launch()["form"] == "grid"
 
 
+def test_sweeps_on_bricks_wait_times_out_and_recovers():
+    """A neighbour wait that expects one pass more than the bricks publish runs out
+    after the short limit, and the handle steps normally afterwards."""
+    mesh = _tets(49, 33, 31)
+    b = _automatic([mesh], block_size=256, wait_timeout_ms=100)
+    ref = xfem.Body(*mesh, _settings(), sync_mode=1, block_size=256)
+    x0 = mesh[0].reshape(-1, 3)
+    for h in (ref, b):  # the locks take hold in the first substep
+        h.set_settings(_settings(**DAMPED))
+        h.step_frames(1, 1, DT)
+        h.set_positions(x0)
+        h.set_velocities(np.zeros_like(x0))
+    assert b.launch()["form"] == "bricks_ext"
+    ref.step_frames(1, 6, DT)
+    xfem.test_hook(b, xfem.HOOK_MISSING_ARRIVAL, 1)
+    b.step_frames(1, 6, DT)
+    with pytest.raises(xfem.XfemError) as e:
+        b.synchronize()
+    assert e.value.code == xfem.EDEVICE_TIMEOUT
+    b.set_positions(x0)
+    b.set_velocities(np.zeros_like(x0))
+    b.step_frames(1, 6, DT)
+    assert b.launch()["form"] == "bricks_ext"
+    assert np.array_equal(b.positions(), ref.positions()) and np.array_equal(b.velocities(), ref.velocities())
+
+
 def test_elements_and_rings():
     nodes, idx = xfem.generate_hex_block(4, 3, 3, (0.05, 0.05, 0.05), 0, 0.2)
     ring = 9 << xfem.ENERGY_BIT
