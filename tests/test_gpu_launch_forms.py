@@ -150,3 +150,33 @@ def test_elements_and_rings():
         b.step_frames(1, 2, DT)
         assert b.launch()["form"] == form and b.launch()["lanes"] == lanes, flags
         assert b.launch()["blocks"] >= 1
+
+
+@pytest.mark.parametrize("volume_passes", [0, 2])
+def test_one_lane_t10s_of_every_energy(volume_passes):
+    """A colour beyond one round of four-lane warps takes a lane per T10
+    (xfem_t10_lane.cu): bodies of every energy, coupled and serial, with every damping
+    type, step in such a batch as each does alone with four lanes."""
+    kinds = (4, 0, 7, 3, 1, 6, 2, 5, 11, 4, 7, 3, 0, 31, 12, 5)
+    meshes, settings = [], []
+    for k in range(48):
+        energy, rtype = kinds[k % len(kinds)], (k + k // 4) % 4
+        meshes.append(xfem.generate_tet_block(12, 10, 9, (0.1, 0.1, 0.1), 0, 0.2) + (1000.0,))
+        settings.append(xfem.default_settings(
+            gravity=(0.3, -9.81, -2.0), compliance=4e-5 * (1 + k % 5), poissons_ratio=0.45,
+            damping=0.0 if k % 3 == 0 else 0.002, pbd_damping=0.02 * (k % 2),
+            volume_and_time_corrected_pbd_damping=0.01, amortized_volume_and_time_corrected_pbd_damping=0.05,
+            volume_passes=volume_passes * (k % 2),
+            flags=xfem.ELEMENT_T10 | (energy << xfem.ENERGY_BIT) | (rtype << 20) | xfem.LOCK_LEFT |
+            ((k % 5 != 1) << xfem.XPBD_SOLVE_BIT)))
+    batch = xfem.Body(meshes=meshes, settings=settings)
+    batch.step_frames(1, 9, DT)
+    assert batch.launch()["lanes"] == 1
+    # every energy with both solves and every damping type
+    for k in range(2 * len(kinds)):
+        one = xfem.Body(*meshes[k], settings[k])
+        one.step_frames(1, 9, DT)
+        assert one.launch()["lanes"] == 4
+        assert np.array_equal(one.positions(), batch.positions(k)), k
+        assert np.array_equal(one.velocities(), batch.velocities(k)), k
+        assert np.isfinite(one.positions()).all(), k
