@@ -180,3 +180,16 @@ def test_one_lane_t10s_of_every_energy(volume_passes):
         assert np.array_equal(one.positions(), batch.positions(k)), k
         assert np.array_equal(one.velocities(), batch.velocities(k)), k
         assert np.isfinite(one.positions()).all(), k
+
+
+def test_h27_rings_fill_the_sms():
+    """A ring is one warp's chain, so large meshes need many warps in flight: 15 per SM
+    (blocks of four with their own copy of the tables left 8)."""
+    torch = pytest.importorskip("torch")
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    nodes, idx = xfem.generate_hex_block(5, 4, 3, (0.05, 0.05, 0.05), 0, 0.2)
+    for kw in ({}, dict(damping=0.005), DAMPED):
+        flags = (9 << xfem.ENERGY_BIT) | xfem.ELEMENT_H27 | (kw.get("flags", 0) & (3 << 20))
+        b = xfem.Body(nodes, idx, 1000.0, _settings(**{**kw, "flags": flags}))
+        b.step_frames(1, 2, DT)
+        assert b.launch()["blocks"] * b.launch()["threads"] // 32 >= 15 * sms

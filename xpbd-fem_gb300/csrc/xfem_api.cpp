@@ -2109,7 +2109,7 @@ int launch_mode(xfem_body* h, const DevCtx& ctx, uint32_t nsub, float dt) {
 	if (h->ring_mode) {
 		const int e = h->el_mode == kElHexes ? launch_hex_rings(ctx, 256, nsub, dt, h->stream)
 		              : h->el_mode == kElT10 ? launch_t10_rings(ctx, 128, nsub, dt, h->stream)
-		              : h->el_mode == kElH27 ? launch_h27_rings(ctx, 128, nsub, dt, h->stream)
+		              : h->el_mode == kElH27 ? launch_h27_rings(ctx, nsub, dt, h->stream)
 		                                     : launch_rings(ctx, nsub, dt, h->stream);
 		if (e) return fail(XFEM_ECUDA, std::string("ring launch: ") + cudaGetErrorString((cudaError_t)e));
 		h->launched[XFEM_LAUNCH_STEP] = t_launched;

@@ -563,7 +563,7 @@ int launch_t10_lane(const DevCtx& ctx, uint32_t nsub, float dt, void* stream);  
 // of one-ring solves over the T10s around the mesh vertices, a cooperative
 // persistent launch (canonical (X, V) in and out).
 int launch_t10_rings(const DevCtx& ctx, int block, uint32_t nsub, float dt, void* stream);
-int launch_h27_rings(const DevCtx& ctx, int block, uint32_t nsub, float dt, void* stream);
+int launch_h27_rings(const DevCtx& ctx, uint32_t nsub, float dt, void* stream);  // block size: kRingWarps of xfem_h27.cu
 // A mesh mixing T10s and H27s: ch27 with the H27 element arrays, ct10 the
 // same context with the T10 element arrays (blocks of 256 threads).
 int launch_qmixed(const DevCtx& ch27, const DevCtx& ct10, int block, uint32_t nsub, float dt, void* stream);
