@@ -193,3 +193,23 @@ def test_h27_rings_fill_the_sms():
         b = xfem.Body(nodes, idx, 1000.0, _settings(**{**kw, "flags": flags}))
         b.step_frames(1, 2, DT)
         assert b.launch()["blocks"] * b.launch()["threads"] // 32 >= 15 * sms
+
+
+@pytest.mark.parametrize("energy", [xfem.ENERGY_CUBE_NEO, xfem.ENERGY_CUBE_SKIN])
+@pytest.mark.parametrize("opts", [dict(sync_mode=1, block_size=128), dict(sync_mode=2, block_size=128),
+                                  dict(sync_mode=1, block_size=128, keep_lambdas=True),
+                                  dict(sync_mode=2, block_size=128, cluster_mode=1, keep_lambdas=True)])
+def test_cube_models_leave_tets_alone(energy, opts):
+    """Every vertex of a tet mesh with a cube model falls as one, and the multipliers
+    are zero, in the forms of whole cubes and of single tets."""
+    nodes, idx, density = _tets(9, 7, 5)
+    s = _settings(flags=(energy << xfem.ENERGY_BIT) | (1 << xfem.XPBD_SOLVE_BIT))
+    b = xfem.Body(nodes, idx, density, s, **opts)
+    b.step_frames(1, 6, DT)
+    assert b.launch()["form"] == ("graph" if opts["sync_mode"] == 2 else "grid" if "keep_lambdas" in opts else "cluster")
+    v = b.velocities()
+    # each substep rounds (v + g dt) drag and the position it is taken from: a few ulps of x / dt
+    tol = 6 * 4 * 2.0 ** -24 * np.abs(nodes).max() / DT
+    assert np.abs(v - v.mean(0)).max() <= tol and v[:, 1].max() < -6 * 9.0 * DT
+    if "keep_lambdas" in opts:
+        assert not b.lambdas().any()
