@@ -213,3 +213,30 @@ def test_cube_models_leave_tets_alone(energy, opts):
     assert np.abs(v - v.mean(0)).max() <= tol and v[:, 1].max() < -6 * 9.0 * DT
     if "keep_lambdas" in opts:
         assert not b.lambdas().any()
+
+
+def test_a_handle_follows_its_settings_off_the_bricks_and_back():
+    """A damped handle whose sweeps run on the bricks keeps them when the damping is
+    switched off, takes a form with the extended solves for the Pixar models, and comes
+    back; each time it steps as a handle that stays on the grid."""
+    mesh = _tets(49, 33, 31)
+    b = None
+    for _ in range(8):  # its forms are timed: on a busy GPU another one can win
+        b = xfem.Body(*mesh, _settings(**DAMPED))
+        b.step_frames(1, 20, DT)
+        if b.launch()["form"] == "bricks_ext":
+            break
+    else:
+        pytest.skip("the GPU is busy: another form was timed fastest eight times")
+    a = xfem.Body(*mesh, _settings(**DAMPED), sync_mode=1, block_size=256)
+    a.step_frames(1, 20, DT)
+    pixar = _settings(flags=(xfem.ENERGY_PIXAR_SEL << xfem.ENERGY_BIT) | (1 << xfem.XPBD_SOLVE_BIT) | xfem.LOCK_LEFT)
+    plain, damped = _settings(), _settings(**DAMPED)
+    for s, forms in ((plain, ["bricks"]), (damped, ["bricks_ext"]), (pixar, ["graph", "grid"]), (plain, ["bricks"]),
+                     (pixar, ["graph", "grid"]), (damped, ["bricks_ext"]), (pixar, ["graph", "grid"]),
+                     (damped, ["bricks_ext"]), (plain, ["bricks"])):
+        for h in (a, b):
+            h.set_settings(s)
+            h.step_frames(1, 3, DT)
+        assert b.launch()["form"] in forms
+        assert np.array_equal(a.positions(), b.positions()) and np.array_equal(a.velocities(), b.velocities())

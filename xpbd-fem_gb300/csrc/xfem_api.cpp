@@ -187,6 +187,9 @@ struct xfem_body {
 	bool tuned = false;
 	int brick_block = 256;  // the brick form's default block size (192 with two bricks per SM)
 	float tune_ms = 0.0f;  // the autotuner's best trial time (3 calls), when it timed any
+	// A handle whose sweeps run on the bricks (cfg.brick_ext): the fastest form timed beside
+	// them, and the bricks' block size while the settings need that form (follow_settings)
+	int off_bricks_sync = 0, off_bricks_block = 0, left_bricks_block = 0;
 	// cached CUDA graph (graph mode)
 	cudaGraphExec_t graph = nullptr;
 	xfem_launch graph_launch{};  // of the captured launches
@@ -1943,6 +1946,29 @@ int set_config(xfem_body* h, int sync_mode, int block) {
 	return XFEM_OK;
 }
 
+// After a change of the settings, for a tuned handle that fixes no form: where the sweeps ran
+// on the bricks, the plain solve does too (sync_mode 4; step() brings them back with the
+// sweeps), and the extended solves, which have no brick kernel, take the fastest other form
+// of the tuning. The block size chosen for the bricks does not suit the grid: 1,572,864 tets,
+// after damping, in one frame of the grid at 192 threads 1,597 us (a second round of chunks;
+// with Pixar 1,842), on the bricks 890 (the colour graph with Pixar 1,429).
+void follow_settings(xfem_body* h, bool was_on_bricks, int block) {
+	if (!h->tuned || h->opt.sync_mode != 0 || h->cfg.brick_ext || h->cfg.cluster.blocks) return;
+	const int level = h->cfg.ext_level();
+	if (!was_on_bricks) {
+		if (!h->left_bricks_block || level == 2) return;
+		block = h->left_bricks_block;
+	}
+	// a form that does not fit leaves the handle as it is
+	if (level == 0)
+		set_config(h, 4, block);
+	else if (level == 1)
+		set_config(h, 1, block);
+	else if (h->off_bricks_sync)
+		set_config(h, h->off_bricks_sync, h->off_bricks_block);
+	h->left_bricks_block = level == 2 ? block : 0;
+}
+
 int run(xfem_body* h, uint32_t nsub, float dt) {
 	if (h->cfg.sync_mode == 1 || h->cfg.sync_mode == 3 || h->cfg.sync_mode == 4) {
 		const int e = launch_substeps(h->ctx, h->cfg, nsub, dt, h->stream);
@@ -2015,7 +2041,7 @@ int autotune(xfem_body* h, uint32_t nsub, float dt, bool force_time = false) {
 	XCUDA(cudaEventCreate(&e0));
 	XCUDA(cudaEventCreate(&e1));
 	const uint32_t ns = std::max(1u, std::min(nsub, 20u));
-	float best = 1e30f;
+	float best = 1e30f, best_off_bricks = 1e30f;
 	std::pair<int, int> pick = cand[0];
 	for (auto& c : cand) {
 		if (set_config(h, c.first, c.second)) continue;
@@ -2030,6 +2056,11 @@ int autotune(xfem_body* h, uint32_t nsub, float dt, bool force_time = false) {
 		if (ms < best) {
 			best = ms;
 			pick = c;
+		}
+		if (ms < best_off_bricks && c.first <= 2 && !(c.first == 1 && h->cfg.brick_ext)) {
+			best_off_bricks = ms;
+			h->off_bricks_sync = c.first;
+			h->off_bricks_block = c.second;
 		}
 	}
 	cudaEventDestroy(e0);
@@ -2412,8 +2443,10 @@ int xfem_set_settings(xfem_body* h, uint32_t body, const xfem_settings* s) {
 			int blocks = 0;
 			if (persistent_grid(h->cfg, &blocks) == 0) h->cfg.blocks = blocks;
 		}
+		const bool was_on_bricks = h->cfg.brick_ext;
 		if (const int e = pick_cluster(h))
 			return fail(XFEM_ECUDA, std::string("cluster query failed: ") + cudaGetErrorString((cudaError_t)e));
+		follow_settings(h, was_on_bricks, h->cfg.block);
 	}
 	if (h->ring_mode) h->ctx.ext = ring_damp_of(h->bodies) ? 1u : 0u;
 	const float4* rt_before = h->ctx.right_target;
