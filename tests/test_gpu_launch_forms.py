@@ -152,34 +152,114 @@ def test_elements_and_rings():
         assert b.launch()["blocks"] >= 1
 
 
-@pytest.mark.parametrize("volume_passes", [0, 2])
-def test_one_lane_t10s_of_every_energy(volume_passes):
-    """A colour beyond one round of four-lane warps takes a lane per T10
-    (xfem_t10_lane.cu): bodies of every energy, coupled and serial, with every damping
-    type, step in such a batch as each does alone with four lanes."""
-    kinds = (4, 0, 7, 3, 1, 6, 2, 5, 11, 4, 7, 3, 0, 31, 12, 5)
-    meshes, settings = [], []
-    for k in range(48):
-        energy, rtype = kinds[k % len(kinds)], (k + k // 4) % 4
-        meshes.append(xfem.generate_tet_block(12, 10, 9, (0.1, 0.1, 0.1), 0, 0.2) + (1000.0,))
-        settings.append(xfem.default_settings(
+def _quadratic_kinds(flags, volume_passes):
+    """Settings of every energy, coupled and serial, with every damping type."""
+    out = []
+    for k, energy in enumerate(2 * (4, 0, 7, 3, 1, 6, 2, 5, 11, 4, 7, 3, 0, 31, 12, 5)):
+        out.append(xfem.default_settings(
             gravity=(0.3, -9.81, -2.0), compliance=4e-5 * (1 + k % 5), poissons_ratio=0.45,
             damping=0.0 if k % 3 == 0 else 0.002, pbd_damping=0.02 * (k % 2),
             volume_and_time_corrected_pbd_damping=0.01, amortized_volume_and_time_corrected_pbd_damping=0.05,
             volume_passes=volume_passes * (k % 2),
-            flags=xfem.ELEMENT_T10 | (energy << xfem.ENERGY_BIT) | (rtype << 20) | xfem.LOCK_LEFT |
+            flags=flags | (energy << xfem.ENERGY_BIT) | (((k + k // 4) % 4) << 20) | xfem.LOCK_LEFT |
             ((k % 5 != 1) << xfem.XPBD_SOLVE_BIT)))
-    batch = xfem.Body(meshes=meshes, settings=settings)
-    batch.step_frames(1, 9, DT)
-    assert batch.launch()["lanes"] == 1
-    # every energy with both solves and every damping type
-    for k in range(2 * len(kinds)):
-        one = xfem.Body(*meshes[k], settings[k])
-        one.step_frames(1, 9, DT)
-        assert one.launch()["lanes"] == 4
-        assert np.array_equal(one.positions(), batch.positions(k)), k
-        assert np.array_equal(one.velocities(), batch.velocities(k)), k
-        assert np.isfinite(one.positions()).all(), k
+    return out
+
+
+def _coupled(flags):
+    return _settings(flags=flags | W.NH_FLAGS)
+
+
+@pytest.mark.parametrize("volume_passes", [0, 2])
+def test_one_and_four_lane_t10s_of_every_energy(volume_passes):
+    """Which kernel a handle of T10s takes follows from its largest colour and from what
+    most of its T10s solve: bodies of every kind step alike in a batch that takes one lane
+    per T10, in one that takes four, and alone."""
+    kinds = _quadratic_kinds(xfem.ELEMENT_T10, volume_passes)
+    mesh = xfem.generate_tet_block(12, 10, 9, (0.1, 0.1, 0.1), 0, 0.2) + (1000.0,)
+    small = xfem.generate_tet_block(3, 2, 2, (0.1, 0.1, 0.1), 0, 0.2) + (1000.0,)
+    one = xfem.Body(meshes=[mesh] * 48, settings=kinds + kinds[:16])
+    # a few larger coupled bodies are most of the T10s
+    four = xfem.Body(meshes=[small] * len(kinds) + [mesh], settings=kinds + [_coupled(xfem.ELEMENT_T10)])
+    alone = [xfem.Body(*small, s) for s in kinds]
+    for h in [one, four] + alone:
+        h.step_frames(1, 9, DT)
+    assert one.launch()["lanes"] == 1 and four.launch()["lanes"] == 4
+    assert {a.launch()["lanes"] for a in alone} == {1, 4}
+    for k, a in enumerate(alone):
+        assert np.array_equal(a.positions(), four.positions(k)), k
+        assert np.array_equal(a.velocities(), four.velocities(k)), k
+    for k in (0, 1, 2, 3, 5, 6, 7, 9, 13, 17, 18, 22):  # and at the larger size
+        lanes = xfem.Body(meshes=[mesh] * 3, settings=[kinds[k]] + 2 * [_coupled(xfem.ELEMENT_T10)])
+        lanes.step_frames(1, 9, DT)
+        assert lanes.launch()["lanes"] == 4
+        assert np.array_equal(one.positions(k), lanes.positions(0)), k
+        assert np.array_equal(one.velocities(k), lanes.velocities(0)), k
+        assert np.isfinite(one.positions(k)).all(), k
+
+
+@pytest.mark.parametrize("kw,lanes", [
+    (dict(), 4), (dict(flags=W.YEOH_FLAGS), 4), (dict(damping=0.002), 1), (dict(pbd_damping=0.02), 4),
+    (dict(damping=0.002, flags=W.NH_FLAGS | (2 << 20)), 4), (dict(volume_passes=2), 4),
+    (dict(flags=(xfem.ENERGY_MIXED_SEL << xfem.ENERGY_BIT) | xfem.LOCK_LEFT), 1),
+    (dict(flags=(xfem.ENERGY_MIXED << xfem.ENERGY_BIT) | xfem.LOCK_LEFT), 4),
+    (dict(flags=(xfem.ENERGY_PIXAR << xfem.ENERGY_BIT) | xfem.LOCK_LEFT, damping=0.002), 4),
+    (dict(flags=(xfem.ENERGY_PIXAR_SEL << xfem.ENERGY_BIT) | xfem.LOCK_LEFT, damping=0.002), 1)])
+def test_lanes_per_t10_by_settings(kw, lanes):
+    flags = kw.get("flags", W.NH_FLAGS) | xfem.ELEMENT_T10
+    b = xfem.Body(*_tets(4, 3, 2), _settings(**{**kw, "flags": flags}))
+    b.step_frames(1, 1, DT)
+    assert b.launch()["lanes"] == lanes
+    b.set_settings(_settings(flags=W.NH_FLAGS | xfem.ELEMENT_T10))
+    b.step_frames(1, 1, DT)
+    assert b.launch()["lanes"] == 4
+
+
+def _tets_and_hexes(w, h, d, every):
+    """A block of hexes, all but each `every`-th cell split into six tets."""
+    nodes, idx = xfem.generate_hex_block(w, h, d, (0.1, 0.1, 0.1), 0, 0.2)
+    six = ((0, 1, 5, 7), (0, 7, 3, 1), (0, 2, 3, 7), (0, 7, 6, 2), (0, 4, 6, 7), (0, 7, 5, 4))
+    out = []
+    for k, c in enumerate(idx.reshape(-1, 9)):
+        if k % every == 0:
+            out.extend(c)
+        else:
+            for t in six:
+                out.append(4)
+                out.extend(c[1:][list(t)])
+    return nodes, np.array(out, np.uint32), 1000.0
+
+
+@pytest.mark.parametrize("volume_passes", [0, 2])
+def test_one_and_four_lane_t10s_beside_h27s(volume_passes):
+    """The same on meshes mixing T10s and H27s."""
+    kinds = _quadratic_kinds(xfem.ELEMENT_H27, volume_passes)
+    mesh, small = _tets_and_hexes(12, 10, 9, 20), _tets_and_hexes(3, 3, 2, 4)
+    one = xfem.Body(meshes=[mesh] * 40, settings=kinds + kinds[:8])
+    four = xfem.Body(meshes=[small] * len(kinds) + [mesh], settings=kinds + [_coupled(xfem.ELEMENT_H27)])
+    alone = [xfem.Body(*small, s) for s in kinds]
+    for h in [one, four] + alone:
+        h.step_frames(1, 9, DT)
+    assert one.launch()["lanes"] == 1 and four.launch()["lanes"] == 4
+    assert {a.launch()["lanes"] for a in alone} == {1, 4}
+    for k, a in enumerate(alone):
+        assert np.array_equal(a.positions(), four.positions(k)), k
+        assert np.array_equal(a.velocities(), four.velocities(k)), k
+    for k in (0, 1, 3, 5, 9, 13, 18):
+        lanes = xfem.Body(meshes=[mesh] * 3, settings=[kinds[k]] + 2 * [_coupled(xfem.ELEMENT_H27)])
+        lanes.step_frames(1, 9, DT)
+        assert lanes.launch()["lanes"] == 4
+        assert np.array_equal(one.positions(k), lanes.positions(0)), k
+        assert np.array_equal(one.velocities(k), lanes.velocities(0)), k
+        assert np.isfinite(one.positions(k)).all(), k
+
+
+# most of the cells tets: up to one round of four-lane warps (8 T10s x 8 warps a SM), beyond it
+@pytest.mark.parametrize("bodies,lanes", [(6, 4), (40, 1)])
+def test_lanes_per_t10_beside_h27s_by_size(bodies, lanes):
+    b = xfem.Body(meshes=[_tets_and_hexes(12, 10, 9, 20)] * bodies, settings=[_coupled(xfem.ELEMENT_H27)] * bodies)
+    b.step_frames(1, 1, DT)
+    assert b.launch()["lanes"] == lanes
 
 
 def test_h27_rings_fill_the_sms():

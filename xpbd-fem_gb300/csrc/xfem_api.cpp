@@ -124,6 +124,7 @@ struct AdjointRun {
 
 struct xfem_body {
 	int device = 0;
+	uint32_t sms = 0;
 	cudaStream_t stream = nullptr;
 	bool own_stream = false;
 	xfem_options opt{};
@@ -180,6 +181,7 @@ struct xfem_body {
 	DevBuf<uint32_t> q_cb, q_flat;
 	DevBuf<float> q_tab;
 	uint32_t q_colours = 0, q_nel = 0;
+	uint32_t max_colour_t10 = 0;  // T10s of the largest colour
 	uint32_t nisolated = 0, max_deps = 0;
 	LaunchCfg cfg;
 	DevCtx ctx{};
@@ -1067,13 +1069,14 @@ static int build_element_set(xfem_body* h, uint32_t kind, bool qt) {
 	XCUDA(up(flatb.p, flat.data(), flat.size() * 4));
 	XCUDA(up(tabb.p, g4.data(), g4.size() * 4));
 	XCUDA(cudaStreamSynchronize(h->stream));
+	if (kind == kElT10)
+		for (uint32_t c = 0; c < ncol; c++) h->max_colour_t10 = std::max(h->max_colour_t10, cb[c + 1] - cb[c]);
 	if (qt) {
 		h->q_colours = ncol;
 		h->q_nel = nel;
 	} else {
 		h->ctx.el_colours = ncol;
 		h->ctx.nel = nel;
-		for (uint32_t c = 0; c < ncol; c++) h->ctx.max_colour_el = std::max(h->ctx.max_colour_el, cb[c + 1] - cb[c]);
 	}
 	h->device_bytes += vid.size() * 16 + rec.size() * 16 + cb.size() * 4 + flat.size() * 4 + g4.size() * 4;
 	return XFEM_OK;
@@ -2100,6 +2103,9 @@ int create_common(uint32_t nbodies, const xfem_mesh* meshes, const xfem_settings
 		XCUDA(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking));
 		h->own_stream = true;
 	}
+	int sms = 0;
+	XCUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device));
+	h->sms = (uint32_t)sms;
 	h->bodies.resize(nbodies);
 	SetupClock clk;
 	int rc = prepare_bodies(h.get(), nbodies, meshes, settings, mode, morton);
@@ -2135,6 +2141,62 @@ BodyHost* body_of(xfem_body* h, uint32_t body) {
 	return &h->bodies[body];
 }
 
+// The largest colour, as a share of the T10s that one round of four-lane warps takes, up
+// to which four lanes per T10 step a body with these settings at least as fast as one. Four
+// lanes finish a pass of few T10s sooner; one lane does less work per T10, by more the more
+// of the solve is not shared out: the prefactored term's energy, sums in node order, the
+// steps of a serial or damped solve, which every lane of the four goes through. Measured,
+// us per frame of 20 substeps with one lane and with four, T10s of the largest colour in
+// brackets (a round: 14,592):
+//   MixedSel, YeohSkinFast: coupled [10,080] 4,303 and 3,500, [14,118] 5,247 and 4,027,
+//     [52,000] 12.3 and 14.0 ms; serial [8] 2,809 and 2,902, [323] 3,538 and 3,645, [10,080]
+//     4,376 and 5,165; damped in the solve [8] 2,840 and 3,122, [14,118] 5,342 and 6,540;
+//     damped after it [5,724] 7,975 and 7,653, [10,080] 8,725 and 9,175
+//   Mixed, YeohSkin: [5,724] 3,952 and 3,727, [10,080] 4,257 and 4,402; serial [5,724] 4,464
+//     and 4,429, [10,080] 4,780 and 5,217; damped in the solve [323] 3,594 and 3,634;
+//     volume sweeps [2,328] 9,177 and 9,022, [5,724] 9,963 and 10,114
+//   YeohSkinSel: [10,080] 4,763 and 4,422, [14,118] 4,818 and 5,131; serial [5,724] 4,499 and
+//     4,446; damped in the solve [5,724] 4,548 and 4,406, [10,080] 4,866 and 5,257; serial too
+//     [323] 4,103 and 4,119; volume sweeps [5,724] 10,455 and 10,127, [10,080] 11,250 and 12,101
+//   Pixar, PixarReduced: [5,724] 3,271 and 3,087, [10,080] 3,556 and 3,713; damped in the solve
+//     [2,328] 3,048 and 3,051; volume sweeps [2,328] 8,480 and 8,398, [5,724] 9,275 and 9,488
+//   PixarSel: [323] 3,156 and 3,055, [2,328] 3,349 and 3,367; damped in the solve [323] 3,206
+//     and 3,313; damped after it [8] 5,167 and 5,199, [2,328] 6,977 and 7,224
+float four_lane_share(const xfem_settings& s) {
+	const uint32_t energy = (s.flags >> XFEM_ENERGY_BIT) & XFEM_ENERGY_MASK;
+	const bool serial = !((s.flags >> XFEM_XPBD_SOLVE_BIT) & 1u);
+	const bool in_solve = s.damping > 0.0f && ((s.flags >> XFEM_RAYLEIGH_TYPE_BIT) & 3u) < XFEM_RAYLEIGH_POST;
+	const bool sweeps = s.volume_passes > 0 || (s.damping > 0.0f && !in_solve);
+	switch (energy) {
+	case XFEM_ENERGY_PIXAR:
+	case XFEM_ENERGY_PIXAR_REDUCED: return in_solve ? 0.15f : sweeps ? 0.25f : 0.55f;
+	case XFEM_ENERGY_PIXAR_SEL: return in_solve || sweeps || s.pbd_damping > 0.0f ? 0.0f : 0.1f;
+	case XFEM_ENERGY_MIXED:
+	case XFEM_ENERGY_YEOH_SKIN: return in_solve ? 0.0f : sweeps ? 0.25f : serial ? 0.4f : 0.55f;
+	case XFEM_ENERGY_YEOH_SKIN_SEL: return in_solve && serial ? 0.0f : serial ? 0.4f : in_solve || sweeps ? 0.5f : 0.85f;
+	case XFEM_ENERGY_CUBE_NEO:
+	case XFEM_ENERGY_CUBE_SKIN: return 1.0f;  // T10s are left alone
+	default: return in_solve || serial ? 0.0f : sweeps ? 0.56f : 1.0f;
+	}
+}
+
+// Lanes of a warp per T10 for this handle, whose four-lane kernel takes `round` T10s of a
+// colour at once: four where most of its T10s are in bodies that gain by it. general: the
+// shares below one are for the T10 mode's kernel, which fetches elements ahead; meshes that
+// mix T10s and H27s do not, and cross over at three quarters (95% of the cells tets, Pixar
+// [3,976 of 9,728] 3,301 and 3,282, [7,883] 3,517 and 4,161; coupled MixedSel [12,510] 5,273
+// and 5,304, [24,772] 6,323 and 8,377).
+int t10_lanes(const xfem_body* h, uint32_t round, float general = 1.0f) {
+	uint64_t all = 0, four = 0;
+	for (const BodyHost& b : h->bodies) {
+		const uint64_t n = b.el == kElQMixed ? b.nqt : b.nh;
+		const float share = four_lane_share(b.settings);
+		all += n;
+		if ((float)h->max_colour_t10 <= (share < 1.0f ? general * share : share) * (float)round) four += n;
+	}
+	return 2 * four >= all ? 4 : 1;
+}
+
 // The element and one-ring launches (no autotuner, no CUDA graph).
 int launch_mode(xfem_body* h, const DevCtx& ctx, uint32_t nsub, float dt) {
 	if (h->ring_mode) {
@@ -2156,13 +2218,13 @@ int launch_mode(xfem_body* h, const DevCtx& ctx, uint32_t nsub, float dt) {
 		ct.el_flat = h->q_flat.p;
 		ct.el_colours = h->q_colours;
 		ct.nel = h->q_nel;
-		const int e = launch_qmixed(ctx, ct, 256, nsub, dt, h->stream);
+		const int e = launch_qmixed(ctx, ct, t10_lanes(h, 8u * 8u * h->sms, 0.75f), nsub, dt, h->stream);
 		if (e) return fail(XFEM_ECUDA, std::string("element launch: ") + cudaGetErrorString((cudaError_t)e));
 		h->launched[XFEM_LAUNCH_STEP] = t_launched;
 		return XFEM_OK;
 	}
 	const int e = h->el_mode == kElH27     ? launch_h27(ctx, nsub, dt, h->stream)
-	              : h->el_mode == kElT10   ? launch_t10(ctx, nsub, dt, h->stream)
+	              : h->el_mode == kElT10   ? launch_t10(ctx, t10_lanes(h, 8u * kT10QuadWarps * h->sms), nsub, dt, h->stream)
 	              : h->el_mode == kElMixed ? launch_mixed(ctx, 256, nsub, dt, h->stream)
 	                                       : launch_hexes(ctx, nsub, dt, h->stream);
 	if (e) return fail(XFEM_ECUDA, std::string("element launch: ") + cudaGetErrorString((cudaError_t)e));

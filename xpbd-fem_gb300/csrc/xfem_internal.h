@@ -367,7 +367,6 @@ struct DevCtx {
 	const uint4* el_vid;
 	const float4* el_rec;
 	const uint32_t* colour_el_begin;  // el_colours + 1
-	uint32_t max_colour_el;           // elements of the largest colour
 	const uint32_t* el_flat;
 	uint32_t nel;
 	uint32_t mt_colours;
@@ -557,8 +556,10 @@ int launch_hex_rings(const DevCtx& ctx, int block, uint32_t nsub, float dt, void
 // colour then every hex colour per sweep, a cooperative persistent launch.
 int launch_mixed(const DevCtx& ctx, int block, uint32_t nsub, float dt, void* stream);
 // Quadratic-tet mode (xfem_t10.cu): nsub substeps of a T10 mesh, likewise.
-int launch_t10(const DevCtx& ctx, uint32_t nsub, float dt, void* stream);
-int launch_t10_lane(const DevCtx& ctx, uint32_t nsub, float dt, void* stream);  // one lane per T10
+// lanes: of a warp per T10, four or one (launch_t10_lane).
+int launch_t10(const DevCtx& ctx, int lanes, uint32_t nsub, float dt, void* stream);
+int launch_t10_lane(const DevCtx& ctx, uint32_t nsub, float dt, void* stream);
+constexpr uint32_t kT10QuadWarps = 12;  // warps of a block of the four-lane kernel, eight T10s each
 // The continuous-pressure models on a T10 mesh (xfem_t10.cu): nsub substeps
 // of one-ring solves over the T10s around the mesh vertices, a cooperative
 // persistent launch (canonical (X, V) in and out).
@@ -566,7 +567,8 @@ int launch_t10_rings(const DevCtx& ctx, int block, uint32_t nsub, float dt, void
 int launch_h27_rings(const DevCtx& ctx, uint32_t nsub, float dt, void* stream);  // block size: kRingWarps of xfem_h27.cu
 // A mesh mixing T10s and H27s: ch27 with the H27 element arrays, ct10 the
 // same context with the T10 element arrays (blocks of 256 threads).
-int launch_qmixed(const DevCtx& ch27, const DevCtx& ct10, int block, uint32_t nsub, float dt, void* stream);
+int launch_qmixed(const DevCtx& ch27, const DevCtx& ct10, int t10_lanes, uint32_t nsub, float dt, void* stream);
+int launch_qmixed_lane(const DevCtx& ch27, const DevCtx& ct10, uint32_t nsub, float dt, void* stream);
 // Quadratic-hex mode (xfem_h27.cu): nsub substeps of an H27 mesh, one warp
 // per element (block must be 256).
 int launch_h27(const DevCtx& ctx, uint32_t nsub, float dt, void* stream);

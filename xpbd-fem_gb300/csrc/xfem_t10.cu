@@ -5,7 +5,7 @@
 // :437-564 with Nodes = 10 and the 4-point rule, PointsLo = PointsHi = 4; the
 // cube models leave a tet alone), SolveVolumeOnly (:840-867), DampElement
 // (:910-928) and PbdDamp (XPBDFEM/Xpbd.h:306-346), in the element kernel of
-// xfem_elements.cuh with four lanes of a warp per T10 or one (launch_t10).
+// xfem_elements.cuh with four lanes of a warp per T10 or one (t10_lanes, xfem_api.cpp).
 //
 // Records: 14 float4 per T10 as a structure of arrays (float4 k of element i
 // at el_rec[k * nel + i]): Qi column-major, volume, surface area, the
@@ -310,17 +310,8 @@ int launch_t10_rings(const DevCtx& ctx, int block, uint32_t nsub, float dt, void
 	return (int)cudaLaunchCooperativeKernel(f, dim3(per_sm * sms), dim3(block), args, smem, st);
 }
 
-// Four lanes per T10 while one round of their warps takes the largest colour,
-// else one: 1,572,864 T10s (52,000 in a colour) take 12.3 ms a frame with one
-// lane and 14.0 with four, 230,400 (10,080) 4.2 and 3.5, 720 3.5 and 2.4.
-int launch_t10(const DevCtx& ctx, uint32_t nsub, float dt, void* stream) {
-	int dev = 0, sms = 0;
-	cudaError_t e = cudaGetDevice(&dev);
-	if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-	if (e != cudaSuccess) return (int)e;
-	if (ctx.max_colour_el <= 8u * (uint32_t)t10e::kQuadWarps * (uint32_t)sms)
-		return launch_elements<t10e::T10Elem>(ctx, nsub, dt, stream);
-	return launch_t10_lane(ctx, nsub, dt, stream);
+int launch_t10(const DevCtx& ctx, int lanes, uint32_t nsub, float dt, void* stream) {
+	return lanes == 4 ? launch_elements<t10e::T10Elem>(ctx, nsub, dt, stream) : launch_t10_lane(ctx, nsub, dt, stream);
 }
 
 }  // namespace xfem

@@ -6,7 +6,7 @@
 // :437-564 with Nodes = 10 and the 4-point rule, PointsLo = PointsHi = 4; the
 // cube models leave a tet alone), SolveVolumeOnly (:840-867), DampElement
 // (:910-928) and PbdDamp (XPBDFEM/Xpbd.h:306-346), in the element kernel of
-// xfem_elements.cuh with four lanes of a warp per T10 or one (launch_t10).
+// xfem_elements.cuh with four lanes of a warp per T10 or one (t10_lanes, xfem_api.cpp).
 //
 // Records: 14 float4 per T10 as a structure of arrays (float4 k of element i
 // at el_rec[k * nel + i]): Qi column-major, volume, surface area, the
@@ -135,9 +135,10 @@ __device__ __forceinline__ void q_rel(const float4 O[10], const float4 D[10], bo
 // 230,400 T10s (31 colours of up to 10,080), 20 substeps: 4,202 us with a lane
 // per T10, 3,515 us with four and the next eight fetched ahead. Twelve warps a
 // block: with eight, a colour of 10,000 needs a second round of a few warps
-// (3,855 us); with sixteen the registers spill (3,914 us). A colour that needs
-// a second round of these warps (over 14,592 T10s on 152 SMs) keeps a lane per
-// T10 (xfem_t10_lane.cu), whose work per element is less.
+// (3,855 us); with sixteen the registers spill (3,914 us). Solves and sizes that
+// run faster with a lane per T10, whose work per element is less, keep one
+// (xfem_t10_lane.cuh; four_lane_share in xfem_api.cpp, at most one round of these
+// warps: 14,592 T10s of a colour on 152 SMs).
 
 // A warp's shared memory. rec: the records, element-major (60 floats apart:
 // eight elements' 16-byte reads fall in different banks); the others
@@ -152,7 +153,7 @@ struct QuadScratch {
 	float4 g0[10][8], g1[10][8];  // the nodes' gradients
 	float4 dots[10][8];    // per node: g0.g0, g1.g0, g1.g1, w
 };
-constexpr int kQuadWarps = 12;
+constexpr int kQuadWarps = (int)kT10QuadWarps;
 struct QuadShared {
 	float4 tab[40];  // shape-function gradients, [point][node]
 	QuadScratch w[kQuadWarps];
