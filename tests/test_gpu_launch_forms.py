@@ -80,9 +80,10 @@ def test_fixed_forms(mode, form):
         assert b.launch()["form"] == form and b.launch()["blocks"] > 1
 
 
+# the reverse as one cluster: up to two chunks of a colour per block (32 x 16 x 16: 32 in 16)
 @pytest.mark.parametrize("dims,record,reverse,lanes", [
     ((8, 2, 2), "cluster", "cluster", 1), ((20, 9, 9), "cluster", "cluster", 1), ((32, 16, 12), "cluster", "cluster", 1),
-    ((32, 20, 16), "cluster", "cluster", 1), ((32, 21, 20), "cluster", "grid", 8)])
+    ((32, 16, 16), "cluster", "cluster", 1), ((32, 17, 16), "cluster", "grid", 8), ((32, 21, 20), "cluster", "grid", 8)])
 def test_adjoint(dims, record, reverse, lanes, monkeypatch):
     b = xfem.Body(*_tets(*dims), _settings(), block_size=256)
     b.adjoint_forward(4, DT, np.uint32([0]))

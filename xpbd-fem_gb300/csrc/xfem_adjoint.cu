@@ -817,9 +817,12 @@ __global__ void __launch_bounds__(256, 1) k_reverse_cluster(DevCtx C, AdjCtx A, 
 }
 
 // Blocks of the one-cluster reverse, 0 when the handle does not take it: all
-// clusters whole cubes, at most 16 colours and at most three chunks of a
-// colour per block (a chunk's chain is a third of a pass of the grid form,
-// which takes any number of chunks up to one per SM in the same time).
+// clusters whole cubes, at most 16 colours and at most two chunks of a colour per
+// block. The grid form takes any number of chunks up to one per SM in about the
+// same time, the cluster one round of its blocks after the other. Measured, 50
+// substeps, cluster and grid: 16 chunks of a colour (one round) 1,476 and 2,992 us,
+// 18 and 32 (two) 2,614 and 3,026, 2,560 and 3,101; 34 and 40 (three) 3,253 and
+// 3,049, 3,726 and 3,209.
 cudaError_t reverse_cluster_blocks(const DevCtx& C, uint32_t max_colour_chunks, uint32_t* blocks, uint32_t* rounds,
                                    size_t* smem) {
 	*blocks = 0;
@@ -827,7 +830,7 @@ cudaError_t reverse_cluster_blocks(const DevCtx& C, uint32_t max_colour_chunks, 
 	uint32_t G = 1;
 	while (G < 16u && G < max_colour_chunks) G *= 2;
 	*rounds = (max_colour_chunks + G - 1) / G;
-	if (*rounds > 3u) return cudaSuccess;
+	if (*rounds > 2u) return cudaSuccess;
 	int dev = 0, optin = 0;
 	cudaError_t e = cudaGetDevice(&dev);
 	if (e == cudaSuccess) e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
