@@ -184,7 +184,6 @@ __device__ __noinline__ void hex_ring_solve(const DevCtx& C, HexRingScratch& S, 
 		w = S.O[lane].w;
 		Dn = S.D[lane];
 	}
-	float none = 0.0f;
 	if (__ldg(&bp.energy) == 8u) {
 		// ContinuousPixar: mu = 2, one constraint U0 + (lambda / 2) U1 with
 		// compliance per the ring volume
@@ -192,13 +191,13 @@ __device__ __noinline__ void hex_ring_solve(const DevCtx& C, HexRingScratch& S, 
 		const float U = fmaxf(0.000001f, fmaf(hw, U1, U0));
 		const Vec3 g = {fmaf(hw, g1.x, g0.x), fmaf(hw, g1.y, g0.y), fmaf(hw, g1.z, g0.z)};
 		ring_update1<DAMP, VMODE>(C, bp, lane, nn, dv, S.O[lane], Dn, w, g, U, __ldg(&bp.compliance) / volume, inv_dt,
-		                          inv_dt2, rd, none);
+		                          inv_dt2, rd);
 		return;
 	}
 	// ContinuousMixed / ContinuousSkin: the deviatoric and hydrostatic pair
 	const float mu = __ldg(&bp.mu), lambda = __ldg(&bp.lambda);
 	ring_update2<DAMP, VMODE>(C, bp, lane, nn, dv, S.O[lane], Dn, w, g0, g1, fmaxf(0.0001f, U0), U1,
-	                          1.0f / (mu * volume), 1.0f / (lambda * volume), inv_dt, inv_dt2, rd, none);
+	                          1.0f / (mu * volume), 1.0f / (lambda * volume), inv_dt, inv_dt2, rd);
 }
 
 // The persistent hex ring kernel (cooperative launch, co-resident grid):

@@ -36,17 +36,18 @@ __device__ __forceinline__ void warp_sums(float (&v)[N]) {
 
 // One constraint U with gradient g and compliance `comp` (per the ring
 // volume). VMODE: RayleighDamp of the velocities (Dn holds V) with ratio rd.
-// also: a value of the caller's summed over the lanes with the rest.
-template <bool DAMP, bool VMODE>
+// also: a value of the caller's summed over the lanes with the rest (none: hex
+// rings paid its butterfly with up to 1% of a pass).
+template <bool DAMP, bool VMODE, class... Also>
 __device__ __forceinline__ void ring_update1(const DevCtx& C, const BodyParams& bp, uint32_t lane, uint32_t nn,
                                              uint32_t dv, const float4& On, float4 Dn, float w, Vec3 g, float U,
-                                             float comp, float inv_dt, float inv_dt2, float rd, float& also) {
+                                             float comp, float inv_dt, float inv_dt2, float rd, Also&... also) {
 	const float damp = DAMP && __ldg(&bp.rayleigh_type) < 2u ? __ldg(&bp.damping) : 0.0f;
 	const bool limit = __ldg(&bp.rayleigh_type) == 1u;
 	const float alpha = comp * inv_dt2;
-	float sums[2] = {w * dot(g, g), also};
+	float sums[1 + sizeof...(Also)] = {w * dot(g, g), also...};
 	warp_sums(sums);
-	also = sums[1];
+	((also = sums[1]), ...);
 	const float wgg = 1.0e-22f + sums[0];
 	if constexpr (VMODE) {
 		const float gV = warp_sum(lane < nn ? dot(g, v3(Dn)) : 0.0f);
@@ -84,18 +85,18 @@ __device__ __forceinline__ void ring_update1(const DevCtx& C, const BodyParams& 
 
 // The deviatoric and hydrostatic pair (U0, g0), (U1, g1) with compliances
 // comp0, comp1 (per the ring volume).
-template <bool DAMP, bool VMODE>
+template <bool DAMP, bool VMODE, class... Also>
 __device__ __forceinline__ void ring_update2(const DevCtx& C, const BodyParams& bp, uint32_t lane, uint32_t nn,
                                              uint32_t dv, const float4& On, float4 Dn, float w, Vec3 g0, Vec3 g1,
                                              float U0, float U1, float comp0, float comp1, float inv_dt, float inv_dt2,
-                                             float rd, float& also) {
+                                             float rd, Also&... also) {
 	const float damp = DAMP && __ldg(&bp.rayleigh_type) < 2u ? __ldg(&bp.damping) : 0.0f;
 	const bool limit = __ldg(&bp.rayleigh_type) == 1u;
 	const float alpha0 = comp0 * inv_dt2, alpha1 = comp1 * inv_dt2;
-	float sums[4] = {w * dot(g0, g0), w * dot(g1, g0), w * dot(g1, g1), also};
+	float sums[3 + sizeof...(Also)] = {w * dot(g0, g0), w * dot(g1, g0), w * dot(g1, g1), also...};
 	warp_sums(sums);
 	const float wgg0 = 1.0e-22f + sums[0], wgg1 = 1.0e-22f + sums[1], wgg2 = 1.0e-22f + sums[2];
-	also = sums[3];
+	((also = sums[3]), ...);
 	float l0, l1;
 	if constexpr (VMODE) {
 		const float b0 = -warp_sum(lane < nn ? dot(g0, v3(Dn)) : 0.0f);
