@@ -176,11 +176,14 @@ __device__ __forceinline__ void h27_ring_solve(const DevCtx& C, H27RingScratch& 
 // warp's scratch 12.8 KB, so that of blocks of four warps only two fit an SM. A frame of
 // 20 substeps, 64 x 48 x 36 H27s: 85.8 ms with those (78.6 with the tables read through L1
 // and four such blocks), 54.9 so; 48 x 25 x 24 H27s 21.4 and 17.6 ms. The bound names one
-// block per SM: without it the compiler plans for two, at 64 registers (57.6 ms).
-constexpr int kRingWarps = 15;
+// block per SM: without it the compiler plans for two, at 64 registers (57.6 ms). With
+// damping 12 warps: at 15 its 128 registers cost small meshes more than two blocks of
+// four warps took (ContinuousMixed with sweeps after the step, 10 substeps: 12 x 10 x 8
+// H27s 11.79 ms then, 12.11 at 15 warps, 11.73 at 12; 64 x 48 x 36 88.5, 57.7, 70.1).
+constexpr int ring_warps(bool damp) { return damp ? 12 : 15; }
 
 template <bool DAMP>
-__global__ void __launch_bounds__(32 * kRingWarps, 1) k_h27_rings(DevCtx C, uint32_t nsub, float dt) {
+__global__ void __launch_bounds__(32 * ring_warps(DAMP), 1) k_h27_rings(DevCtx C, uint32_t nsub, float dt) {
 	extern __shared__ __align__(128) unsigned char smem[];
 	const float inv_dt = 1.0f / dt, inv_dt2 = 1.0f / (dt * dt);
 	const uint32_t lane = threadIdx.x & 31u, wib = threadIdx.x >> 5;
@@ -254,11 +257,11 @@ __global__ void __launch_bounds__(32 * kRingWarps, 1) k_h27_rings(DevCtx C, uint
 
 int launch_h27_rings(const DevCtx& ctx, uint32_t nsub, float dt, void* stream) {
 	if (nsub == 0) return 0;
-	constexpr int block = 32 * kRingWarps;
+	const int block = 32 * ring_warps(ctx.ext != 0u);
 	cudaStream_t st = (cudaStream_t)stream;
 	const void* f = ctx.ext ? (const void*)k_h27_rings<true> : (const void*)k_h27_rings<false>;
-	constexpr size_t smem = sizeof(Tables) + kRingWarps * sizeof(H27RingScratch);
-	static_assert(smem <= 227u * 1024u, "a block's shared memory");
+	const size_t smem = sizeof(Tables) + (size_t)(block / 32) * sizeof(H27RingScratch);
+	static_assert(sizeof(Tables) + ring_warps(false) * sizeof(H27RingScratch) <= 227u * 1024u, "a block's shared memory");
 	int dev = 0, sms = 0, per_sm = 0;
 	cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
 	if (e == cudaSuccess) e = cudaGetDevice(&dev);

@@ -564,7 +564,7 @@ constexpr uint32_t kT10QuadWarps = 12;  // warps of a block of the four-lane ker
 // of one-ring solves over the T10s around the mesh vertices, a cooperative
 // persistent launch (canonical (X, V) in and out).
 int launch_t10_rings(const DevCtx& ctx, int block, uint32_t nsub, float dt, void* stream);
-int launch_h27_rings(const DevCtx& ctx, uint32_t nsub, float dt, void* stream);  // block size: kRingWarps of xfem_h27.cu
+int launch_h27_rings(const DevCtx& ctx, uint32_t nsub, float dt, void* stream);  // block size: ring_warps of xfem_h27.cu
 // A mesh mixing T10s and H27s: ch27 with the H27 element arrays, ct10 the
 // same context with the T10 element arrays (blocks of 256 threads).
 int launch_qmixed(const DevCtx& ch27, const DevCtx& ct10, int t10_lanes, uint32_t nsub, float dt, void* stream);
