@@ -321,3 +321,24 @@ def test_a_handle_follows_its_settings_off_the_bricks_and_back():
             h.step_frames(1, 3, DT)
         assert b.launch()["form"] in forms
         assert np.array_equal(a.positions(), b.positions()) and np.array_equal(a.velocities(), b.velocities())
+
+
+def test_brick_tables_of_the_sweeps_are_built_when_needed():
+    """A handle that never damps does not hold the sweeps' tables on the bricks; one that
+    cannot allocate them sweeps on the grid, and on the bricks once it can."""
+    mesh = _tets(49, 33, 31)
+    b = _automatic([mesh], block_size=256)
+    a = xfem.Body(*mesh, _settings(), sync_mode=1, block_size=256)
+    a.step_frames(1, 20, DT)
+    plain, damped = _settings(), _settings(**DAMPED)
+    before = b.info()["device_bytes"]
+    for s, fail, form in ((damped, True, "grid"), (plain, False, None), (damped, False, "bricks_ext"), (plain, False, "bricks")):
+        if fail:
+            xfem.test_hook(None, xfem.HOOK_FAIL_ALLOC, 1)
+        for h in (b, a):
+            h.set_settings(s)
+            h.step_frames(1, 3, DT)
+        if form:
+            assert b.launch()["form"] == form
+        assert (b.info()["device_bytes"] > before) == (form in ("bricks_ext", "bricks"))
+        assert np.array_equal(a.positions(), b.positions()) and np.array_equal(a.velocities(), b.velocities())

@@ -171,6 +171,7 @@ struct xfem_body {
 	DevBuf<uint32_t> tet_brec_dev;  // per tet (all bodies): its c0 word in the brick chunks
 	DevBuf<uint32_t> bcb, bwait, bcnb_begin, bcnb, bpriv_begin, bpriv_vid, bfin_begin, bfin_vid, bnb_begin, bnb, bflag, blastmask, btflat;
 	DevBuf<float> btarea;
+	std::vector<uint32_t> brick_src;  // per brick chunk lane: the chunk lane whose cluster it holds, or kNoLane
 	// meshes mixing tets and hexes (kElMixed): the tets as elements of their own colouring
 	DevBuf<uint4> mt_vid;
 	DevBuf<float4> mt_rec;
@@ -1220,6 +1221,27 @@ void split_bricks(const xfem_body* h, const std::vector<uint64_t>& lanes, uint32
 	}
 }
 
+// What the sweeps on the bricks (k_bricks_ext) read beside the brick chunks: lastmask, tflat
+// and tarea in their order, 52 bytes per cluster. Built when a handle first needs it.
+int build_brick_sweeps(xfem_body* h) {
+	if (!h->ctx.nbricks || h->ctx.btflat) return XFEM_OK;
+	const size_t n = h->brick_src.size();
+	DevBuf<uint32_t> src;
+	XCUDA(src.alloc(n));
+	XCUDA(h->blastmask.alloc(n));
+	XCUDA(h->btflat.alloc(6 * n));
+	XCUDA(h->btarea.alloc(6 * n));
+	XCUDA(cudaMemcpyAsync(src.p, h->brick_src.data(), n * 4, cudaMemcpyHostToDevice, h->stream));
+	const int e = launch_brick_sweeps(h->ctx, src.p, (uint32_t)n, h->blastmask.p, h->btflat.p, h->btarea.p, h->stream);
+	if (e) return fail(XFEM_ECUDA, "brick sweep tables: launch failed");
+	XCUDA(cudaStreamSynchronize(h->stream));
+	h->ctx.blastmask = h->blastmask.p;
+	h->ctx.btflat = h->btflat.p;
+	h->ctx.btarea = h->btarea.p;
+	h->device_bytes += n * 13 * 4;
+	return XFEM_OK;
+}
+
 // The brick layout of the launch form sync_mode 4 (k_bricks), built from the
 // packed cube chunks. The clusters are divided into `nbricks` runs along the
 // Morton curve (by lowest device vertex), or by split_bricks, of equal length
@@ -1231,8 +1253,7 @@ void split_bricks(const xfem_body* h, const std::vector<uint64_t>& lanes, uint32
 // and the clusters are those of the other launch forms.
 int build_bricks(xfem_body* h, const std::vector<uint32_t>& ccb, const std::vector<float4>& cblk,
                  const std::vector<ChunkMeta>& meta, const std::vector<uint32_t>& lane_dv,
-                 const std::vector<uint8_t>& lane_nv, const std::vector<uint32_t>& lastmask,
-                 const std::vector<uint32_t>& flat, const std::vector<float>& area) {
+                 const std::vector<uint8_t>& lane_nv) {
 	const uint32_t ncol = h->ncolours, nch = (uint32_t)meta.size();
 	int sms = 0, optin = 0, per_sm_smem = 0;
 	XCUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device));
@@ -1399,18 +1420,12 @@ int build_bricks(xfem_body* h, const std::vector<uint32_t>& ccb, const std::vect
 	// (plane 3 of its record) sits in the brick chunks, so that material
 	// changes reach both layouts
 	std::vector<uint32_t> brec_of_slot((size_t)h->nrows * kLanes, 0);
-	std::vector<uint32_t> blast((size_t)nbc * kLanes, 0), bflat((size_t)nbc * kLanes * 6, 0);
-	std::vector<float> barea((size_t)nbc * kLanes * 6, 0.0f);
+	h->brick_src.assign((size_t)nbc * kLanes, kNoLane);
 	parallel_for((uint32_t)bc.size(), [&](uint32_t q) {
 		for (size_t j = 0; j < bc[q].size(); j++) {
 			const uint32_t i = bc[q][j], k = i / kLanes, a = i % kLanes;
 			const uint32_t dch = bcb[q] + (uint32_t)(j / kLanes), dl = (uint32_t)(j % kLanes);
-			blast[(size_t)dch * kLanes + dl] = lastmask[i];
-			for (uint32_t t = 0; t < 6; t++) {
-				const size_t from = ((size_t)meta[k].trow + t) * kLanes + a, to = ((size_t)dch * 6 + t) * kLanes + dl;
-				bflat[to] = flat[from];
-				barea[to] = area[from];
-			}
+			h->brick_src[(size_t)dch * kLanes + dl] = i;
 			const float4* src = &cblk[meta[k].off16];
 			float4* dst = &blk[(size_t)dch * per16];
 			for (uint32_t t = 0; t < 6; t++)
@@ -1432,9 +1447,6 @@ int build_bricks(xfem_body* h, const std::vector<uint32_t>& ccb, const std::vect
 	XCUDA(h->tet_brec_dev.alloc(brec.size()));
 	XCUDA(h->bcblk.alloc(blk.size()));
 	XCUDA(h->bcb.alloc(bcb.size()));
-	XCUDA(h->blastmask.alloc(blast.size()));
-	XCUDA(h->btflat.alloc(bflat.size()));
-	XCUDA(h->btarea.alloc(barea.size()));
 	XCUDA(h->bwait.alloc(bwait.size()));
 	XCUDA(h->bcnb_begin.alloc(cnb_begin.size()));
 	XCUDA(h->bcnb.alloc(std::max<size_t>(1, cnb.size())));
@@ -1451,9 +1463,6 @@ int build_bricks(xfem_body* h, const std::vector<uint32_t>& ccb, const std::vect
 	XCUDA(up(h->bcblk.p, blk.data(), blk.size() * sizeof(float4)));
 	XCUDA(up(h->tet_brec_dev.p, brec.data(), brec.size() * 4));
 	XCUDA(up(h->bcb.p, bcb.data(), bcb.size() * 4));
-	XCUDA(up(h->blastmask.p, blast.data(), blast.size() * 4));
-	XCUDA(up(h->btflat.p, bflat.data(), bflat.size() * 4));
-	XCUDA(up(h->btarea.p, barea.data(), barea.size() * 4));
 	XCUDA(up(h->bwait.p, bwait.data(), bwait.size() * 4));
 	XCUDA(up(h->bcnb_begin.p, cnb_begin.data(), cnb_begin.size() * 4));
 	XCUDA(up(h->bcnb.p, cnb.data(), cnb.size() * 4));
@@ -1466,9 +1475,6 @@ int build_bricks(xfem_body* h, const std::vector<uint32_t>& ccb, const std::vect
 	XCUDA(cudaStreamSynchronize(h->stream));
 	DevCtx& c = h->ctx;
 	c.bcblk = h->bcblk.p;
-	c.blastmask = h->blastmask.p;
-	c.btflat = h->btflat.p;
-	c.btarea = h->btarea.p;
 	c.bchunk_begin = h->bcb.p;
 	c.bchunk_wait_end = h->bwait.p;
 	c.bcnb_begin = h->bcnb_begin.p;
@@ -1482,7 +1488,7 @@ int build_bricks(xfem_body* h, const std::vector<uint32_t>& ccb, const std::vect
 	c.bflag = h->bflag.p;
 	c.nbricks = nb;
 	c.bpriv_max = pmax;
-	h->device_bytes += blk.size() * 16 + (brec.size() + blast.size() + bflat.size() + barea.size() + bcb.size() + bwait.size() + cnb_begin.size() + cnb.size() + pbeg.size() + pvid.size() + fbeg.size() + fvid.size() +
+	h->device_bytes += blk.size() * 16 + (brec.size() + bcb.size() + bwait.size() + cnb_begin.size() + cnb.size() + pbeg.size() + pvid.size() + fbeg.size() + fvid.size() +
 	                                      nbeg.size() + nbv.size() + (size_t)nb * kBrickFlagStride) * 4;
 	if (getenv("XFEM_SETUP_TIMING"))
 		fprintf(stderr, "xfem bricks: %u bricks, %u chunks, %zu private and %zu shared vertices, at most %u private "
@@ -1596,8 +1602,6 @@ int build_device(xfem_body* h) {
 	clk.lap("chunk shapes");
 	std::vector<float4> cblk((size_t)total16, make_float4(0, 0, 0, 0));
 	std::vector<uint32_t> lastmask(nlanes, 0);
-	std::vector<uint32_t> flat;  // per tet row: the tet's index in its body's order
-	std::vector<float> area;     // and its surface area
 	for (auto& b : h->bodies) {
 		b.tet_slot.assign(b.nt, 0xffffffffu);
 		b.tet_rec.assign(b.nt, 0);
@@ -1776,8 +1780,8 @@ int build_device(xfem_body* h) {
 		XCUDA(up(h->tet_inv_mu.p, inv_mu.data(), inv_mu.size() * 4));
 		// per tet row: the index in the body's flattened order (the amortized
 		// damping slices) and the surface area (PBD damping)
-		flat.assign((size_t)trows * kLanes, 0);
-		area.assign((size_t)trows * kLanes, 1.0f);
+		std::vector<uint32_t> flat((size_t)trows * kLanes, 0);
+		std::vector<float> area((size_t)trows * kLanes, 1.0f);
 		for (const BodyHost& b : h->bodies) {
 			const Schedule& sc = b.sched;
 			uint32_t o = 0;
@@ -1879,8 +1883,10 @@ int build_device(xfem_body* h) {
 	h->cfg.total_chunks = nch;
 	h->cfg.colour_chunk_begin_host = ccb;
 	if (all_cube && !h->ring_mode && !h->el_mode && nch && (h->opt.sync_mode == 0 || h->opt.sync_mode == 4)) {
-		const int rb = build_bricks(h, ccb, cblk, meta, lane_dv, lane_nv, lastmask, flat, area);
+		const int rb = build_bricks(h, ccb, cblk, meta, lane_dv, lane_nv);
 		if (rb) return rb;
+		if (h->cfg.ext_level() == 1)
+			if (const int rs = build_brick_sweeps(h)) return rs;
 		clk.lap("bricks");
 	}
 	return update_right_targets(h);
@@ -1894,7 +1900,7 @@ int pick_cluster(xfem_body* h) {
 	h->cfg.brick_ext = false;
 	if (h->cfg.sync_mode != 1 || h->cfg.lambdas || !h->nchunks) return 0;
 	const int e = cluster_plan(h->ctx, h->max_colour_chunks, h->cfg.block, false, h->cfg.ext_level(), &h->cfg.cluster);
-	if (e || h->cfg.cluster.blocks || h->cfg.ext_level() != 1) return e;
+	if (e || h->cfg.cluster.blocks || h->cfg.ext_level() != 1 || !h->ctx.btflat) return e;
 	return brick_ext_fits(h->ctx, h->cfg.block, &h->cfg.brick_ext);
 }
 
@@ -2506,6 +2512,8 @@ int xfem_set_settings(xfem_body* h, uint32_t body, const xfem_settings* s) {
 			if (persistent_grid(h->cfg, &blocks) == 0) h->cfg.blocks = blocks;
 		}
 		const bool was_on_bricks = h->cfg.brick_ext;
+		// without memory for the bricks' tables the sweeps run on the grid
+		if (h->cfg.ext_level() == 1 && h->opt.sync_mode == 0 && build_brick_sweeps(h)) (void)cudaGetLastError();
 		if (const int e = pick_cluster(h))
 			return fail(XFEM_ECUDA, std::string("cluster query failed: ") + cudaGetErrorString((cudaError_t)e));
 		follow_settings(h, was_on_bricks, h->cfg.block);

@@ -224,12 +224,34 @@ __global__ void __launch_bounds__(PAIR ? 192 : 256, PAIR ? 2 : 1) k_bricks_ext(c
 	}
 }
 
+__global__ void k_brick_sweeps(DevCtx C, const uint32_t* __restrict__ src, uint32_t n, uint32_t* __restrict__ lastmask,
+                               uint32_t* __restrict__ flat, float* __restrict__ area) {
+	const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+	if (i >= n) return;
+	const uint32_t from = src[i], chunk = i / kLanes, lane = i % kLanes;
+	const bool on = from != kNoLane;
+	const uint32_t trow = on ? C.chunks[from / kLanes].trow : 0u;
+	lastmask[i] = on ? C.lastmask[from] : 0u;
+	for (uint32_t t = 0; t < 6; t++) {
+		const size_t to = ((size_t)chunk * 6 + t) * kLanes + lane, at = ((size_t)trow + t) * kLanes + from % kLanes;
+		flat[to] = on ? C.tflat[at] : 0u;
+		area[to] = on ? C.tarea[at] : 0.0f;
+	}
+}
+
 const void* brick_ext_fn(bool one, bool pair) {
 	if (pair) return one ? (const void*)k_bricks_ext<true, true> : (const void*)k_bricks_ext<false, true>;
 	return one ? (const void*)k_bricks_ext<true, false> : (const void*)k_bricks_ext<false, false>;
 }
 
 }  // namespace
+
+int launch_brick_sweeps(const DevCtx& ctx, const uint32_t* src, uint32_t n, uint32_t* lastmask, uint32_t* flat, float* area,
+                        void* stream) {
+	if (!n) return 0;
+	k_brick_sweeps<<<(n + 255) / 256, 256, 0, (cudaStream_t)stream>>>(ctx, src, n, lastmask, flat, area);
+	return (int)cudaGetLastError();
+}
 
 // Whether the bricks run at once at this block size. Two bricks per SM have blocks
 // of 192 threads at most: 168 registers a thread.

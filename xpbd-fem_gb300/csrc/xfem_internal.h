@@ -510,6 +510,11 @@ int brick_grid_fits(int block, uint32_t bpriv_max, uint32_t nbricks, bool* fits)
 // size fits, and its launch. Both return a cudaError_t value.
 int brick_ext_fits(const DevCtx& ctx, int block, bool* fits);
 int launch_bricks_ext(const DevCtx& ctx, int block, uint32_t nsub, float dt, void* stream);
+// lastmask, tflat and tarea of the chunks in the order of the brick chunks: src gives each of
+// the n brick chunk lanes its chunk lane.
+constexpr uint32_t kNoLane = 0xffffffffu;
+int launch_brick_sweeps(const DevCtx& ctx, const uint32_t* src, uint32_t n, uint32_t* lastmask, uint32_t* flat, float* area,
+                        void* stream);
 // Dynamic shared memory bytes per block of the solve kernels.
 size_t solve_smem_bytes(int block, uint32_t warp_smem);
 
