@@ -342,3 +342,30 @@ def test_brick_tables_of_the_sweeps_are_built_when_needed():
             assert b.launch()["form"] == form
         assert (b.info()["device_bytes"] > before) == (form in ("bricks_ext", "bricks"))
         assert np.array_equal(a.positions(), b.positions()) and np.array_equal(a.velocities(), b.velocities())
+
+
+def test_a_handle_tuned_with_a_pixar_model_steps_plain_bodies_on_the_bricks():
+    mesh = _tets(49, 33, 31)
+    pixar = _settings(flags=(xfem.ENERGY_PIXAR_SEL << xfem.ENERGY_BIT) | (1 << xfem.XPBD_SOLVE_BIT) | xfem.LOCK_LEFT)
+    a = xfem.Body(*mesh, pixar, sync_mode=1, block_size=256)
+    b = xfem.Body(*mesh, pixar)
+    forms = []
+    for s in (pixar, _settings(), pixar, _settings(**DAMPED), _settings(), pixar):
+        for h in (a, b):
+            h.set_settings(s)
+            h.step_frames(1, 3, DT)
+        forms.append(b.launch()["form"])
+        assert np.array_equal(a.positions(), b.positions()) and np.array_equal(a.velocities(), b.velocities())
+    assert forms[1] == forms[4] == "bricks" and forms[3] == "bricks_ext"
+    assert {forms[0], forms[2], forms[5]} <= {"graph", "grid"} and forms[0] == forms[2] == forms[5]
+
+
+def test_a_handle_tuned_plain_returns_to_its_form():
+    mesh = _tets(49, 33, 31)
+    b = xfem.Body(*mesh, _settings())
+    b.step_frames(1, 20, DT)
+    first = b.launch()
+    for s in (_settings(**DAMPED), _settings(), _settings(flags=W.NH_FLAGS | xfem.LOCK_RIGHT)):
+        b.set_settings(s)
+        b.step_frames(1, 3, DT)
+    assert b.launch() == first

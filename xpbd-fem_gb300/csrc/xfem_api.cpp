@@ -190,9 +190,9 @@ struct xfem_body {
 	bool tuned = false;
 	int brick_block = 256;  // the brick form's default block size (192 with two bricks per SM)
 	float tune_ms = 0.0f;  // the autotuner's best trial time (3 calls), when it timed any
-	// A handle whose sweeps run on the bricks (cfg.brick_ext): the fastest form timed beside
-	// them, and the bricks' block size while the settings need that form (follow_settings)
-	int off_bricks_sync = 0, off_bricks_block = 0, left_bricks_block = 0;
+	// For follow_settings: the fastest form timed beside the bricks, the form timed for the plain
+	// solve, and the bricks' block size while the settings need a form off them
+	int off_bricks_sync = 0, off_bricks_block = 0, plain_sync = 0, plain_block = 0, left_bricks_block = 0;
 	// cached CUDA graph (graph mode)
 	cudaGraphExec_t graph = nullptr;
 	xfem_launch graph_launch{};  // of the captured launches
@@ -1955,27 +1955,30 @@ int set_config(xfem_body* h, int sync_mode, int block) {
 	return XFEM_OK;
 }
 
-// After a change of the settings, for a tuned handle that fixes no form: where the sweeps ran
-// on the bricks, the plain solve does too (sync_mode 4; step() brings them back with the
-// sweeps), and the extended solves, which have no brick kernel, take the fastest other form
-// of the tuning. The block size chosen for the bricks does not suit the grid: 1,572,864 tets,
-// after damping, in one frame of the grid at 192 threads 1,597 us (a second round of chunks;
-// with Pixar 1,842), on the bricks 890 (the colour graph with Pixar 1,429).
-void follow_settings(xfem_body* h, bool was_on_bricks, int block) {
-	if (!h->tuned || h->opt.sync_mode != 0 || h->cfg.brick_ext || h->cfg.cluster.blocks) return;
+// After a change of the settings, for a tuned handle of whole cubes that fixes no form and
+// is too large for one cluster. The plain solve takes the form that was timed for it, else
+// the bricks (sync_mode 4; step() brings the sweeps onto them); the extended solves, which
+// have no brick kernel, take the fastest form timed beside the bricks, whose block size does
+// not suit the grid. 1,572,864 tets, us per frame: plain after damping 1,597 on the grid at
+// the bricks' 192 threads (a second round of chunks), after Pixar 1,328 as the colour graph,
+// 868 on the bricks; Pixar after damping 1,842 on that grid, 1,380 as the colour graph.
+void follow_settings(xfem_body* h, bool swept_on_bricks) {
+	if (!h->tuned || h->opt.sync_mode != 0 || !h->ctx.nbricks || h->cfg.lambdas || h->cfg.cluster.blocks) return;
 	const int level = h->cfg.ext_level();
-	if (!was_on_bricks) {
-		if (!h->left_bricks_block || level == 2) return;
-		block = h->left_bricks_block;
-	}
+	const bool on_bricks = swept_on_bricks || h->cfg.sync_mode == 4;
+	const int block = on_bricks ? h->cfg.block : h->left_bricks_block ? h->left_bricks_block : h->brick_block;
 	// a form that does not fit leaves the handle as it is
-	if (level == 0)
-		set_config(h, 4, block);
-	else if (level == 1)
-		set_config(h, 1, block);
-	else if (h->off_bricks_sync)
+	if (level == 0) {
+		if (h->plain_sync)
+			set_config(h, h->plain_sync, h->plain_block);
+		else if (h->cfg.sync_mode != 4)
+			set_config(h, 4, block);
+	} else if (level == 1) {
+		if (h->left_bricks_block && !h->cfg.brick_ext) set_config(h, 1, block);
+	} else if (on_bricks && h->off_bricks_sync) {
 		set_config(h, h->off_bricks_sync, h->off_bricks_block);
-	h->left_bricks_block = level == 2 ? block : 0;
+	}
+	h->left_bricks_block = level < 2 ? 0 : on_bricks ? block : h->left_bricks_block;
 }
 
 int run(xfem_body* h, uint32_t nsub, float dt) {
@@ -2080,6 +2083,7 @@ int autotune(xfem_body* h, uint32_t nsub, float dt, bool force_time = false) {
 	int rc = check_device_error(h);
 	if (rc) return rc;
 	h->tune_ms = best;
+	if (h->cfg.ext_level() == 0) h->plain_sync = pick.first, h->plain_block = pick.second;
 	return set_config(h, pick.first, pick.second);
 }
 
@@ -2511,12 +2515,12 @@ int xfem_set_settings(xfem_body* h, uint32_t body, const xfem_settings* s) {
 			int blocks = 0;
 			if (persistent_grid(h->cfg, &blocks) == 0) h->cfg.blocks = blocks;
 		}
-		const bool was_on_bricks = h->cfg.brick_ext;
+		const bool swept_on_bricks = h->cfg.brick_ext;
 		// without memory for the bricks' tables the sweeps run on the grid
 		if (h->cfg.ext_level() == 1 && h->opt.sync_mode == 0 && build_brick_sweeps(h)) (void)cudaGetLastError();
 		if (const int e = pick_cluster(h))
 			return fail(XFEM_ECUDA, std::string("cluster query failed: ") + cudaGetErrorString((cudaError_t)e));
-		follow_settings(h, was_on_bricks, h->cfg.block);
+		follow_settings(h, swept_on_bricks);
 	}
 	if (h->ring_mode) h->ctx.ext = ring_damp_of(h->bodies) ? 1u : 0u;
 	const float4* rt_before = h->ctx.right_target;
