@@ -1,9 +1,10 @@
 // Element modes of libxfem.so (sm_103a): the pieces shared by the hex mode
-// (xfem_hexes.cu) and the quadratic-tet mode (xfem_t10.cu). The constraint
+// (xfem_hexes.cu), the quadratic-tet mode (xfem_t10.cu) and the quadratic-hex
+// mode (xfem_h27.cu). The constraint
 // solves over N nodes (XPBDFEM/Xpbd.h:87-215), PbdDamp over N nodes
 // (XPBDFEM/Xpbd.h:306-346), and the persistent kernel that runs a substep as
 // GeoLinear3d / GeoQuadratic3d do: one pass that advances every vertex, one
-// pass per colour with one thread per element, the volume sweeps, and with
+// pass per colour with one lane, four lanes or a warp per element, the volume sweeps, and with
 // post-step damping a finalize pass and the damping passes, each pass ended
 // by the bounded grid barrier. Internal linkage: each translation unit gets
 // its own copy.

@@ -547,8 +547,8 @@ int launch_scatter_xyz(float4* vert, int which, const uint32_t* dev_of_caller, u
                        void* stream);
 int launch_volume(const float4* vert, const uint32_t* tets_dev, uint32_t nt, double* out, void* stream);
 // One-ring mode (xfem_rings.cu): nsub substeps of the continuous-pressure
-// models, a cooperative persistent launch of `block` threads per block
-// (canonical (X, V) in and out).
+// models, a cooperative persistent launch (canonical (X, V) in and out;
+// ring_block of xfem_rings.cu threads per block).
 int launch_rings(const DevCtx& ctx, uint32_t nsub, float dt, void* stream);
 // Hex mode (xfem_hexes.cu): nsub substeps of a hex mesh, a cooperative
 // persistent launch (canonical (X, V) in and out).
@@ -571,11 +571,12 @@ constexpr uint32_t kT10QuadWarps = 12;  // warps of a block of the four-lane ker
 int launch_t10_rings(const DevCtx& ctx, int block, uint32_t nsub, float dt, void* stream);
 int launch_h27_rings(const DevCtx& ctx, uint32_t nsub, float dt, void* stream);  // block size: ring_warps of xfem_h27.cu
 // A mesh mixing T10s and H27s: ch27 with the H27 element arrays, ct10 the
-// same context with the T10 element arrays (blocks of 256 threads).
+// same context with the T10 element arrays (blocks of 256 threads), t10_lanes of a
+// warp per T10.
 int launch_qmixed(const DevCtx& ch27, const DevCtx& ct10, int t10_lanes, uint32_t nsub, float dt, void* stream);
 int launch_qmixed_lane(const DevCtx& ch27, const DevCtx& ct10, uint32_t nsub, float dt, void* stream);
 // Quadratic-hex mode (xfem_h27.cu): nsub substeps of an H27 mesh, one warp
-// per element (block must be 256).
+// per element.
 int launch_h27(const DevCtx& ctx, uint32_t nsub, float dt, void* stream);
 // Per-tet material (n tets from the given per-tet tables): c0 of each record
 // and 1/mu; mu null = mu_uniform for all.
