@@ -369,3 +369,20 @@ def test_a_handle_tuned_plain_returns_to_its_form():
         b.set_settings(s)
         b.step_frames(1, 3, DT)
     assert b.launch() == first
+
+
+# one brick per SM of few chunks with slots for every vertex of its own (generic accesses); a
+# chosen number of bricks: with more chunks, and with vertices that get no slot (the branch)
+@pytest.mark.parametrize("bodies", [1, 2])
+@pytest.mark.parametrize("dims,bricks", [((40, 24, 20), 0), ((40, 24, 20), 9), ((48, 32, 24), 3)])
+def test_chosen_numbers_of_bricks(dims, bricks, bodies):
+    meshes = [_tets(*dims)] * bodies
+    s = [_settings(ground=1, ground_normal=(0.0, 1.0, 0.0), ground_offset=-0.01, friction=0.4)] * bodies
+    a = xfem.Body(meshes=meshes, settings=s, sync_mode=1, block_size=256)
+    b = xfem.Body(meshes=meshes, settings=s, sync_mode=4, block_size=256, bricks=bricks)
+    for n in (7, 2):
+        for h in (a, b):
+            h.step_frames(1, n, DT)
+    assert b.launch()["form"] == "bricks" and (not bricks or b.launch()["blocks"] == bricks)
+    for k in range(bodies):
+        assert np.array_equal(a.positions(k), b.positions(k)) and np.array_equal(a.velocities(k), b.velocities(k))

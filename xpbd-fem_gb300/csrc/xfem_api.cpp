@@ -1335,6 +1335,7 @@ int build_bricks(xfem_body* h, const std::vector<uint32_t>& ccb, const std::vect
 	std::vector<uint32_t> slot(nvv, 0xffffffffu), npriv(nb, 0);
 	std::vector<std::vector<uint32_t>> priv(nb), fin(nb);
 	std::vector<std::vector<uint32_t>> nbl(nb);
+	uint32_t unslotted = 0;  // vertices of one brick only that its shared memory has no slot for
 	for (uint32_t v = 0; v < nvv; v++) {
 		const uint32_t t0 = toff[v], t1 = toff[v + 1];
 		if (t0 == t1) continue;  // in no cluster
@@ -1348,6 +1349,7 @@ int build_bricks(xfem_body* h, const std::vector<uint32_t>& ccb, const std::vect
 			slot[v] = npriv[bmin]++;
 			priv[bmin].push_back(v);
 		} else {
+			unslotted += one ? 1u : 0u;
 			fin[bmin].push_back(v);  // the lowest brick touching it finalizes it
 			for (uint32_t x = t0; x < t1; x++)
 				for (uint32_t y = t0; y < t1; y++)
@@ -1487,6 +1489,7 @@ int build_bricks(xfem_body* h, const std::vector<uint32_t>& ccb, const std::vect
 	c.bnb = h->bnb.p;
 	c.bflag = h->bflag.p;
 	c.nbricks = nb;
+	c.bgeneric = !unslotted && L <= 6ull * nb * kLanes * ncol ? 1u : 0u;  // bricks_fn
 	c.bpriv_max = pmax;
 	h->device_bytes += blk.size() * 16 + (brec.size() + bcb.size() + bwait.size() + cnb_begin.size() + cnb.size() + pbeg.size() + pvid.size() + fbeg.size() + fvid.size() +
 	                                      nbeg.size() + nbv.size() + (size_t)nb * kBrickFlagStride) * 4;
@@ -1920,7 +1923,7 @@ int set_config(xfem_body* h, int sync_mode, int block) {
 		if (brick_smem_bytes(block, h->ctx.bpriv_max) > (size_t)optin)
 			return fail(XFEM_EINVAL, "the bricks need more shared memory than the device allows");
 		bool fits = false;
-		if (const int e = brick_grid_fits(block, h->ctx.bpriv_max, h->ctx.nbricks, &fits))
+		if (const int e = brick_grid_fits(h->ctx, block, &fits))
 			return fail(XFEM_ECUDA, std::string("brick kernel configuration: ") + cudaGetErrorString((cudaError_t)e));
 		if (!fits) return fail(XFEM_EUNSUPPORTED, "the bricks do not fit on the device at once");
 		h->cfg.sync_mode = 4;

@@ -408,6 +408,7 @@ struct DevCtx {
 	const uint32_t* bnb;
 	uint32_t* bflag;
 	uint32_t nbricks, bpriv_max;
+	uint32_t bgeneric;  // one brick per SM: generic vertex accesses (bricks_fn)
 	uint32_t nbodies;
 	const uint32_t* blastmask;  // lastmask, tflat and tarea of the brick chunks (six tet rows each)
 	const uint32_t* btflat;
@@ -505,7 +506,7 @@ int launch_cluster(const DevCtx& ctx, const ClusterPlan& plan, int block, bool t
 // cooperative launch needs the whole grid resident). Returns a cudaError_t
 // value; *fits is set on success.
 size_t brick_smem_bytes(int block, uint32_t bpriv_max);
-int brick_grid_fits(int block, uint32_t bpriv_max, uint32_t nbricks, bool* fits);
+int brick_grid_fits(const DevCtx& ctx, int block, bool* fits);
 // The extended kernel on the bricks (xfem_bricks_ext.cu): whether this block
 // size fits, and its launch. Both return a cudaError_t value.
 int brick_ext_fits(const DevCtx& ctx, int block, bool* fits);

@@ -243,9 +243,9 @@ __device__ __forceinline__ int next_brick_chunk(const uint32_t* bcb, uint32_t nc
 // bodies: the body parameters (a shared-memory copy when the handle has few).
 // ONE: a single body, whose parameters bp1 and material mat1 the kernel holds
 // in registers.
-template <bool ONE, bool PAIR>
+template <bool ONE, bool PAIR, bool GENERIC>
 __device__ __forceinline__ void run_chunk_brick(const DevCtx& C, Stage& st, const BrickLane& bl, int next, uint32_t lane, bool first,
-                                                float dt, float inv_dt, float inv_dt2, const BrickVerts<!PAIR>& vs,
+                                                float dt, float inv_dt, float inv_dt2, const BrickVerts<GENERIC>& vs,
                                                 const BodyParams* bodies, bool bshared,
                                                 const BodyParams& bp1, const Mat& mat1) {
 	const float4* rec = reinterpret_cast<const float4*>(st.buf);
@@ -287,7 +287,7 @@ __device__ __forceinline__ void run_chunk_brick(const DevCtx& C, Stage& st, cons
 // per SM has registers left, and reads a tet's record while the one before is
 // solved (four frames of a batch of 96 uneven bodies: 4,086 -> 3,815 us, and 3,695
 // with the vertices through generic addresses).
-template <bool ONE, bool PAIR>
+template <bool ONE, bool PAIR, bool GENERIC>
 __global__ void __launch_bounds__(PAIR ? 192 : 256, PAIR ? 2 : 1) k_bricks(DevCtx C, uint32_t nsub, float dt) {
 	extern __shared__ __align__(128) uint8_t smem[];
 	__shared__ uint32_t s_bcb[65], s_bwait[64];
@@ -300,7 +300,7 @@ __global__ void __launch_bounds__(PAIR ? 192 : 256, PAIR ? 2 : 1) k_bricks(DevCt
 	Stage st = brick_stage_init(lane);
 	float4* sv = reinterpret_cast<float4*>(smem + (size_t)wpb * kBrickChunkBytes);
 	uint32_t* spid = reinterpret_cast<uint32_t*>(sv + 2 * (size_t)C.bpriv_max);
-	const BrickVerts<!PAIR> vs = {sv, spid, C.bpriv_max};
+	const BrickVerts<GENERIC> vs = {sv, spid, C.bpriv_max};
 	for (uint32_t i = threadIdx.x; i <= ncol; i += blockDim.x) {
 		s_bcb[i] = __ldg(C.bchunk_begin + (size_t)b * ncol + i);
 		if (i < ncol) s_bwait[i] = __ldg(C.bchunk_wait_end + (size_t)b * ncol + i);
@@ -365,7 +365,7 @@ __global__ void __launch_bounds__(PAIR ? 192 : 256, PAIR ? 2 : 1) k_bricks(DevCt
 					if (bad) break;
 				}
 				if (PAIR) bl = brick_lane(st, lane);
-				run_chunk_brick<ONE, PAIR>(C, st, bl, next, lane, s == 0, dt, inv_dt, inv_dt2, vs, bodies, bshared, bp1,
+				run_chunk_brick<ONE, PAIR, GENERIC>(C, st, bl, next, lane, s == 0, dt, inv_dt, inv_dt2, vs, bodies, bshared, bp1,
 				                     mat1);
 			}
 			if (__syncthreads_or(bad ? 1 : 0)) {
@@ -596,25 +596,35 @@ size_t brick_smem_bytes(int block, uint32_t bpriv_max) {
 	return (size_t)(block / 32) * kBrickChunkBytes + (size_t)bpriv_max * kBrickVertexBytes;
 }
 
-const void* bricks_fn(bool one, bool pair) {
-	if (pair) return one ? (const void*)k_bricks<true, true> : (const void*)k_bricks<false, true>;
-	return one ? (const void*)k_bricks<true, false> : (const void*)k_bricks<false, false>;
+// GENERIC vertex accesses with one brick per SM, of six chunks of a colour at most, where every
+// vertex of one brick only has a slot: the bricks of every handle that leaves their number to
+// the library. Larger ones (a number that the caller chose) keep the branch: with more of
+// their vertices in vert, one 256-bit access is faster than two generic ones, and a second
+// round of chunks hides the branch. Measured, us per frame, generic and branch: 98,304 cubes
+// in 152 bricks (2.5 chunks) 651 and 688, in 80 (4.8) 755 and 779, in 50 (7.7) 1,197 and
+// 1,173; 262,144 in 152 (6.7) 1,050 and 1,001, in 80 (12.8) 1,768 and 1,480; without slots for
+// all, 98,304 in 5 13,310 and 7,080, 737,280 in 152 2,820 and 2,225. Two bricks per SM: the
+// branch (BrickVerts).
+const void* bricks_fn(bool one, bool pair, bool generic) {
+	if (pair) return one ? (const void*)k_bricks<true, true, false> : (const void*)k_bricks<false, true, false>;
+	if (generic) return one ? (const void*)k_bricks<true, false, true> : (const void*)k_bricks<false, false, true>;
+	return one ? (const void*)k_bricks<true, false, false> : (const void*)k_bricks<false, false, false>;
 }
 
-int brick_grid_fits(int block, uint32_t bpriv_max, uint32_t nbricks, bool* fits) {
-	const size_t smem = brick_smem_bytes(block, bpriv_max);
+int brick_grid_fits(const DevCtx& ctx, int block, bool* fits) {
+	const size_t smem = brick_smem_bytes(block, ctx.bpriv_max);
 	int dev = 0, sms = 0, per_sm = 1 << 20;
 	cudaError_t e = cudaGetDevice(&dev);
 	if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
 	for (int one = 0; one < 2 && e == cudaSuccess; one++) {
-		const void* f = bricks_fn(one != 0, nbricks > (uint32_t)sms);
+		const void* f = bricks_fn(one != 0, ctx.nbricks > (uint32_t)sms, ctx.bgeneric != 0u);
 		int n = 0;
 		e = set_smem_attr(f, smem);
 		if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, f, block, smem);
 		per_sm = std::min(per_sm, n);
 	}
 	if (e != cudaSuccess) return (int)e;
-	*fits = (uint64_t)per_sm * (uint64_t)sms >= nbricks && nbricks > 0;
+	*fits = (uint64_t)per_sm * (uint64_t)sms >= ctx.nbricks && ctx.nbricks > 0;
 	return 0;
 }
 
@@ -652,7 +662,7 @@ int launch_substeps(const DevCtx& ctx, const LaunchCfg& cfg, uint32_t nsub, floa
 			DevCtx c = ctx;
 			float dtv = dt;
 			void* args[] = {&c, &n, &dtv};
-			const void* f = bricks_fn(ctx.nbodies == 1, ctx.nbricks > (uint32_t)sms);
+			const void* f = bricks_fn(ctx.nbodies == 1, ctx.nbricks > (uint32_t)sms, ctx.bgeneric != 0u);
 			note_launch(XFEM_FORM_BRICKS, ctx.nbricks, (uint32_t)cfg.block, 1);
 			e = cudaLaunchCooperativeKernel(f, dim3(ctx.nbricks), dim3(cfg.block), args, smem_b, st);
 			if (e != cudaSuccess) return (int)e;
