@@ -386,3 +386,12 @@ def test_chosen_numbers_of_bricks(dims, bricks, bodies):
     assert b.launch()["form"] == "bricks" and (not bricks or b.launch()["blocks"] == bricks)
     for k in range(bodies):
         assert np.array_equal(a.positions(k), b.positions(k)) and np.array_equal(a.velocities(k), b.velocities(k))
+
+
+def test_a_chosen_number_of_bricks_is_for_sync_mode_4():
+    """The sweeps of an automatic handle stay off bricks whose number the caller chose."""
+    b = xfem.Body(*_tets(49, 33, 31), _settings(), bricks=3)
+    b.step_frames(1, 5, DT)
+    b.set_settings(_settings(**DAMPED))
+    b.step_frames(1, 2, DT)
+    assert b.launch()["form"] in ("grid", "graph")

@@ -1903,7 +1903,8 @@ int pick_cluster(xfem_body* h) {
 	h->cfg.brick_ext = false;
 	if (h->cfg.sync_mode != 1 || h->cfg.lambdas || !h->nchunks) return 0;
 	const int e = cluster_plan(h->ctx, h->max_colour_chunks, h->cfg.block, false, h->cfg.ext_level(), &h->cfg.cluster);
-	if (e || h->cfg.cluster.blocks || h->cfg.ext_level() != 1 || !h->ctx.btflat) return e;
+	// (a number of bricks that the caller chose is for sync_mode 4 and may be far from the SMs')
+	if (e || h->cfg.cluster.blocks || h->cfg.ext_level() != 1 || !h->ctx.btflat || h->opt.bricks) return e;
 	return brick_ext_fits(h->ctx, h->cfg.block, &h->cfg.brick_ext);
 }
 
@@ -1966,7 +1967,7 @@ int set_config(xfem_body* h, int sync_mode, int block) {
 // the bricks' 192 threads (a second round of chunks), after Pixar 1,328 as the colour graph,
 // 868 on the bricks; Pixar after damping 1,842 on that grid, 1,380 as the colour graph.
 void follow_settings(xfem_body* h, bool swept_on_bricks) {
-	if (!h->tuned || h->opt.sync_mode != 0 || !h->ctx.nbricks || h->cfg.lambdas || h->cfg.cluster.blocks) return;
+	if (!h->tuned || h->opt.sync_mode != 0 || !h->ctx.nbricks || h->opt.bricks || h->cfg.lambdas || h->cfg.cluster.blocks) return;
 	const int level = h->cfg.ext_level();
 	const bool on_bricks = swept_on_bricks || h->cfg.sync_mode == 4;
 	const int block = on_bricks ? h->cfg.block : h->left_bricks_block ? h->left_bricks_block : h->brick_block;
